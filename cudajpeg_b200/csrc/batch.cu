@@ -86,6 +86,7 @@ struct CJBatchCtl {
   int next_sync, next_write, next_fix[3];  // dynamic work counters
   unsigned pix_done;                      // pixel-kernel CTAs finished
   int next_hyp, next_probe;               // work counters of the phase-hypothesis decodes and probes
+  int on_sm[256], slot_ctas[8];           // CTA ranks (BTRank)
   // %globaltimer (ns) at each phase start (CTA 0); t[BT_NPHASE] = end of the
   // pixel kernel (its last CTA)
   unsigned long long t[BT_NPHASE + 1];
@@ -109,6 +110,7 @@ struct CJBatchArgs {
   const CJImageHeader* hdr;
   const CJImageDesc* desc;
   CJScanParams* prm;
+  CJSpecTab* spec;  // per image (only those whose own tables serve: CJScanParams::tab)
   CJStatus* st;
   const uint8_t* blob;
   uint8_t* data;
@@ -130,6 +132,7 @@ struct CJBatchArgs {
   int64_t npix;   // fancy mode: pixels of the batch
   CJBatchCtl* ctl;
   int n, ntiles, nwarps, nptiles, max_passes;
+  int tab_ref;  // the image whose DHT contents the others are compared with
   unsigned wait_limit;  // grid-barrier polls before a timeout (0 = default)
   // MCU-phase hypotheses (0 or 1: none): subsequences not at a segment start
   // are also decoded from their first bit under MCU phases 0 .. nhyp - 1
@@ -241,14 +244,20 @@ __device__ __forceinline__ uint64_t bt_map_compose(uint64_t f, uint64_t g, int n
 // checkpoints) without decoding; the other moved lanes re-decode as in
 // cj_warp_settle.  Lane u is final after the round, so the loop ends within
 // 33 rounds; with the maps defined it ends after one.
-__device__ __forceinline__ bool bt_settle_map(const CJBatchArgs& a, const CJScanParams& sp, const CJSteps& T,
-                                           const uint32_t* words, const CJLane& ln, bool pred_head, CJSubRec& r,
-                                           uint64_t lane0_in, CJCkpt* ck, uint32_t cs, int64_t gs, int nhi) {
+__device__ __forceinline__ bool bt_settle_map(const CJBatchArgs& a, CJSpecJob& x, const CJLane& ln, bool pred_head,
+                                           uint64_t lane0_in, int64_t gs, int nhi, uint32_t* hpp) {
   const int lane = threadIdx.x & 31;
   const int NH = a.nhyp;
   const int64_t hb = gs * 2 * NH;
   const CJCkpt* hck = cj_lane_ckpts(a.hckpt, hb);
   const CJSubRec* hrec = a.hrecs + hb;
+  CJSubRec& r = x.r;
+  CJCkpt* ck = x.ck;
+  x.resume = true;
+  x.hck = hck;
+  x.hrec = hrec;
+  x.hpp = (uint32_t)__cvta_generic_to_shared(hpp);
+  x.nh = nhi + 1;
   uint64_t M = BT_MAP_NONE;
   if (ln.active && ln.head) {
     M = 0;  // a segment's first subsequence starts exactly: its hypothesis 0
@@ -259,7 +268,7 @@ __device__ __forceinline__ bool bt_settle_map(const CJBatchArgs& a, const CJScan
     for (int p = 0; p < 16; p++)
       if (p < NH) M &= ~((uint64_t)(15u ^ ((wv[p >> 2] >> (8 * (p & 3))) & 15u)) << (4 * p));
   }
-  bool dirty = false;
+  bool dirty = false, filled = false;
   for (int it = 0; it < 34; it++) {
     const uint64_t pred = __shfl_up_sync(CJ_FULL, r.exit, 1);
     const uint64_t want = ln.head ? r.start : (lane == 0 ? lane0_in : pred);
@@ -285,7 +294,8 @@ __device__ __forceinline__ bool bt_settle_map(const CJBatchArgs& a, const CJScan
     }
     uint32_t pidx = __shfl_up_sync(CJ_FULL, (uint32_t)v & 15u, 1);
     if (lane == u) pidx = q;
-    if (ln.active && !ln.head && lane >= u && pidx < 15) {
+    const bool probe = ln.active && !ln.head && lane >= u && pidx < 15, redo = change && !probe;
+    if (probe) {
       const CJSubRec* pr = hrec + NH + pidx;
       if (__ldcg(&pr->start) != r.start) {
         r = bt_load_rec(pr);
@@ -295,37 +305,68 @@ __device__ __forceinline__ bool bt_settle_map(const CJBatchArgs& a, const CJScan
                          __ldcg(&pc[k].d2)};
         dirty = true;
       }
-    } else if (change) {
-      r = cj_spec_decode<true, true>(sp, T, words, ln, want, ck, r, cs, hck, hrec, nhi + 1);
-      dirty = true;
+    }
+    if (__any_sync(CJ_FULL, redo)) {
+      if (!filled && ln.active && !ln.head) cj_hyp_fill(hpp, hck, nhi + 1);
+      filled = true;
+      cj_spec_warp<true>(&x, redo, want);
+      dirty = dirty || redo;
     }
   }
   return dirty;
 }
 
-// Next warp item from a work counter (lane 0 takes it, the warp shares it).
-__device__ __forceinline__ int bt_next_item(int* counter) {
+// Work items.  A phase's first items are dealt out by the CTA's rank, the rest
+// through a work counter, so slow items do not hold up what is behind them.
+// Ranks count through the SMs: the CTAs that are the first on their SM, then
+// the second ones, and so on, so a batch with fewer items than the grid has
+// CTAs spreads over the SMs.  (Block indices do not: the hardware fills the
+// SMs of one processing cluster before the others -- blocks 0-17 of a 3-per-SM
+// grid run on 6 SMs -- and with the counter alone 19 groups on 148 SMs took
+// twice as long as 3.)
+struct BTRank {
+  int slot, r;  // how many CTAs were on the SM before this one; order among their equals
+  int rank;     // after the first grid barrier
+};
+#define BT_SM_SLOTS 8  // (entries of slot_ctas)
+// Thread 0, before the first grid barrier.
+__device__ __forceinline__ void bt_rank_begin(CJBatchCtl* ctl, BTRank& k) {
+  uint32_t sm;
+  asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
+  k.slot = sm < 256 ? min(atomicAdd(&ctl->on_sm[sm], 1), BT_SM_SLOTS - 1) : BT_SM_SLOTS - 1;
+  k.r = atomicAdd(&ctl->slot_ctas[k.slot], 1);
+}
+// Thread 0, after it.
+__device__ __forceinline__ void bt_rank_end(CJBatchCtl* ctl, BTRank& k) {
+  k.rank = k.r;
+  for (int s = 0; s < k.slot; s++) k.rank += __ldcg(&ctl->slot_ctas[s]);
+}
+
+// Next warp item: item w * gridDim + rank to warp w first.
+__device__ __forceinline__ int bt_next_item(int* counter, int rank, bool& first) {
+  const int nw = blockDim.x >> 5;
   int w = 0;
-  if ((threadIdx.x & 31) == 0) w = atomicAdd(counter, 1);
+  if (first) {
+    first = false;
+    return (int)(threadIdx.x >> 5) * (int)gridDim.x + rank;
+  }
+  if ((threadIdx.x & 31) == 0) w = atomicAdd(counter, 1) + nw * (int)gridDim.x;
   return __shfl_sync(0xFFFFFFFFu, w, 0);
 }
 
-// Next group of BT_WARPS consecutive items for the whole CTA (thread 0 takes
-// it, the CTA shares it).  The leading barrier also ends the previous group:
-// every warp is done with it and with the tables staged for it.
-__device__ __forceinline__ int bt_next_group(int* counter, int* s_slot) {
+// Next group of BT_WARPS consecutive items for the whole CTA: group `rank`
+// first, then thread 0 takes one and the CTA shares it.  The leading barrier
+// also ends the previous group: every warp is done with it and with the tables
+// staged for it.
+__device__ __forceinline__ int bt_next_group(int* counter, int* s_slot, int rank, bool& first) {
   __syncthreads();
-  if (threadIdx.x == 0) *s_slot = atomicAdd(counter, BT_WARPS);
+  if (first) {
+    first = false;
+    return rank * BT_WARPS;
+  }
+  if (threadIdx.x == 0) *s_slot = atomicAdd(counter, BT_WARPS) + (int)gridDim.x * BT_WARPS;
   __syncthreads();
   return *s_slot;
-}
-
-// Copy one image's decode-step tables (16 KB) into shared memory.  The
-// tables were built by another CTA in this kernel: read them from L2.
-__device__ __forceinline__ void bt_copy_steps(CJSteps* dst, const CJSteps* src) {
-  const int4* s = reinterpret_cast<const int4*>(src);
-  int4* d = reinterpret_cast<int4*>(dst);
-  for (int k = threadIdx.x; k < (int)(sizeof(CJSteps) / 16); k += blockDim.x) d[k] = __ldcg(s + k);
 }
 
 // Largest i with key(i) <= v over a sorted int32 field of the descriptors.
@@ -340,108 +381,179 @@ __device__ __forceinline__ int bt_find(int n, int v, F key) {
   return lo;
 }
 
-// Step tables of the sync and fix-up phases, staged per item group: a group's warps
-// [wa, wb] span few images, and the step tables of the first and the last
-// of them are copied into shared memory (slots 0 and 1), so every symbol
-// lookup is a shared-memory load instead of an L2 round trip (the tables of
-// all images of a batch do not fit in L1).  Images strictly between the two
-// (a run of tiny images) read their tables from global memory.
-struct BTStaged {
-  int ia, ib;
-};
-// Dynamic shared memory of the decode kernel: two staged table slots in the
-// sync and fix-up phases, the write-out's block buffers (one 64-entry int16
-// block per thread) in phase 8.  More would shrink the L1 share the
-// bitstream reads of the sync phase depend on.
+// Dynamic shared memory of the decode kernel: two slots of speculative-decode
+// tables and the warps' bit windows in the sync and fix-up phases (54 KB: 4
+// CTAs per SM), the write-out's block buffers (one 64-entry int16 block per thread) in
+// phase 8.
 #define BT_WBUF_BYTES (BT_THREADS * 64 * 2)
-#define BT_DECODE_SMEM (2 * sizeof(CJSteps))
+#define BT_SPEC_OFF (2 * sizeof(CJSpecTab))  // the warps' rings and phase entries
+#define BT_HPP_OFF (BT_SPEC_OFF + BT_WARPS * sizeof(CJSpecWarp))  // hypothesis variant: checkpoint positions
+#define BT_DECODE_SMEM BT_HPP_OFF
+static constexpr size_t bt_decode_smem(int nhyp) {
+  return BT_DECODE_SMEM + (nhyp > 1 ? (size_t)BT_WARPS * nhyp * CJ_CKPTS * 32 * 4 : 0);
+}
 static_assert(BT_DECODE_SMEM >= BT_WBUF_BYTES, "write-out block buffers");
-static_assert(sizeof(CJSteps) % 16 == 0 && offsetof(CJScanParams, steps) % 16 == 0, "int4 table copy");
+static_assert(sizeof(CJSpecTab) % 16 == 0, "int4 table copy");
 static_assert(BT_DECODE_SMEM >= BT_THREADS * sizeof(CJAgg5), "phase 7 scan space");
 
 __device__ __forceinline__ int bt_image_of_warp(const CJBatchArgs& a, int w) {
   return bt_find(a.n, w, [&](int k) { return a.desc[k].sub0 >> 5; });
 }
 
-// All threads of the CTA: stage the tables of warps [wa, wb]'s first and last image.
-__device__ __forceinline__ BTStaged bt_stage(const CJBatchArgs& a, int wa, int wb, CJSteps* tab) {
-  BTStaged g;
-  g.ia = bt_image_of_warp(a, wa);
-  g.ib = bt_image_of_warp(a, wb);
-  bt_copy_steps(&tab[0], &a.prm[g.ia].steps);
-  if (g.ib != g.ia) bt_copy_steps(&tab[1], &a.prm[g.ib].steps);
-  __syncthreads();
-  return g;
+// Warp w of the batch: its image, the image whose tables serve it (-1: the
+// warp has no subsequences, or the image no MCU phase h), its first subsequence.
+struct BTItem {
+  int i, tab, j0, nsub, nseg;
+};
+__device__ __forceinline__ BTItem bt_item(const CJBatchArgs& a, int w, int h) {
+  BTItem it = {0, -1, 0, 0, 0};
+  if (w >= a.nwarps) return it;
+  it.i = bt_image_of_warp(a, w);
+  it.j0 = w * 32 - a.desc[it.i].sub0;
+  it.nsub = __ldcg(&a.st[it.i].nsub);
+  it.nseg = __ldcg(&a.st[it.i].nseg);
+  if (it.j0 < it.nsub && (!h || h < a.prm[it.i].bpm)) it.tab = __ldcg(&a.prm[it.i].tab);
+  return it;
 }
 
-__device__ __forceinline__ const CJSteps& bt_steps_of(const CJBatchArgs& a, const BTStaged& g, const CJSteps* tab,
-                                                      int i) {
-  return i == g.ia ? tab[0] : (i == g.ib ? tab[1] : a.prm[i].steps);
+// Speculative-decode tables of the sync and fix-up phases.  The 8 warps of an item
+// group work on consecutive warps of the batch, so they need the tables of a
+// few images, and of one if the images share their DHT contents, as files of
+// one encoder do.  The CTA keeps the tables of two images in shared memory
+// (`id`: which, -1: none) and serves its warps in rounds: stage what the first
+// waiting warp and the next one with other tables need (nothing when they are
+// there from an earlier group), and run f(tables) in the warps with either.
+// `tab`: the warp's table image, -1: no work.  Every thread calls it.
+struct BTTabs {
+  int want[BT_WARPS], id[2];
+};
+template <class F>
+__device__ __forceinline__ void bt_with_tables(const CJBatchArgs& a, BTTabs& s, CJSpecTab* slots, int tab, F f) {
+  if ((threadIdx.x & 31) == 0) s.want[threadIdx.x >> 5] = tab;
+  __syncthreads();
+  unsigned todo = 0;
+  for (int w = 0; w < BT_WARPS; w++) todo |= (s.want[w] >= 0 ? 1u : 0u) << w;
+  while (todo) {  // CTA-uniform
+    const int ta = s.want[__ffs(todo) - 1];
+    unsigned mask = 0;
+    int tb = -1;
+    for (int w = 0; w < BT_WARPS; w++) {
+      if (!((todo >> w) & 1)) continue;
+      const int t = s.want[w];
+      if (t != ta && tb < 0) tb = t;
+      if (t == ta || t == tb) mask |= 1u << w;
+    }
+    int sa = s.id[0] == ta ? 0 : (s.id[1] == ta ? 1 : -1);
+    int sb = tb < 0 ? -1 : (s.id[0] == tb ? 0 : (s.id[1] == tb ? 1 : -1));
+    const bool load_a = sa < 0, load_b = tb >= 0 && sb < 0;
+    if (load_a) sa = sb == 0 ? 1 : 0;
+    if (load_b) sb = 1 - sa;
+    if (load_a || load_b) {
+      __syncthreads();  // every thread has read the ids
+      // built by another CTA in this kernel: read from L2
+      for (int h = 0; h < 2; h++) {
+        if (!(h ? load_b : load_a)) continue;
+        const int4* src = reinterpret_cast<const int4*>(a.spec + (h ? tb : ta));
+        int4* dst = reinterpret_cast<int4*>(slots + (h ? sb : sa));
+        for (int k = threadIdx.x; k < (int)(sizeof(CJSpecTab) / 16); k += BT_THREADS) dst[k] = __ldcg(src + k);
+        if (threadIdx.x == 0) s.id[h ? sb : sa] = h ? tb : ta;
+      }
+      __syncthreads();
+    }
+    if (tab >= 0 && (tab == ta || tab == tb)) f(slots[tab == ta ? sa : sb]);
+    todo &= ~mask;
+    if (todo) __syncthreads();  // before a slot is overwritten
+  }
 }
 
 __constant__ uint8_t c_bt_zz[64] = CJ_ZIGZAG_INIT;  // zig-zag -> natural index
 
-// Phase 0: one CTA builds one image's CJScanParams (the device twin of
-// cj_build_huff + cj_fill_params).
-__device__ void bt_build_params(const CJImageHeader& h, CJScanParams& p) {
-  for (int e = threadIdx.x; e < 4 * (1 << CJ_FAST_BITS); e += blockDim.x) {
-    int slot = e >> CJ_FAST_BITS, f = e & ((1 << CJ_FAST_BITS) - 1);
-    uint16_t out = 0;
-    if (h.huff_mask & (1 << slot)) {
-      int code = 0, k = 0;
-      for (int l = 1; l <= CJ_FAST_BITS; l++) {
-        int n = h.counts[slot][l - 1];
-        int c = f >> (CJ_FAST_BITS - l);
-        if (c >= code && c < code + n) {
-          out = (uint16_t)((l << 8) | h.symbols[slot][k + c - code]);
-          break;
-        }
-        k += n;
-        code = (code + n) << 1;
-      }
-    }
-    p.huff[slot].fast[f] = out;
-  }
-  for (int e = threadIdx.x; e < 4 * 256; e += blockDim.x) p.huff[e >> 8].vals[e & 255] = h.symbols[e >> 8][e & 255];
-  if (threadIdx.x < 4) {
-    int slot = threadIdx.x;
+// Whether images x and y define the same Huffman tables in every slot that x
+// uses (every thread of the CTA calls it).
+__device__ __forceinline__ bool bt_same_tables(const CJImageHeader& x, const CJImageHeader& y) {
+  bool same = (x.huff_mask & ~y.huff_mask) == 0;
+  const uint32_t* cx = reinterpret_cast<const uint32_t*>(x.counts);
+  const uint32_t* cy = reinterpret_cast<const uint32_t*>(y.counts);
+  const uint32_t* sx = reinterpret_cast<const uint32_t*>(x.symbols);
+  const uint32_t* sy = reinterpret_cast<const uint32_t*>(y.symbols);
+  if (threadIdx.x < 16) same = same && (!(x.huff_mask >> (threadIdx.x >> 2) & 1) || cx[threadIdx.x] == cy[threadIdx.x]);
+  same = same && (!(x.huff_mask >> (threadIdx.x >> 6) & 1) || sx[threadIdx.x] == sy[threadIdx.x]);
+  return __syncthreads_and(same);
+}
+static_assert(BT_THREADS == 256, "one thread per symbol word");
+static_assert(offsetof(CJImageHeader, symbols) % 4 == 0, "symbol words");
+
+// Phase 0: one CTA builds one Huffman table slot of one image on the device --
+// the canonical table, its decode steps and its CJSpecTab entries -- in
+// shared memory, where every entry's searches are short, and copies them out.
+struct BTBuild {
+  CJHuff t;
+  uint16_t pri[1 << CJ_FAST_BITS];
+  uint8_t counts[16];
+  int pmin, pmax;
+};
+static_assert(sizeof(BTBuild) <= BT_DECODE_SMEM && sizeof(CJHuff) % 4 == 0, "table build space");
+__device__ void bt_build_slot(const CJImageHeader& h, CJScanParams& p, CJSpecTab& tb, int slot, BTBuild& s) {
+  const bool defined = (h.huff_mask >> slot) & 1, ac = slot >= 2;
+  if (threadIdx.x < 16) s.counts[threadIdx.x] = h.counts[slot][threadIdx.x];
+  s.t.vals[threadIdx.x] = h.symbols[slot][threadIdx.x];
+  __syncthreads();
+  if (threadIdx.x == 0) {  // cj_build_huff's canonical arrays
     int code = 0, k = 0;
-    p.huff[slot].maxcode[0] = -1;
-    p.huff[slot].valoff[0] = 0;
+    s.t.maxcode[0] = -1;
+    s.t.valoff[0] = 0;
     for (int l = 1; l <= 16; l++) {
-      int n = h.counts[slot][l - 1];
-      p.huff[slot].valoff[l] = k - code;
+      const int n = s.counts[l - 1];
+      s.t.valoff[l] = k - code;
       code += n;
       k += n;
-      p.huff[slot].maxcode[l] = n ? code - 1 : -1;
+      s.t.maxcode[l] = n ? code - 1 : -1;
       code <<= 1;
     }
-    p.huff[slot].maxcode[17] = -1;
-    p.huff[slot].valoff[17] = 0;
+    s.t.maxcode[17] = -1;
+    s.t.valoff[17] = 0;
   }
-  // decode steps from the finished canonical tables (cj_build_steps); the
-  // long-code prefix range of each slot is computed once
-  __shared__ int s_pre[4][2];
-  if (threadIdx.x < 4) {
-    int pmin = 1 << CJ_FAST_BITS, pmax = -1;
-    if (h.huff_mask & (1 << threadIdx.x)) cj_long_prefixes(h.counts[threadIdx.x], &pmin, &pmax);
-    s_pre[threadIdx.x][0] = pmin;
-    s_pre[threadIdx.x][1] = pmax;
+  if (threadIdx.x == 32) {
+    s.pmin = 1 << CJ_FAST_BITS;
+    s.pmax = -1;
+    if (defined) cj_long_prefixes(s.counts, &s.pmin, &s.pmax);
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < 4 * (1 << CJ_FAST_BITS); e += blockDim.x) {
-    const int slot = e >> CJ_FAST_BITS, f = e & ((1 << CJ_FAST_BITS) - 1);
-    const bool defined = (h.huff_mask & (1 << slot)) != 0;
-    p.steps.pri[slot][f] = defined ? cj_step_primary(p.huff[slot], s_pre[slot][0], s_pre[slot][1], f, slot >= 2)
-                                   : (uint16_t)CJ_STEP_BAD;
+  for (int f = threadIdx.x; f < (1 << CJ_FAST_BITS); f += blockDim.x) {
+    uint32_t e = 0;
+    for (int l = 1; defined && l <= CJ_FAST_BITS; l++) {
+      const int c = f >> (CJ_FAST_BITS - l);
+      if (c <= s.t.maxcode[l]) {
+        e = ((uint32_t)l << 8) | s.t.vals[(s.t.valoff[l] + c) & 255];
+        break;
+      }
+    }
+    s.t.fast[f] = (uint16_t)e;
+    const uint16_t st = defined ? cj_step_primary(s.t, s.pmin, s.pmax, f, ac) : (uint16_t)CJ_STEP_BAD;
+    s.pri[f] = st;
+    p.steps.pri[slot][f] = st;
   }
-  for (int e = threadIdx.x; e < 4 * CJ_STEP_SUBS * 64; e += blockDim.x) {
-    const int slot = e / (CJ_STEP_SUBS * 64), i = (e >> 6) % CJ_STEP_SUBS, j = e & 63;
-    const int pmin = s_pre[slot][0], pmax = s_pre[slot][1];
-    const bool used = (h.huff_mask & (1 << slot)) && pmin + i <= pmax;
-    p.steps.sub[slot][i][j] = used ? cj_step_sub(p.huff[slot], pmin, i, j, slot >= 2) : (uint16_t)CJ_STEP_BAD;
+  for (int e = threadIdx.x; e < CJ_STEP_SUBS * 64; e += blockDim.x) {
+    const int i = e >> 6, j = e & 63;
+    const uint16_t st = defined && s.pmin + i <= s.pmax ? cj_step_sub(s.t, s.pmin, i, j, ac) : (uint16_t)CJ_STEP_BAD;
+    p.steps.sub[slot][i][j] = st;
+    if (ac) tb.sub[slot - 2][i][j] = cj_spec_sub(st);
   }
-  __syncthreads();  // s_pre is reused by the next image of this CTA
+  __syncthreads();
+  for (int k = threadIdx.x; k < (int)(sizeof(CJHuff) / 4); k += blockDim.x)
+    reinterpret_cast<uint32_t*>(&p.huff[slot])[k] = reinterpret_cast<const uint32_t*>(&s.t)[k];
+  if (ac) {
+    for (int e = threadIdx.x; e < (1 << CJ_MULTI_BITS); e += blockDim.x) tb.acm[slot - 2][e] = cj_spec_acm(s.pri, e);
+    for (int e = threadIdx.x; e < (1 << CJ_FAST_BITS); e += blockDim.x) tb.ac1[slot - 2][e] = cj_spec_ac1(s.pri[e]);
+  } else {
+    for (int e = threadIdx.x; e < (1 << CJ_MULTI_DC_BITS); e += blockDim.x) tb.dc[slot][e] = cj_spec_dc(s.pri, e);
+  }
+  __syncthreads();  // s is reused by the CTA's next slot
+}
+
+// Phase 0: one CTA writes one image's geometry and quantisation tables (the
+// device twin of cj_fill_params); `tab`: the image whose tables serve it.
+__device__ void bt_build_params(const CJImageHeader& h, CJScanParams& p, int tab) {
   for (int e = threadIdx.x; e < 4 * 64; e += blockDim.x) p.qnat[e >> 6][c_bt_zz[e & 63]] = h.dq[e >> 6][e & 63];
   if (threadIdx.x < 64) p.zz[threadIdx.x] = c_bt_zz[threadIdx.x];
   if (threadIdx.x == 0) {
@@ -474,6 +586,7 @@ __device__ void bt_build_params(const CJImageHeader& h, CJScanParams& p) {
     p.nseg_expected = h.nseg_expected;
     p.total_blocks = h.total_blocks;
     p.phase_pack = cj_phase_pack(p);
+    p.tab = tab;
   }
 }
 
@@ -493,15 +606,26 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) k_decode_batch(CJBatchArgs a
   __shared__ int2 sm2[33];
   __shared__ uint8_t s_zz[64];
   __shared__ int s_grp, s_ok;
+  __shared__ BTTabs s_tabs;
+  __shared__ BTRank s_rank;
   unsigned gen = 0;
-  if (threadIdx.x == 0) gen = atomicAdd(&a.ctl->bar_gen, 0);
+  if (threadIdx.x == 0) {
+    gen = atomicAdd(&a.ctl->bar_gen, 0);
+    bt_rank_begin(a.ctl, s_rank);
+  }
   if (threadIdx.x < 64) s_zz[threadIdx.x] = c_bt_zz[threadIdx.x];
   const int lane = threadIdx.x & 31;
 
   bt_stamp(a.ctl, 0);
-  // ---- phase 0: tables + status
-  for (int i = blockIdx.x; i < a.n; i += gridDim.x) {
-    bt_build_params(a.hdr[i], a.prm[i]);
+  // ---- phase 0: tables + status, one item per image and table slot (a single
+  // image's four slots go to four CTAs).  An image whose DHT contents equal
+  // the reference image's is served by that image's tables.
+  for (int e = blockIdx.x; e < 4 * a.n; e += gridDim.x) {
+    const int i = e >> 2, slot = e & 3;
+    const int tab = i != a.tab_ref && bt_same_tables(a.hdr[i], a.hdr[a.tab_ref]) ? a.tab_ref : i;
+    if (tab == i) bt_build_slot(a.hdr[i], a.prm[i], a.spec[i], slot, *reinterpret_cast<BTBuild*>(smem));
+    if (slot) continue;
+    bt_build_params(a.hdr[i], a.prm[i], tab);
     if (threadIdx.x == 0) {
       CJStatus z;
       memset(&z, 0, sizeof(z));
@@ -543,6 +667,7 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) k_decode_batch(CJBatchArgs a
   }
   if (!bt_grid_sync(a.ctl, gen, a.wait_limit, &s_ok)) return;
 
+  if (threadIdx.x == 0) bt_rank_end(a.ctl, s_rank);
   bt_stamp(a.ctl, 2);
   // ---- phase 2: per-image tile offsets
   for (int i = blockIdx.x; i < a.n; i += gridDim.x) {
@@ -691,7 +816,10 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) k_decode_batch(CJBatchArgs a
   if (!bt_grid_sync(a.ctl, gen, a.wait_limit, &s_ok)) return;
 
   bt_stamp(a.ctl, 5);
-  CJSteps* tab = reinterpret_cast<CJSteps*>(smem);
+  CJSpecTab* tabs = reinterpret_cast<CJSpecTab*>(smem);
+  if (threadIdx.x < 2) s_tabs.id[threadIdx.x] = -1;  // (the first group's barrier orders it)
+  const CJSpecWarp& spw = reinterpret_cast<const CJSpecWarp*>(smem + BT_SPEC_OFF)[threadIdx.x >> 5];
+  uint32_t* hpp = reinterpret_cast<uint32_t*>(smem + BT_HPP_OFF) + (threadIdx.x >> 5) * a.nhyp * CJ_CKPTS * 32 + lane;
   // ---- phase 5a (latency-bound decodes only): MCU-phase hypotheses.  A
   // subsequence's guessed start (its first bit, MCU phase 0) lines up with
   // the true decode only after hundreds to thousands of bits for
@@ -699,44 +827,38 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) k_decode_batch(CJBatchArgs a
   // under the other phases usually does within a few blocks; the settle
   // below may join any of them at a checkpoint.  Items: (hypothesis, group
   // of BT_WARPS warps), each hypothesis's warps padded to whole groups.
-  const int nh = HYP && a.nhyp > 1 ? a.nhyp - 1 : 0;
-  if (HYP && nh) {
+  const int nh = a.nhyp - 1;
+  if constexpr (HYP) {
     const int nw8 = (a.nwarps + BT_WARPS - 1) / BT_WARPS * BT_WARPS;
+    bool first = true;
     for (;;) {
-      const int g0 = bt_next_group(&a.ctl->next_hyp, &s_grp);
+      const int g0 = bt_next_group(&a.ctl->next_hyp, &s_grp, s_rank.rank, first);
       if (g0 >= (nh + 1) * nw8) break;
       const int h = g0 / nw8, wg = g0 - h * nw8;  // hypothesis h = 0 .. nh (0: the usual guess)
       if (wg >= a.nwarps) continue;  // CTA-uniform
-      const BTStaged sg = bt_stage(a, wg, min(wg + BT_WARPS, a.nwarps) - 1, tab);
       const int w = wg + (int)(threadIdx.x >> 5);
-      if (w >= a.nwarps) continue;  // warp-uniform
-      const int i = bt_image_of_warp(a, w);
-      const CJImageDesc& d = a.desc[i];
-      const int nsub = __ldcg(&a.st[i].nsub), nseg = __ldcg(&a.st[i].nseg);
-      const int j0 = w * 32 - d.sub0;
-      if (j0 >= nsub) continue;  // warp-uniform
-      const CJScanParams& sp = a.prm[i];
-      if (h && h >= sp.bpm) continue;  // warp-uniform: no such phase in this image
-      CJLane ln = cj_lane(a.segs + d.seg0, nseg, nsub, j0 + lane, d.sub_bits);
-      // a segment's first subsequence starts exactly: phase 0 only.
-      // Hypothesis 0 is also the settle's starting record.
-      if (ln.active && (h == 0 || !ln.head)) {
-        const int64_t gs = d.sub0 + j0 + lane, hs = gs * 2 * (nh + 1) + h;
-        CJSubRec r;
-        r.start = cj_state(ln.begin, (uint32_t)h);
-        r.exit = r.start;
-        r.nblocks = r.dc[0] = r.dc[1] = r.dc[2] = 0;
+      const BTItem it = bt_item(a, w, h);
+      bt_with_tables(a, s_tabs, tabs, it.tab, [&](const CJSpecTab& tb) {
+        const CJImageDesc& d = a.desc[it.i];
+        const CJScanParams &sp = a.prm[it.i], &tp = a.prm[it.tab];
+        CJLane ln = cj_lane(a.segs + d.seg0, it.nseg, it.nsub, it.j0 + lane, d.sub_bits);
+        // a segment's first subsequence starts exactly: phase 0 only.
+        // Hypothesis 0 is also the settle's starting record.
+        const bool run = ln.active && (h == 0 || !ln.head);
+        const int64_t gs = d.sub0 + it.j0 + lane, hs = gs * 2 * (nh + 1) + h;
         CJCkpt* hc = cj_lane_ckpts(a.hckpt, hs);
-        r = cj_spec_decode<false>(sp, bt_steps_of(a, sg, tab, i),
-                                  reinterpret_cast<const uint32_t*>(a.data + d.data_off), ln, r.start, hc, r,
-                                  cj_ckpt_step(d.sub_bits));
-        a.hrecs[hs] = r;
-        if (h == 0) {
-          a.recs[gs] = r;
-          CJCkpt* ck = cj_lane_ckpts(a.ckpt, gs);
-          for (int k = 0; k < CJ_CKPTS; k++) ck[k] = hc[k];
+        CJSpecJob x;
+        cj_spec_job(x, sp, tp, tb, a.data + d.data_off, ln, hc, cj_ckpt_step(d.sub_bits), spw);
+        cj_spec_warp<true>(&x, run, cj_state(ln.begin, (uint32_t)h));
+        if (run) {
+          a.hrecs[hs] = x.r;
+          if (h == 0) {
+            a.recs[gs] = x.r;
+            CJCkpt* ck = cj_lane_ckpts(a.ckpt, gs);
+            for (int k = 0; k < CJ_CKPTS; k++) ck[k] = hc[k];
+          }
         }
-      }
+      });
     }
     if (!bt_grid_sync(a.ctl, gen, a.wait_limit, &s_ok)) return;
     // ---- phase 5b: probes.  Each subsequence decoded from each of its
@@ -745,87 +867,81 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) k_decode_batch(CJBatchArgs a
     // predecessor is known to end on that hypothesis, and the map entry
     // naming the hypothesis it ends on.  Items: (predecessor hypothesis,
     // group of BT_WARPS warps), as in phase 5a.
+    first = true;
     for (;;) {
-      const int g0 = bt_next_group(&a.ctl->next_probe, &s_grp);
+      const int g0 = bt_next_group(&a.ctl->next_probe, &s_grp, s_rank.rank, first);
       if (g0 >= (nh + 1) * nw8) break;
       const int p = g0 / nw8, wg = g0 - p * nw8;
       if (wg >= a.nwarps) continue;  // CTA-uniform
-      const BTStaged sg = bt_stage(a, wg, min(wg + BT_WARPS, a.nwarps) - 1, tab);
       const int w = wg + (int)(threadIdx.x >> 5);
-      if (w >= a.nwarps) continue;  // warp-uniform
-      const int i = bt_image_of_warp(a, w);
-      const CJImageDesc& d = a.desc[i];
-      const int nsub = __ldcg(&a.st[i].nsub), nseg = __ldcg(&a.st[i].nseg);
-      const int j0 = w * 32 - d.sub0;
-      if (j0 >= nsub) continue;  // warp-uniform
-      const CJScanParams& sp = a.prm[i];
-      const int nhi = min(nh, sp.bpm - 1);
-      CJLane ln = cj_lane(a.segs + d.seg0, nseg, nsub, j0 + lane, d.sub_bits);
-      const int64_t gs = d.sub0 + j0 + lane, hb = gs * 2 * (nh + 1);
-      uint8_t mk = 15;
-      const bool pred_head = ln.active && !ln.head && j0 + lane - 1 == a.segs[d.seg0 + ln.seg].first_sub;
-      if (ln.active && !ln.head && p <= (pred_head ? 0 : nhi)) {
+      const BTItem it = bt_item(a, w, 0);
+      bt_with_tables(a, s_tabs, tabs, it.tab, [&](const CJSpecTab& tb) {
+        const CJImageDesc& d = a.desc[it.i];
+        const CJScanParams &sp = a.prm[it.i], &tp = a.prm[it.tab];
+        const int nhi = min(nh, sp.bpm - 1);
+        CJLane ln = cj_lane(a.segs + d.seg0, it.nseg, it.nsub, it.j0 + lane, d.sub_bits);
+        const int64_t gs = d.sub0 + it.j0 + lane, hb = gs * 2 * (nh + 1);
+        uint8_t mk = 15;
+        const bool pred_head = ln.active && !ln.head && it.j0 + lane - 1 == a.segs[d.seg0 + ln.seg].first_sub;
+        const bool run = ln.active && !ln.head && p <= (pred_head ? 0 : nhi);
         CJCkpt* pc = cj_lane_ckpts(a.hckpt, hb + (nh + 1) + p);
-        for (int k = 0; k < CJ_CKPTS; k++) pc[k].pp = 0xFFFFFFFFu;  // matches no decode state
-        CJSubRec r;
-        r.start = r.exit = __ldcg(&a.hrecs[(gs - 1) * 2 * (nh + 1) + p].exit);
-        r.nblocks = r.dc[0] = r.dc[1] = r.dc[2] = 0;
-        r = cj_spec_decode<true, true>(sp, bt_steps_of(a, sg, tab, i),
-                                       reinterpret_cast<const uint32_t*>(a.data + d.data_off), ln, r.start, pc, r,
-                                       cj_ckpt_step(d.sub_bits), cj_lane_ckpts(a.hckpt, hb), a.hrecs + hb, nhi + 1);
-        a.hrecs[hb + (nh + 1) + p] = r;
-        for (int k = 0; k <= nhi; k++)
-          if (__ldcg(&a.hrecs[hb + k].exit) == r.exit) {
-            mk = (uint8_t)k;
-            break;
-          }
-      }
-      if (ln.active) a.hmap[gs * 16 + p] = mk;
+        CJSpecJob x;
+        cj_spec_job(x, sp, tp, tb, a.data + d.data_off, ln, pc, cj_ckpt_step(d.sub_bits), spw);
+        x.hck = cj_lane_ckpts(a.hckpt, hb);
+        x.hrec = a.hrecs + hb;
+        x.hpp = (uint32_t)__cvta_generic_to_shared(hpp);
+        x.nh = nhi + 1;
+        uint64_t from = 0;
+        if (run) {
+          from = __ldcg(&a.hrecs[(gs - 1) * 2 * (nh + 1) + p].exit);
+          cj_hyp_fill(hpp, x.hck, nhi + 1);
+        }
+        cj_spec_warp<true>(&x, run, from);
+        if (run) {
+          a.hrecs[hb + (nh + 1) + p] = x.r;
+          for (int k = 0; k <= nhi; k++)
+            if (__ldcg(&a.hrecs[hb + k].exit) == x.r.exit) {
+              mk = (uint8_t)k;
+              break;
+            }
+        }
+        if (ln.active) a.hmap[gs * 16 + p] = mk;
+      });
     }
     if (!bt_grid_sync(a.ctl, gen, a.wait_limit, &s_ok)) return;
   }
   // ---- phase 5: speculative decode + warp settle, in groups of BT_WARPS
   // consecutive warps per CTA (handed out dynamically) with staged tables
+  bool first = true;
   for (;;) {
-    const int g0 = bt_next_group(&a.ctl->next_sync, &s_grp);
+    const int g0 = bt_next_group(&a.ctl->next_sync, &s_grp, s_rank.rank, first);
     if (g0 >= a.nwarps) break;
-    const BTStaged sg = bt_stage(a, g0, min(g0 + BT_WARPS, a.nwarps) - 1, tab);
     const int w = g0 + (int)(threadIdx.x >> 5);
-    if (w >= a.nwarps) continue;  // warp-uniform
-    const int i = bt_image_of_warp(a, w);
-    const CJImageDesc& d = a.desc[i];
-    const int nsub = __ldcg(&a.st[i].nsub), nseg = __ldcg(&a.st[i].nseg);
-    const int j0 = w * 32 - d.sub0;
-    if (j0 >= nsub) continue;  // warp-uniform
-    const CJScanParams& sp = a.prm[i];
-    const CJSteps& T = bt_steps_of(a, sg, tab, i);
-    const uint32_t* words = reinterpret_cast<const uint32_t*>(a.data + d.data_off);
-    CJLane ln = cj_lane(a.segs + d.seg0, nseg, nsub, j0 + lane, d.sub_bits);
-    CJSubRec r;
-    r.start = cj_state(ln.begin, 0);
-    r.exit = r.start;
-    r.nblocks = r.dc[0] = r.dc[1] = r.dc[2] = 0;
-    CJCkpt* ck = cj_lane_ckpts(a.ckpt, d.sub0 + j0 + lane);
-    const uint32_t cs = cj_ckpt_step(d.sub_bits);
-    if constexpr (HYP) {
-      // The phase-0 decodes of phase 5a, settled with the probes of phase 5b
-      // (lane 0 keeps its guess until the fix-up passes)
-      if (nh) {
-        const int64_t gs = d.sub0 + j0 + lane;
-        const bool pred_head = ln.active && !ln.head && j0 + lane - 1 == a.segs[d.seg0 + ln.seg].first_sub;
-        if (ln.active) r = bt_load_rec(&a.recs[gs]);
-        bt_settle_map(a, sp, T, words, ln, pred_head, r, r.start, ck, cs, gs, min(nh, sp.bpm - 1));
+    const BTItem it = bt_item(a, w, 0);
+    bt_with_tables(a, s_tabs, tabs, it.tab, [&](const CJSpecTab& tb) {
+      const CJImageDesc& d = a.desc[it.i];
+      const CJScanParams &sp = a.prm[it.i], &tp = a.prm[it.tab];
+      CJLane ln = cj_lane(a.segs + d.seg0, it.nseg, it.nsub, it.j0 + lane, d.sub_bits);
+      const int64_t gs = d.sub0 + it.j0 + lane;
+      const uint64_t guess = cj_state(ln.begin, 0);
+      CJSpecJob x;
+      cj_spec_job(x, sp, tp, tb, a.data + d.data_off, ln, cj_lane_ckpts(a.ckpt, gs), cj_ckpt_step(d.sub_bits), spw);
+      x.r.start = x.r.exit = guess;
+      x.r.nblocks = x.r.dc[0] = x.r.dc[1] = x.r.dc[2] = 0;
+      if constexpr (HYP) {
+        // The phase-0 decodes of phase 5a, settled with the probes of phase 5b
+        // (lane 0 keeps its guess until the fix-up passes)
+        const bool pred_head = ln.active && !ln.head && it.j0 + lane - 1 == a.segs[d.seg0 + ln.seg].first_sub;
+        if (ln.active) x.r = bt_load_rec(&a.recs[gs]);
+        bt_settle_map(a, x, ln, pred_head, x.r.start, gs, min(nh, sp.bpm - 1), hpp);
       } else {
-        if (ln.active) r = cj_spec_decode<false>(sp, T, words, ln, r.start, ck, r, cs);
-        cj_warp_settle(sp, T, words, ln, r, r.start, ck, cs);
+        cj_spec_warp<false>(&x, ln.active, guess);
+        cj_warp_settle(x, ln, guess);
       }
-    } else {
-      if (ln.active) r = cj_spec_decode<false>(sp, T, words, ln, r.start, ck, r, cs);
-      cj_warp_settle(sp, T, words, ln, r, r.start, ck, cs);
-    }
-    if (ln.active) a.recs[d.sub0 + j0 + lane] = r;
-    unsigned act = __ballot_sync(CJ_FULL, ln.active);
-    if (lane == 31 - __clz(act)) a.snap0[w] = r.exit;
+      if (ln.active) a.recs[gs] = x.r;
+      unsigned act = __ballot_sync(CJ_FULL, ln.active);
+      if (lane == 31 - __clz(act)) a.snap0[w] = x.r.exit;
+    });
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     a.ctl->unstable[0] = 0;
@@ -845,28 +961,21 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) k_decode_batch(CJBatchArgs a
       a.ctl->unstable[(pass + 1) % 3] = 0;
       a.ctl->next_fix[(pass + 1) % 3] = 0;
     }
+    first = true;
     for (;;) {
-      const int g0 = bt_next_group(next, &s_grp);
+      const int g0 = bt_next_group(next, &s_grp, s_rank.rank, first);
       if (g0 >= a.nwarps) break;
       const int w = g0 + (int)(threadIdx.x >> 5);
-      bool work = w < a.nwarps;  // warp-uniform, like everything below
-      int i = 0, nsub = 0, nseg = 0, j0 = 0;
-      if (work) {
-        i = bt_image_of_warp(a, w);
-        nsub = __ldcg(&a.st[i].nsub);
-        nseg = __ldcg(&a.st[i].nseg);
-        j0 = w * 32 - a.desc[i].sub0;
-        if (j0 >= nsub) {
-          if (lane == 0) {
-            CJWarpAgg z;
-            memset(&z, 0, sizeof(z));
-            a.wagg[w] = z;
-          }
-          work = false;
-        }
+      const BTItem it = bt_item(a, w, 0);
+      const bool work = it.tab >= 0;  // warp-uniform, like everything below
+      if (!work && w < a.nwarps && lane == 0) {
+        CJWarpAgg z;
+        memset(&z, 0, sizeof(z));
+        a.wagg[w] = z;
       }
-      const CJImageDesc& d = a.desc[i];
-      CJLane ln = cj_lane(a.segs + d.seg0, nseg, work ? nsub : 0, j0 + lane, d.sub_bits);
+      const CJImageDesc& d = a.desc[it.i];
+      const int j0 = it.j0;
+      CJLane ln = cj_lane(a.segs + d.seg0, it.nseg, work ? it.nsub : 0, j0 + lane, d.sub_bits);
       CJSubRec r;
       if (ln.active) r = bt_load_rec(&a.recs[d.sub0 + j0 + lane]);
       else {
@@ -874,29 +983,26 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) k_decode_batch(CJBatchArgs a
         r.nblocks = r.dc[0] = r.dc[1] = r.dc[2] = 0;
       }
       const uint64_t in0 = (work && j0 > 0 && lane == 0) ? __ldcg(&snap_in[w - 1]) : r.start;
-      // the settle's first test; only a group with a lane to re-decode stages tables
+      // the settle's first test; only warps with a lane to re-decode need tables
       const uint64_t pred = __shfl_up_sync(CJ_FULL, r.exit, 1);
       const uint64_t want = ln.head ? r.start : (lane == 0 ? in0 : pred);
-      BTStaged sg = {-1, -1};
-      if (__syncthreads_or(ln.active && want != r.start)) sg = bt_stage(a, g0, min(g0 + BT_WARPS, a.nwarps) - 1, tab);
-      if (!work) continue;
-      const CJScanParams& sp = a.prm[i];
-      const uint32_t* words = reinterpret_cast<const uint32_t*>(a.data + d.data_off);
-      const CJSteps& T = bt_steps_of(a, sg, tab, i);
-      CJCkpt* ck = cj_lane_ckpts(a.ckpt, d.sub0 + j0 + lane);
-      const uint32_t cs = cj_ckpt_step(d.sub_bits);
-      bool moved;
-      if constexpr (HYP) {
-        if (nh) {
+      bool moved = false;
+      const bool redo = __any_sync(CJ_FULL, ln.active && want != r.start);
+      bt_with_tables(a, s_tabs, tabs, redo ? it.tab : -1, [&](const CJSpecTab& tb) {
+        const CJScanParams &sp = a.prm[it.i], &tp = a.prm[it.tab];
+        const int64_t gs = d.sub0 + j0 + lane;
+        CJSpecJob x;
+        cj_spec_job(x, sp, tp, tb, a.data + d.data_off, ln, cj_lane_ckpts(a.ckpt, gs), cj_ckpt_step(d.sub_bits), spw);
+        x.r = r;
+        if constexpr (HYP) {
           const bool pred_head = ln.active && !ln.head && j0 + lane - 1 == a.segs[d.seg0 + ln.seg].first_sub;
-          moved = bt_settle_map(a, sp, T, words, ln, pred_head, r, in0, ck, cs, (int64_t)(d.sub0 + j0 + lane),
-                                min(nh, sp.bpm - 1));
+          moved = bt_settle_map(a, x, ln, pred_head, in0, gs, min(nh, sp.bpm - 1), hpp);
         } else {
-          moved = cj_warp_settle(sp, T, words, ln, r, in0, ck, cs);
+          moved = cj_warp_settle(x, ln, in0);
         }
-      } else {
-        moved = cj_warp_settle(sp, T, words, ln, r, in0, ck, cs);
-      }
+        r = x.r;
+      });
+      if (!work) continue;
       if (moved && ln.active)
         a.recs[d.sub0 + j0 + lane] = r;
       unsigned act = __ballot_sync(CJ_FULL, ln.active);
@@ -991,7 +1097,8 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) k_decode_batch(CJBatchArgs a
     int16_t* wbuf = reinterpret_cast<int16_t*>(smem) + (threadIdx.x >> 5) * 32 * 64;
     for (int k = lane; k < 32 * 64 * 2 / 16; k += 32) reinterpret_cast<uint4*>(wbuf)[k] = make_uint4(0, 0, 0, 0);
     __syncwarp();
-    for (int t = bt_next_item(&a.ctl->next_write); t < nitems; t = bt_next_item(&a.ctl->next_write)) {
+    first = true;
+    for (int t = bt_next_item(&a.ctl->next_write, s_rank.rank, first); t < nitems; t = bt_next_item(&a.ctl->next_write, s_rank.rank, first)) {
       const int w = t / UNITS, part = t % UNITS;
       const int i = bt_image_of_warp(a, w);
       const CJImageDesc& d = a.desc[i];
@@ -1000,7 +1107,7 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) k_decode_batch(CJBatchArgs a
       const int j0 = w * 32 - d.sub0;
       if (j0 >= nsub) continue;
       const CJScanParams& sp = a.prm[i];
-      const CJSteps& T = sp.steps;
+      const CJScanParams& tp = a.prm[__ldcg(&sp.tab)];
       const uint32_t* words = reinterpret_cast<const uint32_t*>(a.data + d.data_off);
       // block / DC prefix of the 32 lanes of warp w (thread = lane `lane`)
       const CJLane lw = cj_lane(a.segs + d.seg0, nseg, nsub, j0 + lane, d.sub_bits);
@@ -1045,7 +1152,7 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) k_decode_batch(CJBatchArgs a
           end = cj_lane_write_end(ln, seg, r, lane_first);
         }
       }
-      cj_write_units_warp(sp, T, words, ln, seg, start, first, dc0, dc1, dc2, a.coef + d.coef0 * 64, st, s_zz, stop,
+      cj_write_units_warp(sp, tp, words, ln, seg, start, first, dc0, dc1, dc2, a.coef + d.coef0 * 64, st, s_zz, stop,
                           end, ln.active, wbuf);
     }
   }
@@ -1053,23 +1160,26 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) k_decode_batch(CJBatchArgs a
 
 typedef void (*bt_decode_fn)(CJBatchArgs);
 #define BT_DECODE_CTAS_DEFAULT 4
+// The hypothesis variant has one build, at the 3 CTAs per SM its shared
+// memory (the hypotheses' checkpoint positions) leaves room for.
+#define BT_HYP_CTAS 3
 static bt_decode_fn bt_decode_kernel(int ctas_per_sm, bool hyp = false) {
+  if (hyp) return k_decode_batch<BT_HYP_CTAS, true>;
   switch (ctas_per_sm) {
-    case 3: return hyp ? k_decode_batch<3, true> : k_decode_batch<3>;
-    case 5: return hyp ? k_decode_batch<5, true> : k_decode_batch<5>;
-    default: return hyp ? k_decode_batch<4, true> : k_decode_batch<4>;
+    case 3: return k_decode_batch<3>;
+    case 5: return k_decode_batch<5>;
+    default: return k_decode_batch<4>;
   }
 }
 
 // The decode kernels' dynamic shared memory is above the 48 KB a launch gets
 // without opting in.
 static cudaError_t bt_decode_attrs() {
-  const int bytes = (int)BT_DECODE_SMEM;
-  cudaError_t e = cudaSuccess;
+  cudaError_t e = cudaFuncSetAttribute((const void*)bt_decode_kernel(BT_HYP_CTAS, true),
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bt_decode_smem(BT_MAX_HYP));
   for (int c = 3; c <= 5 && e == cudaSuccess; c++)
-    for (int h = 0; h < 2 && e == cudaSuccess; h++)
-      e = cudaFuncSetAttribute((const void*)bt_decode_kernel(c, h != 0), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               bytes);
+    e = cudaFuncSetAttribute((const void*)bt_decode_kernel(c), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)bt_decode_smem(1));
   return e;
 }
 
@@ -1544,8 +1654,9 @@ struct CJBatch {
   // device buffers (grow-only)
   CJDevBuf hrecs, hckpt, hmap;  // MCU-phase hypotheses and probes of a latency-bound batch
   int nhyp = 1;
+  int tab_ref = 0;  // the image whose Huffman tables the others are compared with
   bool hyp_enabled = true;  // cjBatchSetHypotheses
-  CJDevBuf hdr, desc, prm, st, blob, data, tile_keep, tile_mark, mpos, mcode, segs, recs, ckpt, snap,
+  CJDevBuf hdr, desc, prm, spec, st, blob, data, tile_keep, tile_mark, mpos, mcode, segs, recs, ckpt, snap,
       wagg, carry, coef, out, ctl, fancy;  // fancy: planar samples of the fancy mode
   CJDevBuf p_size, p_hdr, p_map;           // device parse: file offsets + sizes, headers, image -> file
   // pinned host staging
@@ -1709,7 +1820,7 @@ void cjBatchDestroy(CJBatch* b) {
     CJDevBuf* bufs[] = {&b->hdr,  &b->desc, &b->prm,   &b->st,   &b->blob,  &b->data,
                         &b->tile_keep, &b->tile_mark, &b->mpos, &b->mcode, &b->segs,
                         &b->recs, &b->ckpt, &b->snap, &b->wagg, &b->carry, &b->coef, &b->out, &b->ctl,
-                        &b->fancy, &b->p_size, &b->p_hdr, &b->p_map, &b->hrecs, &b->hckpt, &b->hmap};
+                        &b->fancy, &b->spec, &b->p_size, &b->p_hdr, &b->p_map, &b->hrecs, &b->hckpt, &b->hmap};
     for (CJDevBuf* d : bufs)
       if (d->p) cudaFree(d->p);
     CJHostBuf* hb[] = {&b->h_hdr, &b->h_desc, &b->h_out, &b->h_st, &b->h_ctl, &b->h_psize, &b->h_pmap};
@@ -2030,6 +2141,10 @@ int cjBatchStage(CJBatch* b, int n, const unsigned char* blob, const int64_t* of
     nd++;
   }
   b->n_dev = nd;
+  // a colour image (both table pairs) can serve grey ones too
+  b->tab_ref = 0;
+  while (b->tab_ref < nd && hh[b->tab_ref].huff_mask != 15) b->tab_ref++;
+  if (b->tab_ref == nd) b->tab_ref = 0;
   b->ntiles = ntiles;
   b->nwarps = nsubw;
   b->nptiles = nptiles;
@@ -2044,7 +2159,7 @@ int cjBatchStage(CJBatch* b, int n, const unsigned char* blob, const int64_t* of
   if (!nd) return 0;
   size_t nd_ = (size_t)nd;
   if (bt_ensure(b, b->hdr, nd_ * sizeof(CJImageHeader)) || bt_ensure(b, b->desc, nd_ * sizeof(CJImageDesc)) ||
-      bt_ensure(b, b->prm, nd_ * sizeof(CJScanParams)) || bt_ensure(b, b->st, nd_ * sizeof(CJStatus)) ||
+      bt_ensure(b, b->prm, nd_ * sizeof(CJScanParams)) || bt_ensure(b, b->spec, nd_ * sizeof(CJSpecTab)) || bt_ensure(b, b->st, nd_ * sizeof(CJStatus)) ||
       bt_ensure(b, b->blob, (size_t)blob_bytes + 64) || bt_ensure(b, b->data, (size_t)data_bytes + 64) ||
       bt_ensure(b, b->tile_keep, (size_t)ntiles * 4) || bt_ensure(b, b->tile_mark, (size_t)ntiles * 4) ||
       bt_ensure(b, b->mpos, (size_t)nmark * 4) || bt_ensure(b, b->mcode, (size_t)nmark) ||
@@ -2096,16 +2211,18 @@ int cjBatchStage(CJBatch* b, int n, const unsigned char* blob, const int64_t* of
       maxbpm = std::max(maxbpm, bpm);
     }
     const int nh = std::min(maxbpm, BT_MAX_HYP);
-    int per_sm_hyp = 0;  // the hypothesis variant must fit the same cooperative grid
+    int per_sm_hyp = 0;
     CJ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                    &per_sm_hyp, (const void*)bt_decode_kernel(b->decode_ctas, true), BT_THREADS, b->smem),
+                    &per_sm_hyp, (const void*)bt_decode_kernel(b->decode_ctas, true), BT_THREADS, bt_decode_smem(nh)),
                 CUDA_KERNEL_LAUNCH_ERROR);
-    if (nh > 1 && per_sm_hyp * b->sm_count >= b->grid && (int64_t)nsubw * nh <= (int64_t)b->grid * BT_WARPS) {
+    if (nh > 1 && per_sm_hyp > 0 && (int64_t)nsubw * nh <= (int64_t)b->grid * BT_WARPS) {
       const size_t nsub = (size_t)nsubw * 32, nrec = nsub * 2 * nh;  // hypotheses and probes
       if (bt_ensure(b, b->hrecs, nrec * sizeof(CJSubRec)) || bt_ensure(b, b->hckpt, nrec * CJ_CKPTS * sizeof(CJCkpt)) ||
           bt_ensure(b, b->hmap, nsub * 16))
         return CUDA_MEM_ERROR;
       b->nhyp = nh;
+      b->smem = bt_decode_smem(nh);
+      b->grid = std::min(per_sm_hyp, BT_HYP_CTAS) * b->sm_count;
     }
   }
   const void* pk = (const void*)bt_pixel_kernel(b->idct, bt_pix_format(b));
@@ -2125,6 +2242,8 @@ static CJBatchArgs bt_args(const CJBatch* b) {
   a.hdr = (const CJImageHeader*)b->hdr.p;
   a.desc = (const CJImageDesc*)b->desc.p;
   a.prm = (CJScanParams*)b->prm.p;
+  a.spec = (CJSpecTab*)b->spec.p;
+  a.tab_ref = b->tab_ref;
   a.st = (CJStatus*)b->st.p;
   a.blob = (const uint8_t*)b->blob.p;
   a.data = (uint8_t*)b->data.p;
@@ -2560,7 +2679,8 @@ int cj_reader_decode(JPGReader* jpg, bool stage) {
     bt_plan_one(h, n, sub, &desc);
     const int nwarps = desc.sub_cap / 32;
     if (cj_dev_ensure(d->bhdr, sizeof(CJImageHeader)) || cj_dev_ensure(d->bdesc, sizeof(CJImageDesc)) ||
-        cj_dev_ensure(d->params, sizeof(CJScanParams)) || cj_dev_ensure(d->status, sizeof(CJStatus)) ||
+        cj_dev_ensure(d->params, sizeof(CJScanParams)) || cj_dev_ensure(d->spec, sizeof(CJSpecTab)) ||
+        cj_dev_ensure(d->status, sizeof(CJStatus)) ||
         cj_dev_ensure(d->raw, (size_t)n + 64) || cj_dev_ensure(d->data, (size_t)n + 64) ||
         cj_dev_ensure(d->tile_keep, (size_t)desc.ntiles * 4) || cj_dev_ensure(d->tile_mark, (size_t)desc.ntiles * 4) ||
         cj_dev_ensure(d->mpos, (size_t)desc.mark_cap * 4) || cj_dev_ensure(d->mcode, (size_t)desc.mark_cap) ||
@@ -2576,31 +2696,25 @@ int cj_reader_decode(JPGReader* jpg, bool stage) {
     // MCU-phase hypotheses when their decodes fit in one round of the grid
     // (one image leaves most of the GPU idle while its settle chains run)
     d->b_nhyp = 1;
-    d->b_ctas = BT_DECODE_CTAS_DEFAULT;
+    int cap_run = cap;  // co-resident CTAs of the variant that runs
     const int groups = (nwarps + BT_WARPS - 1) / BT_WARPS;
     if (nh > 1 && (int64_t)nwarps * nh <= (int64_t)cap * BT_WARPS) {
-      // the hypothesis variant must fit the cooperative grid: its 3-CTA
-      // build (no register spills) when the grid allows, else the 4-CTA one
-      const int grid_h = std::max(1, std::min(cap, std::max(desc.ntiles, groups * nh)));
-      int per3 = 0, per4 = 0;
-      CJ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per3, (const void*)bt_decode_kernel(3, true),
-                                                                BT_THREADS, BT_DECODE_SMEM),
+      int per_hyp = 0;
+      CJ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_hyp, (const void*)bt_decode_kernel(BT_HYP_CTAS, true),
+                                                                BT_THREADS, bt_decode_smem(nh)),
                   CUDA_KERNEL_LAUNCH_ERROR);
-      CJ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                      &per4, (const void*)bt_decode_kernel(BT_DECODE_CTAS_DEFAULT, true), BT_THREADS, BT_DECODE_SMEM),
-                  CUDA_KERNEL_LAUNCH_ERROR);
-      const int ctas = per3 * sms >= grid_h ? 3 : (per4 * sms >= grid_h ? BT_DECODE_CTAS_DEFAULT : 0);
-      if (ctas) {
+      if (per_hyp > 0) {
         const size_t nsub = (size_t)desc.sub_cap, nrec = nsub * 2 * nh;  // hypotheses and probes
         if (cj_dev_ensure(d->hrecs, nrec * sizeof(CJSubRec)) ||
             cj_dev_ensure(d->hckpt, nrec * CJ_CKPTS * sizeof(CJCkpt)) || cj_dev_ensure(d->hmap, nsub * 16))
           return CUDA_MEM_ERROR;
         d->b_nhyp = nh;
-        d->b_ctas = ctas;
+        cap_run = std::min(per_hyp, BT_HYP_CTAS) * sms;
       }
     }
-    const int work = std::max(desc.ntiles, groups * d->b_nhyp);
-    d->b_grid = std::max(1, std::min(cap, work));
+    // (at least one CTA per SM: work items go to different SMs first)
+    const int work = std::max(std::max(desc.ntiles, groups * d->b_nhyp), sms);
+    d->b_grid = std::max(1, std::min(cap_run, work));
     d->b_ntiles = desc.ntiles;
     d->b_nwarps = nwarps;
     d->b_nptiles = desc.nptiles;
@@ -2621,6 +2735,7 @@ int cj_reader_decode(JPGReader* jpg, bool stage) {
   a.hdr = (const CJImageHeader*)d->bhdr.p;
   a.desc = (const CJImageDesc*)d->bdesc.p;
   a.prm = (CJScanParams*)d->params.p;
+  a.spec = (CJSpecTab*)d->spec.p;
   a.st = (CJStatus*)d->status.p;
   a.blob = (const uint8_t*)d->raw.p;
   a.data = (uint8_t*)d->data.p;
@@ -2649,9 +2764,9 @@ int cj_reader_decode(JPGReader* jpg, bool stage) {
   cj_profile_begin(d);
   CJ_CUDA_TRY(cudaMemsetAsync(d->bctl.p, 0, sizeof(CJBatchCtl), s), CUDA_MEM_ERROR);
   void* args[] = {&a};
-  CJ_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)bt_decode_kernel(d->b_ctas, d->b_nhyp > 1),
+  CJ_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)bt_decode_kernel(BT_DECODE_CTAS_DEFAULT, d->b_nhyp > 1),
                                           dim3(d->b_grid),
-                                          dim3(BT_THREADS), args, BT_DECODE_SMEM, s),
+                                          dim3(BT_THREADS), args, bt_decode_smem(d->b_nhyp), s),
               CUDA_KERNEL_LAUNCH_ERROR);
   cj_after_launch(d, CJ_K_DECODE_BATCH);
   CJ_CUDA_TRY(cudaEventRecord(d->ev_scan, s), CUDA_KERNEL_LAUNCH_ERROR);
@@ -2677,7 +2792,8 @@ int cj_reader_decode_status(const JPGReader* jpg) {
 // memory.  The array is held by every GPU that loads the library until the
 // process exits.
 
-#define CJ_NOALLOC_SCRATCH_BYTES (24u << 20)  // 24 MiB per device
+// 24 MiB per device, and room for the speculative-decode tables
+#define CJ_NOALLOC_SCRATCH_BYTES ((24u << 20) + (32u << 10))
 #define CJ_NOALLOC_MAX_DEVICES 64
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[CJ_NOALLOC_SCRATCH_BYTES];
@@ -2760,7 +2876,7 @@ extern "C" int cjDecodeNoAlloc(const unsigned char* jpeg, size_t size, unsigned 
     return o;
   };
   const size_t o_hdr = carve(sizeof(CJImageHeader)), o_desc = carve(sizeof(CJImageDesc));
-  const size_t o_prm = carve(sizeof(CJScanParams)), o_st = carve(sizeof(CJStatus));
+  const size_t o_prm = carve(sizeof(CJScanParams)), o_st = carve(sizeof(CJStatus)), o_spec = carve(sizeof(CJSpecTab));
   const size_t o_ctl = carve(sizeof(CJBatchCtl));
   const size_t o_blob = carve(size + 64), o_data = carve((size_t)scan_len + 64);
   const size_t o_tk = carve((size_t)d.ntiles * 4), o_tm = carve((size_t)d.ntiles * 4);
@@ -2803,6 +2919,7 @@ extern "C" int cjDecodeNoAlloc(const unsigned char* jpeg, size_t size, unsigned 
   a.hdr = (const CJImageHeader*)(base + o_hdr);
   a.desc = (const CJImageDesc*)(base + o_desc);
   a.prm = (CJScanParams*)(base + o_prm);
+  a.spec = (CJSpecTab*)(base + o_spec);
   a.st = (CJStatus*)(base + o_st);
   a.blob = base + o_blob;
   a.data = base + o_data;
@@ -2825,6 +2942,7 @@ extern "C" int cjDecodeNoAlloc(const unsigned char* jpeg, size_t size, unsigned 
   a.nwarps = nwarps;
   a.nptiles = d.nptiles;
   a.max_passes = nwarps + 2;
+  a.nhyp = 1;
   a.wait_limit = 0;
 
   // From the first queued copy on, every return waits for the stream: the

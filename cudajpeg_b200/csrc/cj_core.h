@@ -62,6 +62,36 @@ struct CJSteps {
   uint16_t sub[4][CJ_STEP_SUBS][64];
 };
 
+// Tables of the speculative decode (which needs positions and DC sums, not AC
+// values), in shared memory.  One 16-bit entry:
+//   bits 0-4   bits consumed (codes and magnitudes)
+//   bits 5-8   DC: the magnitude size; long code: its row in `sub`
+//   bits 9-15  advance of the zig-zag position (DC 1, from -1 to 0; an EOB or an
+//              invalid code adds 63, in a DC table 64); 0: the first 10 bits of
+//              a longer code, decoded on from its row by the next 6 bits
+// CJ_SPEC_FAR (nothing consumed, the position past every other): decode the
+// symbol through the CJSteps in memory -- DC codes of more than 9 bits and AC
+// tables with more long-code prefixes than rows.
+//   acm  every whole symbol the next CJ_MULTI_BITS bits determine, as one entry,
+//        while they advance by at most 16 together (an EOB after at most 15):
+//        up to position CJ_MULTI_MAXK no symbol of an entry can lie behind the
+//        block's end, so an entry is always taken whole
+//   ac1  one symbol (positions above CJ_MULTI_MAXK)
+// An 11-bit window holds 1.5 symbols on average at high bit rates and more
+// than two at low ones.
+#define CJ_MULTI_BITS 11
+#define CJ_MULTI_DC_BITS 9
+#define CJ_MULTI_MAXK 47
+#define CJ_SPEC_FAR (127u << 9)
+#define CJ_SPEC_FARK 126  // positions from here on: a CJ_SPEC_FAR entry (the rest end at 62 + 63)
+#define CJ_SPEC_EOB 63u
+struct CJSpecTab {
+  uint16_t acm[2][1 << CJ_MULTI_BITS];
+  uint16_t ac1[2][1 << CJ_FAST_BITS];
+  uint16_t dc[2][1 << CJ_MULTI_DC_BITS];
+  uint16_t sub[2][CJ_STEP_SUBS][64];
+};
+
 // Per-scan parameters, built on the host after SOS and copied once.
 struct alignas(16) CJScanParams {
   CJHuff huff[4];                 // DC0, DC1, AC0, AC1
@@ -84,6 +114,7 @@ struct alignas(16) CJScanParams {
   // phases 0..bpm-1 of an MCU, 6 bits each: component | DC slot << 2 |
   // AC slot << 4 (valid when bpm <= 10, the standard's limit)
   uint64_t phase_pack;
+  int32_t tab;  // batch: the image whose decode tables serve this one (the same DHT contents)
 };
 
 // Component and DC / AC table slots of MCU phase m.
@@ -235,6 +266,46 @@ CJ_HD uint32_t cj_step(const CJSteps& T, const CJScanParams& sp, uint32_t slot, 
 }
 CJ_HD uint32_t cj_step(const CJScanParams& sp, uint32_t slot, uint32_t v) { return cj_step(sp.steps, sp, slot, v); }
 
+
+// Entries of the CJSpecTab from the decode steps: a step, a primary entry of an
+// AC table, entry of a subtable.
+CJ_HD uint16_t cj_spec_entry(uint32_t st, uint32_t behind, bool dc = false) {
+  const uint32_t dk = (st >> 5) & 127;
+  return (uint16_t)(((st & 31) - behind) | ((st >> 12) << 5) | ((dk >= CJ_STEP_EOB ? CJ_SPEC_EOB + dc : dk) << 9));
+}
+CJ_HD uint16_t cj_spec_ac1(uint32_t st) {
+  if (st & 31) return cj_spec_entry(st, 0);
+  return (st >> 5) == CJ_STEP_SEARCH ? (uint16_t)CJ_SPEC_FAR : (uint16_t)(CJ_FAST_BITS | ((st >> 5) << 5));
+}
+CJ_HD uint16_t cj_spec_sub(uint32_t st) {
+  return cj_spec_entry(st, (st & 31) > CJ_FAST_BITS ? CJ_FAST_BITS : 0);  // (no code: 1 bit)
+}
+// The multi-symbol entry for the CJ_MULTI_BITS bits `idx` of an AC slot, from
+// its primary step table.  Bits past the window read as 0 below, but a code
+// after the first is taken only if it lies inside the window (its magnitude
+// may reach past).
+CJ_HD uint16_t cj_spec_acm(const uint16_t* pri, uint32_t idx) {
+  const uint32_t v = idx << (32 - CJ_MULTI_BITS);
+  uint32_t st = pri[v >> (32 - CJ_FAST_BITS)];
+  if (!(st & 31) || ((st >> 5) & 127) > 16) return cj_spec_ac1(st);
+  uint32_t used = st & 31, adv = (st >> 5) & 127;
+  while (used < CJ_MULTI_BITS) {
+    st = pri[(v << used) >> (32 - CJ_FAST_BITS)];
+    const uint32_t total = st & 31, dk = (st >> 5) & 127, len = total - (st >> 12);
+    if (!total || used + len > CJ_MULTI_BITS || used + total > 31) break;
+    if (dk == CJ_STEP_EOB && adv <= 15) return (uint16_t)((used + total) | ((CJ_SPEC_EOB + adv) << 9));
+    if (adv + dk > 16) break;
+    used += total;
+    adv += dk;
+  }
+  return (uint16_t)(used | (adv << 9));
+}
+// The entry for the CJ_MULTI_DC_BITS bits `idx` of a DC slot.
+CJ_HD uint16_t cj_spec_dc(const uint16_t* pri, uint32_t idx) {
+  const uint32_t st = pri[2 * idx];
+  static_assert(CJ_FAST_BITS == CJ_MULTI_DC_BITS + 1, "two primary entries per DC entry");
+  return (st & 31) && st == pri[2 * idx + 1] ? cj_spec_entry(st, 0, true) : (uint16_t)CJ_SPEC_FAR;
+}
 
 // Sign extension of a `size`-bit magnitude category value (T.81 F.2.2.1).
 CJ_HD int32_t cj_extend(uint32_t bits, uint32_t size) {

@@ -4,6 +4,7 @@
 // coefficient write-out.
 #pragma once
 #include <limits.h>
+#include <stddef.h>
 #include <stdint.h>
 
 #include "cj_core.h"
@@ -138,6 +139,106 @@ __device__ __forceinline__ CJLane cj_lane(const CJSegment* segs, int nseg, int n
   return l;
 }
 
+// Shared memory by its 32-bit address: the decode loops are not inlined, and a
+// pointer passed to them would be accessed as a generic one.  cj_tab16 reads a
+// table that does not change while the loop runs, so it may be scheduled
+// freely.
+__device__ __forceinline__ uint32_t cj_lds32(uint32_t a) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ uint32_t cj_tab16(uint32_t a) {
+  uint16_t v;
+  asm("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ void cj_sts32(uint32_t a, uint32_t v) {
+  asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+
+// Bit window of a lane in the warp-synchronous decode loops.  A lane's
+// stream runs through a ring of CJ_RING_WORDS big-endian words in shared
+// memory (word w in slot w mod CJ_RING_WORDS, `col` + 128 bytes per slot: one
+// bank per lane, so every access is conflict-free at any progress of the
+// lanes).  The current and the next word are in registers and the one after
+// them is read a symbol ahead, without branches: a symbol's chain is a funnel
+// shift, the table lookup, the position update and two selects.  Global memory
+// is touched only in refill(), which the whole warp runs together once per
+// CJ_RING_ROUNDS rounds of the loop: a 16-byte chunk fetched there has until
+// the next refill to arrive.
+// Bytes at or past `end_byte` read as 0xFF (the padding the reference's bit
+// reader supplies); memory past them is not relied on.
+#define CJ_RING_WORDS 16
+#define CJ_STEPS_PER_ROUND 3
+// rounds per refill: a round is three symbols of at most 31 bits, so three
+// rounds cross at most 9 words; 9 + 2 read ahead + 3 of the oldest chunk < 16
+#define CJ_RING_ROUNDS 3
+struct CJWin {
+  const uint4* chunks;    // the image's destuffed data, 16-byte aligned
+  uint32_t col;           // this lane's ring column (shared address)
+  uint32_t end_byte, cb;  // chunks cb .. cb + 3 are in the ring, cb + 4 in pf
+  uint4 pf;
+  uint32_t cur, nxt, nn, pos;  // words pos / 32, + 1, + 2; the next bit
+
+  __device__ __forceinline__ uint4 load(uint32_t c) const {
+    return 16u * c < end_byte ? chunks[c] : make_uint4(0, 0, 0, 0);
+  }
+  __device__ __forceinline__ void put(uint32_t c, uint4 v) {
+    uint32_t w[4] = {cj_bswap(v.x), cj_bswap(v.y), cj_bswap(v.z), cj_bswap(v.w)};
+    const uint32_t first = 16u * c;
+    if (first + 16 > end_byte) {  // the last chunks of a segment
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const int valid = (int)(end_byte - first) - 4 * i;  // data bytes of word i
+        if (valid <= 0) w[i] = 0xFFFFFFFFu;
+        else if (valid < 4) w[i] |= 0xFFFFFFFFu >> (8 * valid);
+      }
+    }
+    const uint32_t o = col + 128 * ((4 * c) & (CJ_RING_WORDS - 1));
+#pragma unroll
+    for (int i = 0; i < 4; i++) cj_sts32(o + 128 * i, w[i]);
+  }
+  // word pos / 32 + ahead
+  __device__ __forceinline__ uint32_t word(uint32_t ahead) const {
+    return cj_lds32(col + (((pos + 32 * ahead) << 2) & (128 * (CJ_RING_WORDS - 1))));
+  }
+  __device__ __forceinline__ void init(const uint4* data, uint32_t ring_col, uint32_t eb, uint32_t p) {
+    chunks = data;
+    col = ring_col;
+    end_byte = eb;
+    cb = p >> 7;
+    uint4 v[CJ_RING_WORDS / 4];
+#pragma unroll
+    for (int i = 0; i < CJ_RING_WORDS / 4; i++) v[i] = load(cb + i);
+    pf = load(cb + CJ_RING_WORDS / 4);
+#pragma unroll
+    for (int i = 0; i < CJ_RING_WORDS / 4; i++) put(cb + i, v[i]);
+    pos = p;
+    cur = word(0);
+    nxt = word(1);
+    nn = word(2);
+  }
+  // Replace the chunks the window has left behind.
+  __device__ __forceinline__ void refill() {
+    while ((pos >> 7) > cb) {
+      put(cb + CJ_RING_WORDS / 4, pf);
+      cb++;
+      pf = load(cb + CJ_RING_WORDS / 4);
+    }
+  }
+  __device__ __forceinline__ uint32_t peek() const { return __funnelshift_l(nxt, cur, pos); }
+  // u <= 31: at most one word is crossed
+  __device__ __forceinline__ void skip(uint32_t u) {
+    const uint32_t np = pos + u;
+    const bool cross = ((pos ^ np) & 32) != 0;
+    cur = cross ? nxt : cur;
+    nxt = cross ? nn : nxt;
+    pos = np;
+    nn = word(2);
+  }
+};
+
 // Bit reader of the decode loops: the current and the next big-endian word
 // and a bit offset; a 32-bit window is one funnel shift, and a word boundary
 // is crossed at most once per symbol (a symbol consumes at most 31 bits).
@@ -209,89 +310,156 @@ struct CJCkpt {
   int32_t nb, d0, d1, d2;
 };
 
-// Speculative decode of one subsequence from `start`: blocks beginning
+// The decode under way joined an earlier decode of the same subsequence: the
+// two coincide from the block boundary at checkpoint `j` on.
+struct CJJoin {
+  int j;    // CJ_CKPTS: no join
+  int src;  // -1: the lane's own previous decode, else hypothesis src
+};
+
+// Speculative decode of one subsequence per lane, from `start`, by a whole
+// warp (lanes with run = false take part in the votes only): blocks beginning
 // before the subsequence's end, their DC sums, and the state after them.
-// One Huffman symbol per iteration through the decode-step tables (CJSteps):
-// bits consumed, zig-zag advance and magnitude size come from one lookup, so
-// DC and AC symbols of all lanes take the same instructions; a block ends
-// when the position passes 62 (EOB and invalid symbols advance by >= 64).
-// The DC symbol's window is kept and its difference added when the block
-// ends.  Symbol for symbol this is the serial T.81 block decode
-// (src/decodeScanGPU.cu:78-100): a failing block is counted and
-// decoding goes on after the bits the failing symbol consumed.
+//
+// The loop is straight-line code over the tables of CJSpecTab: a divergent
+// branch costs some 40 cycles whether one lane takes it or all, and with 32
+// lanes at different symbols every branch is taken by some lane in almost
+// every step (measured: 870 cycles per symbol with branches for word
+// crossings, long codes and block ends, against about 60 for the symbol's
+// dependent instructions alone).  So word crossings are selects, a long code
+// is two steps (its prefix entry makes its subtable the next step's table), a
+// lane whose block has ended consumes nothing, and the end of blocks is one
+// branch per round of three steps.  The DC entry and window are kept and the
+// difference added when the block ends.  On a valid stream this is the serial
+// T.81 block decode (src/decodeScanGPU.cu:78-100) symbol for symbol; after a
+// symbol that fails, the block is counted and decoding goes on behind it (the
+// write-out reports the block).
 //
 // Checkpoints (`ck`, CJ_CKPTS of them) are written for every decode.  A
-// re-decode (RESUME) from a corrected start compares each checkpoint it
-// reaches with the previous decode's (`old`): when position and phase agree
-// the two decodes are identical from there on, so it stops and returns the
+// re-decode (`resume`) from a corrected start compares each checkpoint it
+// reaches with those of the previous decode `x.r`: when position and phase agree
+// the two decodes are identical from there on, so it stops and takes the
 // previous totals shifted by the difference in blocks and DC sums before that
 // point (shifting the later checkpoints too).  The result equals a full
-// decode from `start`.
-template <bool RESUME, bool HYP = false>
-__device__ __forceinline__ CJSubRec cj_spec_decode(const CJScanParams& sp, const CJSteps& T,
-                                                   const uint32_t* words, const CJLane& ln, uint64_t start,
-                                                   CJCkpt* __restrict__ ck,
-                                                   const CJSubRec& old, uint32_t cstep,
-                                                   const CJCkpt* hck = nullptr, const CJSubRec* hrec = nullptr,
-                                                   int nh = 0) {
-  CJFBits br;
-  br.init(words, ln.end_byte, cj_state_bit(start));
-  uint32_t m = cj_state_phase(start);
-  const int bpm = sp.bpm;
-  const uint64_t pack = sp.phase_pack;
-  int c;
-  uint32_t aslot, slot;
-  cj_phase(sp, bpm, pack, m, c, slot, aslot);
-  int k = -1, nb = 0, d0 = 0, d1 = 0, d2 = 0;
-  uint32_t dcv = 0, dcst = 0;
-  const uint32_t endrel = (uint32_t)(ln.end - ln.begin);
-  int rem = (int)((int64_t)ln.end - (int64_t)cj_state_bit(start));
-  uint32_t j = 0, thresh = cstep;
+// decode from `start`.  HYP: the same test against the `nh` hypothesis decodes
+// of the subsequence, whose checkpoint positions lie in shared memory (`hpp`,
+// column of cj_hyp_fill).  The tests read registers and shared memory only and
+// the totals of all joined lanes are taken together after the loop: lanes
+// reach their checkpoints at different steps, so a global load there would
+// stall the warp once per lane and checkpoint.
+// A warp's shared memory in the speculative decode: its ring, and per MCU
+// phase the shared addresses of the phase's tables (x: dc | acm << 16), then
+// ac1, the component << 16 and the next phase << 24 (y).
+struct CJSpecWarp {
+  uint32_t ring[CJ_RING_WORDS][32];
+  uint2 phase[CJ_MAX_BPM];
+};
+
+// One lane's part of a decode: where and how (all lanes of the warp agree on
+// sp, tp, tab), and its record in and out.
+struct CJSpecJob {
+  const CJScanParams *sp, *tp;
+  const uint4* data;
+  uint32_t tab, ring, phase, hpp;  // shared addresses: CJSpecTab, ring column, phase entries, hypothesis column
+  uint32_t begin, end, end_byte, cstep;
+  int nh;
+  bool resume;  // r and ck hold an earlier decode of the subsequence
+  CJCkpt* ck;
+  const CJCkpt* hck;
+  const CJSubRec* hrec;
   CJSubRec r;
-  r.start = start;
-  // Checkpoints at the boundary `rel` bits into the subsequence; true when
-  // this decode has joined the previous one (r then holds the result).
-  auto checkpoint = [&](uint32_t rel, bool final) -> bool {
-    while (j < CJ_CKPTS && (final || rel >= thresh)) {
-      const uint32_t pp = (m << 24) | rel;
-      if (RESUME && !final) {
-        // checkpoints may have been written by another SM in an earlier pass
-        // of the same kernel: read them from L2, never a stale L1 line
-        if (__ldcg(&ck[j].pp) == pp) {
-          const int dn = nb - __ldcg(&ck[j].nb), e0 = d0 - __ldcg(&ck[j].d0), e1 = d1 - __ldcg(&ck[j].d1),
-                    e2 = d2 - __ldcg(&ck[j].d2);
-          for (uint32_t q = j; q < CJ_CKPTS; q++) {
-            ck[q].nb = __ldcg(&ck[q].nb) + dn;
-            ck[q].d0 = __ldcg(&ck[q].d0) + e0;
-            ck[q].d1 = __ldcg(&ck[q].d1) + e1;
-            ck[q].d2 = __ldcg(&ck[q].d2) + e2;
-          }
-          r.exit = old.exit;
-          r.nblocks = old.nblocks + dn;
-          r.dc[0] = old.dc[0] + e0;
-          r.dc[1] = old.dc[1] + e1;
-          r.dc[2] = old.dc[2] + e2;
-          return true;
-        }
-        // the same test against the decodes of the subsequence from its
-        // first bit under the other MCU phases (hypotheses): equal position
-        // and phase at a block boundary mean the two decodes coincide from
-        // there on, so this decode takes that path's totals and checkpoints
-        for (int h = 0; HYP && h < nh; h++) {
-          const CJCkpt* hc = hck + h * CJ_CKPTS;
-          if (__ldcg(&hc[j].pp) != pp) continue;
-          const int dn = nb - __ldcg(&hc[j].nb), e0 = d0 - __ldcg(&hc[j].d0), e1 = d1 - __ldcg(&hc[j].d1),
-                    e2 = d2 - __ldcg(&hc[j].d2);
-          for (uint32_t q = j; q < CJ_CKPTS; q++)
-            ck[q] = CJCkpt{__ldcg(&hc[q].pp), __ldcg(&hc[q].nb) + dn, __ldcg(&hc[q].d0) + e0,
-                           __ldcg(&hc[q].d1) + e1, __ldcg(&hc[q].d2) + e2};
-          r.exit = __ldcg(&hrec[h].exit);
-          r.nblocks = __ldcg(&hrec[h].nblocks) + dn;
-          r.dc[0] = __ldcg(&hrec[h].dc[0]) + e0;
-          r.dc[1] = __ldcg(&hrec[h].dc[1]) + e1;
-          r.dc[2] = __ldcg(&hrec[h].dc[2]) + e2;
-          return true;
-        }
+};
+__device__ __forceinline__ void cj_spec_job(CJSpecJob& x, const CJScanParams& sp, const CJScanParams& tp,
+                                            const CJSpecTab& tab, const void* data, const CJLane& ln, CJCkpt* ck,
+                                            uint32_t cstep, const CJSpecWarp& sw) {
+  x.sp = &sp;
+  x.tp = &tp;
+  x.tab = (uint32_t)__cvta_generic_to_shared(&tab);
+  x.data = reinterpret_cast<const uint4*>(data);
+  x.begin = (uint32_t)ln.begin;
+  x.end = (uint32_t)ln.end;
+  x.end_byte = (uint32_t)ln.end_byte;
+  x.ck = ck;
+  x.cstep = cstep;
+  x.ring = (uint32_t)__cvta_generic_to_shared(sw.ring) + 4 * (threadIdx.x & 31);
+  x.phase = (uint32_t)__cvta_generic_to_shared(sw.phase);
+  x.nh = 0;
+  x.resume = false;
+}
+
+// Not inlined: in a function of its own the loop has the kernel's whole
+// register budget, and the phases around it keep their state across the call
+// in local memory instead of squeezing the loop (550 bytes of spills, some in
+// the loop, when inlined at 64 registers).
+template <bool HYP>
+__device__ __noinline__ void cj_spec_warp(CJSpecJob* job, bool run, uint64_t start) {
+  CJSpecJob& x = *job;
+  CJWin br;
+  const uint32_t begin = x.begin, end = x.end, cstep = x.cstep, phases = x.phase;
+  CJCkpt* const ck = x.ck;
+  const int bpm = x.sp->bpm;
+  {  // the phase entries of this image and these tables
+    const int i = threadIdx.x & 31;
+    __syncwarp();
+    if (i < bpm) {
+      const uint32_t c = x.sp->phase_comp[i], d = x.sp->comp_dc[c], a = x.sp->comp_ac[c] - 2u;
+      const uint32_t dc = x.tab + (uint32_t)offsetof(CJSpecTab, dc) + d * (uint32_t)sizeof(CJSpecTab::dc[0]);
+      const uint32_t ac1 = x.tab + (uint32_t)offsetof(CJSpecTab, ac1) + a * (uint32_t)sizeof(CJSpecTab::ac1[0]);
+      const uint32_t acm = x.tab + a * (uint32_t)sizeof(CJSpecTab::acm[0]);
+      cj_sts32(phases + 8 * i, dc | (acm << 16));
+      cj_sts32(phases + 8 * i + 4, ac1 | (c << 16) | ((i + 1 == bpm ? 0u : (uint32_t)i + 1) << 24));
+    }
+    __syncwarp();
+  }
+  static_assert(sizeof(CJSpecTab::sub[0]) == sizeof(CJSpecTab::ac1[0]), "sub follows ac1 at one distance");
+  constexpr uint32_t SUB = (uint32_t)(offsetof(CJSpecTab, sub) - offsetof(CJSpecTab, ac1));
+  int c = 0, k = -1, nb = 0, d0 = 0, d1 = 0, d2 = 0, j = 0;
+  uint32_t dcv = 0, dce = 0, thresh = cstep;
+  uint32_t next = cj_state_phase(start);  // phase of the block after the current one
+  uint32_t tab = x.tab, sh = 32 - CJ_MULTI_DC_BITS, acm = x.tab, ac1 = x.tab;
+  uint2 ph = make_uint2(cj_lds32(phases + 8 * next), cj_lds32(phases + 8 * next + 4));  // entry of phase `next`
+  br.pos = (uint32_t)cj_state_bit(start);
+  br.col = x.ring;
+  br.cur = br.nxt = br.nn = 0;
+  uint32_t old[CJ_CKPTS];
+  CJJoin jn = {CJ_CKPTS, -1};
+#pragma unroll
+  for (int q = 0; q < CJ_CKPTS; q++) old[q] = 0xFFFFFFFFu;  // matches no decode state
+  // checkpoints may have been written by another SM in an earlier pass of
+  // the same kernel: read them from L2, never a stale L1 line
+  if (run && x.resume) {
+#pragma unroll
+    for (int q = 0; q < CJ_CKPTS; q++) old[q] = __ldcg(&ck[q].pp);
+  }
+  auto phase = [&]() { return next ? next - 1 : (uint32_t)bpm - 1; };  // of the current block
+  // Begin the block of phase `next`.
+  auto begin_block = [&]() {
+    tab = ph.x & 0xFFFFu;
+    sh = 32 - CJ_MULTI_DC_BITS;
+    acm = ph.x >> 16;
+    ac1 = ph.y & 0xFFFFu;
+    c = (int)((ph.y >> 16) & 255);
+    next = ph.y >> 24;
+    ph.x = cj_lds32(phases + 8 * next);
+    ph.y = cj_lds32(phases + 8 * next + 4);
+    k = -1;
+  };
+  // The checkpoints at the block boundary `rel` bits into the subsequence;
+  // true when this decode has joined an earlier one.
+  auto checkpoint = [&](uint32_t rel) -> bool {
+    const uint32_t pp = (phase() << 24) | rel;
+    while (j < CJ_CKPTS && rel >= thresh) {
+      uint32_t o = old[0];
+#pragma unroll
+      for (int q = 1; q < CJ_CKPTS; q++) o = j == q ? old[q] : o;
+      int src = o == pp ? -1 : -2;
+      if (HYP)
+        for (int h = 0; src == -2 && h < x.nh; h++)
+          if (cj_lds32(x.hpp + 128 * (h * CJ_CKPTS + j)) == pp) src = h;
+      if (src != -2) {
+        jn.j = j;
+        jn.src = src;
+        return true;
       }
       ck[j] = CJCkpt{pp, nb, d0, d1, d2};
       j++;
@@ -299,45 +467,110 @@ __device__ __forceinline__ CJSubRec cj_spec_decode(const CJScanParams& sp, const
     }
     return false;
   };
-  if (rem > 0) {
-    if (checkpoint(endrel - (uint32_t)rem, false)) return r;
-    for (;;) {
-      const uint32_t v = br.peek();
-      const uint32_t st = cj_step(T, sp, slot, v);
-      const int kn = k + (int)((st >> 5) & 127);
-      const uint32_t used = (st & 31) - (kn > 63 ? (st >> 12) : 0u);
-      const bool isdc = k < 0;
-      dcv = isdc ? v : dcv;
-      dcst = isdc ? st : dcst;
-      br.skip(used);
-      rem -= (int)used;
-      slot = aslot;
-      if (kn >= 63) {
-        const uint32_t size = dcst >> 12, len = (dcst & 31) - size;
-        const int dd = size ? cj_extend((dcv << len) >> (32 - size), size) : 0;
-        if (c == 0) d0 += dd;
-        else if (c == 1) d1 += dd;
-        else d2 += dd;
-        k = -1;
-        nb++;
-        m = (m + 1 == (uint32_t)bpm) ? 0 : m + 1;
-        cj_phase(sp, bpm, pack, m, c, slot, aslot);
-        if (rem <= 0) break;
-        const uint32_t rel = endrel - (uint32_t)rem;
-        if (rel >= thresh && checkpoint(rel, false)) return r;
-      } else {
-        k = kn;
+  bool live = run && br.pos < end;
+  if (live) br.init(x.data, x.ring, x.end_byte, br.pos);
+  begin_block();
+  if (live && br.pos - begin >= thresh) live = !checkpoint(br.pos - begin);
+  // Consume entry st and choose the next step's table.
+  auto apply = [&](uint32_t st) {
+    br.skip(st & 31);
+    k += (int)(st >> 9);
+    const bool prefix = st < (1u << 9);
+    const bool high = k > CJ_MULTI_MAXK;
+    tab = prefix ? ac1 + SUB + ((st & 0x1E0u) << 2) : (high ? ac1 : acm);
+    sh = prefix ? 26 : (high ? 32 - CJ_FAST_BITS : 32 - CJ_MULTI_BITS);
+  };
+  uint32_t p = br.pos;  // the last block boundary
+  while (__any_sync(CJ_FULL, live)) {
+    if (live) br.refill();
+    __syncwarp();
+#pragma unroll 1
+    for (int u = 0; u < CJ_RING_ROUNDS; u++) {
+#pragma unroll
+      for (int q = 0; q < CJ_STEPS_PER_ROUND; q++) {
+        const uint32_t v = br.peek();
+        uint32_t st = cj_tab16(tab + 2 * (v >> sh));
+        if (q == 0) {  // a DC symbol can only come first in a round
+          dcv = k < 0 ? v : dcv;
+          dce = k < 0 ? st : dce;
+        }
+        // (finished lanes decode on behind their end in the first step: their
+        // results are taken already)
+        if (q > 0) st = k < 63 ? st : 0;
+        apply(st);
       }
+      if (live && k >= 63) {
+        if (k >= CJ_SPEC_FARK) {  // rare
+          k -= (int)(CJ_SPEC_FAR >> 9);
+          const uint32_t v = br.peek();
+          const uint32_t st = cj_spec_entry(cj_step(*x.tp, k < 0 ? x.sp->comp_dc[c] : x.sp->comp_ac[c], v), 0, k < 0);
+          if (k < 0) {
+            dcv = v;
+            dce = st;
+          }
+          apply(st);
+        }
+        if (k >= 63) {
+          const uint32_t size = (dce >> 5) & 15, w = dcv << ((dce & 31) - size);
+          // (T.81 F.2.2.1: a magnitude whose first bit is 0 is negative)
+          int dd = (int)__funnelshift_rc(w, 0u, 32 - size);
+          dd -= (int)w >= 0 ? (int)((1u << size) - 1u) : 0;
+          if (c == 0) d0 += dd;
+          else if (c == 1) d1 += dd;
+          else d2 += dd;
+          nb++;
+          begin_block();
+          p = br.pos;
+          if (p >= end) live = false;
+          else if (p - begin >= thresh && j < CJ_CKPTS) live = !checkpoint(p - begin);
+        }
+      }
+      __syncwarp();
     }
   }
-  const uint64_t pend = br.pos();
-  checkpoint((uint32_t)(pend - ln.begin), true);  // thresholds not reached: the exit
-  r.exit = cj_state(pend, m);
-  r.nblocks = nb;
-  r.dc[0] = d0;
-  r.dc[1] = d1;
-  r.dc[2] = d2;
-  return r;
+  const uint32_t m = phase();
+  if (!run) return;
+  CJSubRec& r = x.r;
+  r.start = start;
+  if (jn.j == CJ_CKPTS) {
+    // thresholds not reached: the exit
+    const uint32_t pp = (m << 24) | (p - begin);
+#pragma unroll
+    for (int q = 0; q < CJ_CKPTS; q++)
+      if (q >= j) ck[q] = CJCkpt{pp, nb, d0, d1, d2};
+    r.exit = cj_state(p, m);
+    r.nblocks = nb;
+    r.dc[0] = d0;
+    r.dc[1] = d1;
+    r.dc[2] = d2;
+    return;
+  }
+  const CJCkpt* sc = HYP && jn.src >= 0 ? x.hck + jn.src * CJ_CKPTS : ck;
+  const CJCkpt at = {0, __ldcg(&sc[jn.j].nb), __ldcg(&sc[jn.j].d0), __ldcg(&sc[jn.j].d1), __ldcg(&sc[jn.j].d2)};
+  if (HYP && jn.src >= 0) {
+    const CJSubRec* hr = x.hrec + jn.src;
+    r.exit = __ldcg(&hr->exit);
+    r.nblocks = __ldcg(&hr->nblocks);
+#pragma unroll
+    for (int q = 0; q < 3; q++) r.dc[q] = __ldcg(&hr->dc[q]);
+  }
+  r.nblocks += nb - at.nb;
+  r.dc[0] += d0 - at.d0;
+  r.dc[1] += d1 - at.d1;
+  r.dc[2] += d2 - at.d2;
+#pragma unroll
+  for (int q = 0; q < CJ_CKPTS; q++) {
+    if (q < jn.j) continue;
+    ck[q] = CJCkpt{__ldcg(&sc[q].pp), __ldcg(&sc[q].nb) + nb - at.nb, __ldcg(&sc[q].d0) + d0 - at.d0,
+                   __ldcg(&sc[q].d1) + d1 - at.d1, __ldcg(&sc[q].d2) + d2 - at.d2};
+  }
+}
+
+// The checkpoint positions of a lane's `nh` hypothesis decodes into its
+// column of shared memory (entry 32 * (h * CJ_CKPTS + j)).
+__device__ __forceinline__ void cj_hyp_fill(uint32_t* hpp, const CJCkpt* hck, int nh) {
+#pragma unroll 4
+  for (int q = 0; q < nh * CJ_CKPTS; q++) hpp[32 * q] = __ldcg(&hck[q].pp);
 }
 
 // Checkpoints of global lane `i` and the threshold spacing of a subsequence.
@@ -347,23 +580,17 @@ __device__ __forceinline__ uint32_t cj_ckpt_step(int sub_bits) { return (uint32_
 // Re-decode lanes whose input state (lane 0: `lane0_in`; others: the exit of
 // the previous lane) differs from the state they last decoded from, until no
 // lane changes.  Lane l settles after at most l+1 re-decodes.
-// HYP: hck / hrec / nh are the lane's hypothesis decodes (cj_spec_decode).
-template <bool HYP = false>
-__device__ __forceinline__ bool cj_warp_settle(const CJScanParams& sp, const CJSteps& T, const uint32_t* words,
-                                               const CJLane& ln, CJSubRec& r, uint64_t lane0_in,
-                                               CJCkpt* ck, uint32_t cstep, const CJCkpt* hck = nullptr,
-                                               const CJSubRec* hrec = nullptr, int nh = 0) {
+__device__ __forceinline__ bool cj_warp_settle(CJSpecJob& x, const CJLane& ln, uint64_t lane0_in) {
   int lane = threadIdx.x & 31;
   bool dirty = false;
+  x.resume = true;
   for (int it = 0; it < 34; it++) {
-    uint64_t pred = __shfl_up_sync(CJ_FULL, r.exit, 1);
-    uint64_t want = ln.head ? r.start : (lane == 0 ? lane0_in : pred);
-    bool change = ln.active && want != r.start;
+    uint64_t pred = __shfl_up_sync(CJ_FULL, x.r.exit, 1);
+    uint64_t want = ln.head ? x.r.start : (lane == 0 ? lane0_in : pred);
+    bool change = ln.active && want != x.r.start;
     if (!__any_sync(CJ_FULL, change)) break;
-    if (change) {
-      r = cj_spec_decode<true, HYP>(sp, T, words, ln, want, ck, r, cstep, hck, hrec, nh);
-      dirty = true;
-    }
+    cj_spec_warp<false>(&x, change, want);
+    dirty = dirty || change;
   }
   return dirty;
 }
@@ -450,7 +677,7 @@ __device__ __forceinline__ int64_t cj_lane_write_end(const CJLane& ln, const CJS
 // go to memory whole, so the range needs no zero fill; a unit that stops at
 // an error stores its partial block (as the serial decode leaves it) and zeroes
 // the rest of its range, up to `zero_end`.
-__device__ __forceinline__ void cj_write_units_warp(const CJScanParams& sp, const CJSteps& T, const uint32_t* words,
+__device__ __forceinline__ void cj_write_units_warp(const CJScanParams& sp, const CJScanParams& tp, const uint32_t* words,
                                                     const CJLane& ln, const CJSegment& seg, uint64_t start,
                                                     int64_t first_block, int dc0, int dc1, int dc2,
                                                     int16_t* __restrict__ coef, CJStatus* st, const uint8_t* zz,
@@ -498,7 +725,7 @@ __device__ __forceinline__ void cj_write_units_warp(const CJScanParams& sp, cons
     int done = -1;  // block (of this image) to store after this step
     if (run) {
       const uint32_t v = br.peek();
-      const uint32_t stp = cj_step(T, sp, slot, v);
+      const uint32_t stp = cj_step(tp, slot, v);
       const uint32_t dk = (stp >> 5) & 127, size = stp >> 12, total = stp & 31;
       const int kn = k + (int)dk;
       const uint32_t len = total - size;
