@@ -342,18 +342,6 @@ __device__ __forceinline__ void bt_rank_end(CJBatchCtl* ctl, BTRank& k) {
   for (int s = 0; s < k.slot; s++) k.rank += __ldcg(&ctl->slot_ctas[s]);
 }
 
-// Next warp item: item w * gridDim + rank to warp w first.
-__device__ __forceinline__ int bt_next_item(int* counter, int rank, bool& first) {
-  const int nw = blockDim.x >> 5;
-  int w = 0;
-  if (first) {
-    first = false;
-    return (int)(threadIdx.x >> 5) * (int)gridDim.x + rank;
-  }
-  if ((threadIdx.x & 31) == 0) w = atomicAdd(counter, 1) + nw * (int)gridDim.x;
-  return __shfl_sync(0xFFFFFFFFu, w, 0);
-}
-
 // Next group of BT_WARPS consecutive items for the whole CTA: group `rank`
 // first, then thread 0 takes one and the CTA shares it.  The leading barrier
 // also ends the previous group: every warp is done with it and with the tables
@@ -381,19 +369,25 @@ __device__ __forceinline__ int bt_find(int n, int v, F key) {
   return lo;
 }
 
-// Dynamic shared memory of the decode kernel: two slots of speculative-decode
-// tables and the warps' bit windows in the sync and fix-up phases (54 KB: 4
-// CTAs per SM), the write-out's block buffers (one 64-entry int16 block per thread) in
-// phase 8.
-#define BT_WBUF_BYTES (BT_THREADS * 64 * 2)
+__device__ __forceinline__ uint32_t bt_smem_addr(const void* p) {
+  return (uint32_t)__cvta_generic_to_shared(p);
+}
+
+// Dynamic shared memory of the decode kernel: two slots of tables and the
+// warps' bit windows in the sync and fix-up phases (54 KB: 4 CTAs per SM); in
+// phase 8 the write-out's block buffers (one 64-entry int16 block per thread),
+// one slot of its part of the tables and the warps' windows.
 #define BT_SPEC_OFF (2 * sizeof(CJSpecTab))  // the warps' rings and phase entries
 #define BT_HPP_OFF (BT_SPEC_OFF + BT_WARPS * sizeof(CJSpecWarp))  // hypothesis variant: checkpoint positions
 #define BT_DECODE_SMEM BT_HPP_OFF
 static constexpr size_t bt_decode_smem(int nhyp) {
   return BT_DECODE_SMEM + (nhyp > 1 ? (size_t)BT_WARPS * nhyp * CJ_CKPTS * 32 * 4 : 0);
 }
-static_assert(BT_DECODE_SMEM >= BT_WBUF_BYTES, "write-out block buffers");
-static_assert(sizeof(CJSpecTab) % 16 == 0, "int4 table copy");
+#define BT_WTAB_OFF (BT_THREADS * 64 * 2)
+#define BT_WTAB_FROM ((int)offsetof(CJSpecTab, ac1))  // the write-out needs no multi-symbol entries
+#define BT_WRITE_OFF (BT_WTAB_OFF + sizeof(CJSpecTab) - BT_WTAB_FROM)
+static_assert(BT_DECODE_SMEM >= BT_WRITE_OFF + BT_WARPS * sizeof(CJWriteWarp), "write-out shared memory");
+static_assert(sizeof(CJSpecTab) % 16 == 0 && BT_WTAB_FROM % 16 == 0 && BT_WRITE_OFF % 16 == 0, "int4 table copy");
 static_assert(BT_DECODE_SMEM >= BT_THREADS * sizeof(CJAgg5), "phase 7 scan space");
 
 __device__ __forceinline__ int bt_image_of_warp(const CJBatchArgs& a, int w) {
@@ -416,19 +410,22 @@ __device__ __forceinline__ BTItem bt_item(const CJBatchArgs& a, int w, int h) {
   return it;
 }
 
-// Speculative-decode tables of the sync and fix-up phases.  The 8 warps of an item
-// group work on consecutive warps of the batch, so they need the tables of a
+// Tables of the entropy phases.  The 8 warps of an
+// item group work on consecutive warps of the batch, so they need the tables of a
 // few images, and of one if the images share their DHT contents, as files of
-// one encoder do.  The CTA keeps the tables of two images in shared memory
-// (`id`: which, -1: none) and serves its warps in rounds: stage what the first
-// waiting warp and the next one with other tables need (nothing when they are
-// there from an earlier group), and run f(tables) in the warps with either.
+// one encoder do.  The CTA keeps the tables of SLOTS images in shared memory
+// (`id`: which, -1: none) -- each image's bytes from `off` of its CJSpecTab on --
+// and serves its warps in rounds: stage what the first
+// waiting warp and, with two slots, the next one with other tables need (nothing
+// when they are there from an earlier group), and run f(shared address of the
+// CJSpecTab) in the warps with either.
 // `tab`: the warp's table image, -1: no work.  Every thread calls it.
 struct BTTabs {
   int want[BT_WARPS], id[2];
 };
-template <class F>
-__device__ __forceinline__ void bt_with_tables(const CJBatchArgs& a, BTTabs& s, CJSpecTab* slots, int tab, F f) {
+template <int SLOTS, int OFF, class F>
+__device__ __forceinline__ void bt_with_tables(const CJBatchArgs& a, BTTabs& s, uint8_t* slots, int tab, F f) {
+  constexpr int BYTES = (int)sizeof(CJSpecTab) - OFF;
   if ((threadIdx.x & 31) == 0) s.want[threadIdx.x >> 5] = tab;
   __syncthreads();
   unsigned todo = 0;
@@ -440,27 +437,27 @@ __device__ __forceinline__ void bt_with_tables(const CJBatchArgs& a, BTTabs& s, 
     for (int w = 0; w < BT_WARPS; w++) {
       if (!((todo >> w) & 1)) continue;
       const int t = s.want[w];
-      if (t != ta && tb < 0) tb = t;
+      if (SLOTS > 1 && t != ta && tb < 0) tb = t;
       if (t == ta || t == tb) mask |= 1u << w;
     }
-    int sa = s.id[0] == ta ? 0 : (s.id[1] == ta ? 1 : -1);
+    int sa = s.id[0] == ta ? 0 : (SLOTS > 1 && s.id[1] == ta ? 1 : -1);
     int sb = tb < 0 ? -1 : (s.id[0] == tb ? 0 : (s.id[1] == tb ? 1 : -1));
     const bool load_a = sa < 0, load_b = tb >= 0 && sb < 0;
-    if (load_a) sa = sb == 0 ? 1 : 0;
+    if (load_a) sa = SLOTS > 1 && sb == 0 ? 1 : 0;
     if (load_b) sb = 1 - sa;
     if (load_a || load_b) {
       __syncthreads();  // every thread has read the ids
       // built by another CTA in this kernel: read from L2
       for (int h = 0; h < 2; h++) {
         if (!(h ? load_b : load_a)) continue;
-        const int4* src = reinterpret_cast<const int4*>(a.spec + (h ? tb : ta));
-        int4* dst = reinterpret_cast<int4*>(slots + (h ? sb : sa));
-        for (int k = threadIdx.x; k < (int)(sizeof(CJSpecTab) / 16); k += BT_THREADS) dst[k] = __ldcg(src + k);
+        const int4* src = reinterpret_cast<const int4*>(reinterpret_cast<const uint8_t*>(a.spec + (h ? tb : ta)) + OFF);
+        int4* dst = reinterpret_cast<int4*>(slots + (h ? sb : sa) * BYTES);
+        for (int k = threadIdx.x; k < BYTES / 16; k += BT_THREADS) dst[k] = __ldcg(src + k);
         if (threadIdx.x == 0) s.id[h ? sb : sa] = h ? tb : ta;
       }
       __syncthreads();
     }
-    if (tab >= 0 && (tab == ta || tab == tb)) f(slots[tab == ta ? sa : sb]);
+    if (tab >= 0 && (tab == ta || tab == tb)) f(bt_smem_addr(slots + (tab == ta ? sa : sb) * BYTES) - (uint32_t)OFF);
     todo &= ~mask;
     if (todo) __syncthreads();  // before a slot is overwritten
   }
@@ -592,10 +589,6 @@ __device__ void bt_build_params(const CJImageHeader& h, CJScanParams& p, int tab
 
 // ---------------------------------------------------------------- the kernel
 
-__device__ __forceinline__ uint32_t bt_smem_addr(const void* p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-
 // MINB = CTAs per SM the register allocation is sized for (64 registers at
 // 4); the autotuner picks among the compiled variants.  HYP: the variant
 // with MCU-phase hypotheses (phase 5a), launched only for latency-bound
@@ -613,7 +606,7 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) k_decode_batch(CJBatchArgs a
     gen = atomicAdd(&a.ctl->bar_gen, 0);
     bt_rank_begin(a.ctl, s_rank);
   }
-  if (threadIdx.x < 64) s_zz[threadIdx.x] = c_bt_zz[threadIdx.x];
+  if (threadIdx.x < 64) s_zz[threadIdx.x] = 2 * c_bt_zz[threadIdx.x];
   const int lane = threadIdx.x & 31;
 
   bt_stamp(a.ctl, 0);
@@ -816,7 +809,6 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) k_decode_batch(CJBatchArgs a
   if (!bt_grid_sync(a.ctl, gen, a.wait_limit, &s_ok)) return;
 
   bt_stamp(a.ctl, 5);
-  CJSpecTab* tabs = reinterpret_cast<CJSpecTab*>(smem);
   if (threadIdx.x < 2) s_tabs.id[threadIdx.x] = -1;  // (the first group's barrier orders it)
   const CJSpecWarp& spw = reinterpret_cast<const CJSpecWarp*>(smem + BT_SPEC_OFF)[threadIdx.x >> 5];
   uint32_t* hpp = reinterpret_cast<uint32_t*>(smem + BT_HPP_OFF) + (threadIdx.x >> 5) * a.nhyp * CJ_CKPTS * 32 + lane;
@@ -838,7 +830,7 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) k_decode_batch(CJBatchArgs a
       if (wg >= a.nwarps) continue;  // CTA-uniform
       const int w = wg + (int)(threadIdx.x >> 5);
       const BTItem it = bt_item(a, w, h);
-      bt_with_tables(a, s_tabs, tabs, it.tab, [&](const CJSpecTab& tb) {
+      bt_with_tables<2, 0>(a, s_tabs, smem, it.tab, [&](uint32_t tb) {
         const CJImageDesc& d = a.desc[it.i];
         const CJScanParams &sp = a.prm[it.i], &tp = a.prm[it.tab];
         CJLane ln = cj_lane(a.segs + d.seg0, it.nseg, it.nsub, it.j0 + lane, d.sub_bits);
@@ -875,7 +867,7 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) k_decode_batch(CJBatchArgs a
       if (wg >= a.nwarps) continue;  // CTA-uniform
       const int w = wg + (int)(threadIdx.x >> 5);
       const BTItem it = bt_item(a, w, 0);
-      bt_with_tables(a, s_tabs, tabs, it.tab, [&](const CJSpecTab& tb) {
+      bt_with_tables<2, 0>(a, s_tabs, smem, it.tab, [&](uint32_t tb) {
         const CJImageDesc& d = a.desc[it.i];
         const CJScanParams &sp = a.prm[it.i], &tp = a.prm[it.tab];
         const int nhi = min(nh, sp.bpm - 1);
@@ -918,7 +910,7 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) k_decode_batch(CJBatchArgs a
     if (g0 >= a.nwarps) break;
     const int w = g0 + (int)(threadIdx.x >> 5);
     const BTItem it = bt_item(a, w, 0);
-    bt_with_tables(a, s_tabs, tabs, it.tab, [&](const CJSpecTab& tb) {
+    bt_with_tables<2, 0>(a, s_tabs, smem, it.tab, [&](uint32_t tb) {
       const CJImageDesc& d = a.desc[it.i];
       const CJScanParams &sp = a.prm[it.i], &tp = a.prm[it.tab];
       CJLane ln = cj_lane(a.segs + d.seg0, it.nseg, it.nsub, it.j0 + lane, d.sub_bits);
@@ -988,7 +980,7 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) k_decode_batch(CJBatchArgs a
       const uint64_t want = ln.head ? r.start : (lane == 0 ? in0 : pred);
       bool moved = false;
       const bool redo = __any_sync(CJ_FULL, ln.active && want != r.start);
-      bt_with_tables(a, s_tabs, tabs, redo ? it.tab : -1, [&](const CJSpecTab& tb) {
+      bt_with_tables<2, 0>(a, s_tabs, smem, redo ? it.tab : -1, [&](uint32_t tb) {
         const CJScanParams &sp = a.prm[it.i], &tp = a.prm[it.tab];
         const int64_t gs = d.sub0 + j0 + lane;
         CJSpecJob x;
@@ -1086,74 +1078,103 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) k_decode_batch(CJBatchArgs a
   // so write items are a quarter as long as sync items whatever the
   // subsequence size.  An item is 8 lanes x 4 units of one 32-lane warp w,
   // whose block / DC prefix it recomputes; the warp writes its 32 units'
-  // blocks cooperatively (cj_write_units_warp).  (In a corrupt stream a unit may
+  // blocks cooperatively (cj_write_warp).  (In a corrupt stream a unit may
   // write past an error an earlier unit stopped at; only blocks after that
   // error, so the first error of the image is the same.)
   {
     constexpr int UNITS = CJ_CKPTS + 1, LANES = 32 / UNITS;
     const int nitems = a.nwarps * UNITS;
-    // the warp's block buffers, zero between blocks (the step tables are read
-    // from global memory here: the buffers take the staging space)
-    int16_t* wbuf = reinterpret_cast<int16_t*>(smem) + (threadIdx.x >> 5) * 32 * 64;
-    for (int k = lane; k < 32 * 64 * 2 / 16; k += 32) reinterpret_cast<uint4*>(wbuf)[k] = make_uint4(0, 0, 0, 0);
-    __syncwarp();
+    const int wp = threadIdx.x >> 5;
+    // the warps' block buffers, zero between blocks
+    for (int k = threadIdx.x; k < BT_WTAB_OFF / 16; k += BT_THREADS)
+      reinterpret_cast<uint4*>(smem)[k] = make_uint4(0, 0, 0, 0);
+    if (threadIdx.x == 0) s_tabs.id[0] = -1;  // (the first group's barrier orders it)
+    CJWriteWarp& ww = reinterpret_cast<CJWriteWarp*>(smem + BT_WRITE_OFF)[wp];
     first = true;
-    for (int t = bt_next_item(&a.ctl->next_write, s_rank.rank, first); t < nitems; t = bt_next_item(&a.ctl->next_write, s_rank.rank, first)) {
-      const int w = t / UNITS, part = t % UNITS;
-      const int i = bt_image_of_warp(a, w);
-      const CJImageDesc& d = a.desc[i];
-      CJStatus* st = &a.st[i];
-      const int nsub = __ldcg(&st->nsub), nseg = __ldcg(&st->nseg);
-      const int j0 = w * 32 - d.sub0;
-      if (j0 >= nsub) continue;
-      const CJScanParams& sp = a.prm[i];
-      const CJScanParams& tp = a.prm[__ldcg(&sp.tab)];
-      const uint32_t* words = reinterpret_cast<const uint32_t*>(a.data + d.data_off);
-      // block / DC prefix of the 32 lanes of warp w (thread = lane `lane`)
-      const CJLane lw = cj_lane(a.segs + d.seg0, nseg, nsub, j0 + lane, d.sub_bits);
-      CJSubRec rw;
-      if (lw.active) rw = bt_load_rec(&a.recs[d.sub0 + j0 + lane]);
-      else {
-        rw.start = rw.exit = 0;
-        rw.nblocks = rw.dc[0] = rw.dc[1] = rw.dc[2] = 0;
-      }
-      int64_t bw;
-      int e0, e1, e2;
-      cj_warp_prefix(rw, lw, __ldcg(&a.carry[w].nblocks), __ldcg(&a.carry[w].dc[0]),
-                     __ldcg(&a.carry[w].dc[1]), __ldcg(&a.carry[w].dc[2]), &bw, &e0, &e1, &e2);
-      const int64_t firstw = bw + (lw.active ? a.segs[d.seg0 + lw.seg].first_block : 0);
-      // this thread's unit: lane ul of warp w, quarter q
-      const int ul = part * LANES + lane / UNITS, q = lane % UNITS;
-      const int64_t lane_first = __shfl_sync(CJ_FULL, firstw, ul);
-      int dc0 = __shfl_sync(CJ_FULL, e0, ul), dc1 = __shfl_sync(CJ_FULL, e1, ul), dc2 = __shfl_sync(CJ_FULL, e2, ul);
-      CJSubRec r;
-      r.start = __shfl_sync(CJ_FULL, rw.start, ul);
-      r.nblocks = __shfl_sync(CJ_FULL, rw.nblocks, ul);
-      const CJLane ln = cj_lane(a.segs + d.seg0, nseg, nsub, j0 + ul, d.sub_bits);
-      const CJSegment seg = a.segs[d.seg0 + (ln.active ? ln.seg : 0)];
-      const CJCkpt* ck = cj_lane_ckpts(a.ckpt, d.sub0 + j0 + ul);
-      uint64_t start = r.start, stop = ~0ull;
-      int64_t first = lane_first, end = 0;
-      if (ln.active) {
-        if (q > 0) {
-          const uint32_t pp = __ldcg(&ck[q - 1].pp);
-          start = cj_state(ln.begin + (pp & 0xFFFFFFu), pp >> 24);
-          first += __ldcg(&ck[q - 1].nb);
-          dc0 += __ldcg(&ck[q - 1].d0);
-          dc1 += __ldcg(&ck[q - 1].d1);
-          dc2 += __ldcg(&ck[q - 1].d2);
+    for (;;) {
+      const int g0 = bt_next_group(&a.ctl->next_write, &s_grp, s_rank.rank, first);
+      if (g0 >= nitems) break;
+      const int t = g0 + wp, w = t / UNITS, part = t % UNITS;
+      const BTItem it = bt_item(a, t < nitems ? w : a.nwarps, 0);
+      bt_with_tables<1, BT_WTAB_FROM>(a, s_tabs, smem + BT_WTAB_OFF, it.tab, [&](uint32_t tb) {
+        const CJImageDesc& d = a.desc[it.i];
+        const int j0 = it.j0, nsub = it.nsub, nseg = it.nseg;
+        // block / DC prefix of the 32 lanes of warp w (thread = lane `lane`)
+        const CJLane lw = cj_lane(a.segs + d.seg0, nseg, nsub, j0 + lane, d.sub_bits);
+        CJSubRec rw;
+        if (lw.active) rw = bt_load_rec(&a.recs[d.sub0 + j0 + lane]);
+        else {
+          rw.start = rw.exit = 0;
+          rw.nblocks = rw.dc[0] = rw.dc[1] = rw.dc[2] = 0;
         }
-        if (q < UNITS - 1) {
-          stop = ln.begin + (__ldcg(&ck[q].pp) & 0xFFFFFFu);
-          const int64_t bend = seg.first_block + seg.nblocks;
-          end = lane_first + __ldcg(&ck[q].nb);
-          if (end > bend) end = bend;
-        } else {
-          end = cj_lane_write_end(ln, seg, r, lane_first);
+        int64_t bw;
+        int e0, e1, e2;
+        cj_warp_prefix(rw, lw, __ldcg(&a.carry[w].nblocks), __ldcg(&a.carry[w].dc[0]),
+                       __ldcg(&a.carry[w].dc[1]), __ldcg(&a.carry[w].dc[2]), &bw, &e0, &e1, &e2);
+        const int64_t firstw = bw + (lw.active ? a.segs[d.seg0 + lw.seg].first_block : 0);
+        // this thread's unit: lane ul of warp w, quarter q
+        const int ul = part * LANES + lane / UNITS, q = lane % UNITS;
+        const int64_t lane_first = __shfl_sync(CJ_FULL, firstw, ul);
+        CJWriteJob x;
+        x.dc[0] = __shfl_sync(CJ_FULL, e0, ul);
+        x.dc[1] = __shfl_sync(CJ_FULL, e1, ul);
+        x.dc[2] = __shfl_sync(CJ_FULL, e2, ul);
+        CJSubRec r;
+        r.start = __shfl_sync(CJ_FULL, rw.start, ul);
+        r.nblocks = __shfl_sync(CJ_FULL, rw.nblocks, ul);
+        const CJLane ln = cj_lane(a.segs + d.seg0, nseg, nsub, j0 + ul, d.sub_bits);
+        const CJSegment seg = a.segs[d.seg0 + (ln.active ? ln.seg : 0)];
+        const CJCkpt* ck = cj_lane_ckpts(a.ckpt, d.sub0 + j0 + ul);
+        uint64_t start = r.start;
+        int64_t blk = lane_first, end = 0;
+        x.stop = 0xFFFFFFFFu;
+        if (ln.active) {
+          if (q > 0) {
+            const uint32_t pp = __ldcg(&ck[q - 1].pp);
+            start = cj_state(ln.begin + (pp & 0xFFFFFFu), pp >> 24);
+            blk += __ldcg(&ck[q - 1].nb);
+            x.dc[0] += __ldcg(&ck[q - 1].d0);
+            x.dc[1] += __ldcg(&ck[q - 1].d1);
+            x.dc[2] += __ldcg(&ck[q - 1].d2);
+          }
+          if (q < UNITS - 1) {
+            x.stop = (uint32_t)ln.begin + (__ldcg(&ck[q].pp) & 0xFFFFFFu);
+            const int64_t bend = seg.first_block + seg.nblocks;
+            end = lane_first + __ldcg(&ck[q].nb);
+            if (end > bend) end = bend;
+          } else {
+            end = cj_lane_write_end(ln, seg, r, lane_first);
+          }
         }
-      }
-      cj_write_units_warp(sp, tp, words, ln, seg, start, first, dc0, dc1, dc2, a.coef + d.coef0 * 64, st, s_zz, stop,
-                          end, ln.active, wbuf);
+        x.sp = &a.prm[it.i];
+        x.tp = &a.prm[it.tab];
+        x.st = &a.st[it.i];
+        x.data = reinterpret_cast<const uint4*>(a.data + d.data_off);
+        x.base = __shfl_sync(CJ_FULL, blk, 0);
+        x.coef = a.coef + (d.coef0 + x.base) * 64;
+        x.tab = tb;
+        x.ring = bt_smem_addr(ww.ring) + 4 * lane;
+        x.phase = bt_smem_addr(ww.phase);
+        x.order = bt_smem_addr(ww.order);
+        x.wbuf = bt_smem_addr(smem) + wp * 32 * 128;
+        x.zz = bt_smem_addr(s_zz);
+        x.end_byte = (uint32_t)ln.end_byte;
+        x.end = (uint32_t)ln.end;
+        x.seg_end = (uint32_t)seg.bit_end;
+        x.pos = (uint32_t)cj_state_bit(start);
+        x.m = cj_state_phase(start);
+        x.blk = (int)(blk - x.base);
+        x.bend = (int)(seg.first_block + seg.nblocks - x.base);
+        x.last = ln.last;
+        x.marker = seg.marker_follows != 0;
+        cj_write_warp(&x, ln.active);
+        // blocks of the range an early stop left undecoded read as zeros
+        for (int64_t y = x.base + x.blk + (x.cut ? 1 : 0); ln.active && y < end; y++) {
+          uint4* z = reinterpret_cast<uint4*>(a.coef + (d.coef0 + y) * 64);
+#pragma unroll
+          for (int i = 0; i < 8; i++) z[i] = make_uint4(0, 0, 0, 0);
+        }
+      });
     }
   }
 }

@@ -62,21 +62,22 @@ struct CJSteps {
   uint16_t sub[4][CJ_STEP_SUBS][64];
 };
 
-// Tables of the speculative decode (which needs positions and DC sums, not AC
-// values), in shared memory.  One 16-bit entry:
+// Tables of the entropy loops, in shared memory.  One 16-bit entry:
 //   bits 0-4   bits consumed (codes and magnitudes)
-//   bits 5-8   DC: the magnitude size; long code: its row in `sub`
+//   bits 5-8   one symbol: the magnitude size (15 for an invalid code, 0 for an
+//              EOB); long code: its row in `sub`
 //   bits 9-15  advance of the zig-zag position (DC 1, from -1 to 0; an EOB or an
 //              invalid code adds 63, in a DC table 64); 0: the first 10 bits of
 //              a longer code, decoded on from its row by the next 6 bits
 // CJ_SPEC_FAR (nothing consumed, the position past every other): decode the
 // symbol through the CJSteps in memory -- DC codes of more than 9 bits and AC
 // tables with more long-code prefixes than rows.
-//   acm  every whole symbol the next CJ_MULTI_BITS bits determine, as one entry,
+//   acm  (the speculative decode, which needs positions and DC sums but no AC
+//        values) every whole symbol the next CJ_MULTI_BITS bits determine, as one entry,
 //        while they advance by at most 16 together (an EOB after at most 15):
 //        up to position CJ_MULTI_MAXK no symbol of an entry can lie behind the
 //        block's end, so an entry is always taken whole
-//   ac1  one symbol (positions above CJ_MULTI_MAXK)
+//   ac1  one symbol (positions above CJ_MULTI_MAXK, and the write-out)
 // An 11-bit window holds 1.5 symbols on average at high bit rates and more
 // than two at low ones.
 #define CJ_MULTI_BITS 11
@@ -270,8 +271,8 @@ CJ_HD uint32_t cj_step(const CJScanParams& sp, uint32_t slot, uint32_t v) { retu
 // Entries of the CJSpecTab from the decode steps: a step, a primary entry of an
 // AC table, entry of a subtable.
 CJ_HD uint16_t cj_spec_entry(uint32_t st, uint32_t behind, bool dc = false) {
-  const uint32_t dk = (st >> 5) & 127;
-  return (uint16_t)(((st & 31) - behind) | ((st >> 12) << 5) | ((dk >= CJ_STEP_EOB ? CJ_SPEC_EOB + dc : dk) << 9));
+  const uint32_t dk = (st >> 5) & 127, low = dk >= CJ_STEP_BAD_AC ? 15 : st >> 12;
+  return (uint16_t)(((st & 31) - behind) | (low << 5) | ((dk >= CJ_STEP_EOB ? CJ_SPEC_EOB + dc : dk) << 9));
 }
 CJ_HD uint16_t cj_spec_ac1(uint32_t st) {
   if (st & 31) return cj_spec_entry(st, 0);

@@ -153,27 +153,47 @@ __device__ __forceinline__ uint32_t cj_tab16(uint32_t a) {
   asm("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
   return v;
 }
+__device__ __forceinline__ uint32_t cj_tab8(uint32_t a) {
+  uint32_t v;
+  asm("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ uint4 cj_lds128(uint32_t a) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void cj_sts128_zero(uint32_t a) {
+  asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(a), "r"(0u) : "memory");
+}
+__device__ __forceinline__ void cj_sts16(uint32_t a, uint32_t v) {
+  asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"((uint16_t)v) : "memory");
+}
 __device__ __forceinline__ void cj_sts32(uint32_t a, uint32_t v) {
   asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
 }
 
 // Bit window of a lane in the warp-synchronous decode loops.  A lane's
-// stream runs through a ring of CJ_RING_WORDS big-endian words in shared
-// memory (word w in slot w mod CJ_RING_WORDS, `col` + 128 bytes per slot: one
+// stream runs through a ring of WORDS big-endian words in shared
+// memory (word w in slot w mod WORDS, `col` + 128 bytes per slot: one
 // bank per lane, so every access is conflict-free at any progress of the
 // lanes).  The current and the next word are in registers and the one after
 // them is read a symbol ahead, without branches: a symbol's chain is a funnel
 // shift, the table lookup, the position update and two selects.  Global memory
-// is touched only in refill(), which the whole warp runs together once per
-// CJ_RING_ROUNDS rounds of the loop: a 16-byte chunk fetched there has until
+// is touched only in refill(), which the whole warp runs together every
+// ROUNDS rounds of the loop: a 16-byte chunk fetched there has until
 // the next refill to arrive.
 // Bytes at or past `end_byte` read as 0xFF (the padding the reference's bit
 // reader supplies); memory past them is not relied on.
-#define CJ_RING_WORDS 16
 #define CJ_STEPS_PER_ROUND 3
-// rounds per refill: a round is three symbols of at most 31 bits, so three
-// rounds cross at most 9 words; 9 + 2 read ahead + 3 of the oldest chunk < 16
+// A round is three symbols of at most 31 bits: at most 3 words.  With 2 words
+// read ahead and up to 3 of the oldest chunk passed, 16 words serve 3 rounds,
+// and 8 words one (the word read ahead after a round of 3 crossings is read
+// again by the refill).
+#define CJ_RING_WORDS 16
 #define CJ_RING_ROUNDS 3
+#define CJ_WRITE_WORDS 8
+template <int WORDS>
 struct CJWin {
   const uint4* chunks;    // the image's destuffed data, 16-byte aligned
   uint32_t col;           // this lane's ring column (shared address)
@@ -195,25 +215,25 @@ struct CJWin {
         else if (valid < 4) w[i] |= 0xFFFFFFFFu >> (8 * valid);
       }
     }
-    const uint32_t o = col + 128 * ((4 * c) & (CJ_RING_WORDS - 1));
+    const uint32_t o = col + 128 * ((4 * c) & (WORDS - 1));
 #pragma unroll
     for (int i = 0; i < 4; i++) cj_sts32(o + 128 * i, w[i]);
   }
   // word pos / 32 + ahead
   __device__ __forceinline__ uint32_t word(uint32_t ahead) const {
-    return cj_lds32(col + (((pos + 32 * ahead) << 2) & (128 * (CJ_RING_WORDS - 1))));
+    return cj_lds32(col + (((pos + 32 * ahead) << 2) & (128 * (WORDS - 1))));
   }
   __device__ __forceinline__ void init(const uint4* data, uint32_t ring_col, uint32_t eb, uint32_t p) {
     chunks = data;
     col = ring_col;
     end_byte = eb;
     cb = p >> 7;
-    uint4 v[CJ_RING_WORDS / 4];
+    uint4 v[WORDS / 4];
 #pragma unroll
-    for (int i = 0; i < CJ_RING_WORDS / 4; i++) v[i] = load(cb + i);
-    pf = load(cb + CJ_RING_WORDS / 4);
+    for (int i = 0; i < WORDS / 4; i++) v[i] = load(cb + i);
+    pf = load(cb + WORDS / 4);
 #pragma unroll
-    for (int i = 0; i < CJ_RING_WORDS / 4; i++) put(cb + i, v[i]);
+    for (int i = 0; i < WORDS / 4; i++) put(cb + i, v[i]);
     pos = p;
     cur = word(0);
     nxt = word(1);
@@ -222,9 +242,10 @@ struct CJWin {
   // Replace the chunks the window has left behind.
   __device__ __forceinline__ void refill() {
     while ((pos >> 7) > cb) {
-      put(cb + CJ_RING_WORDS / 4, pf);
+      put(cb + WORDS / 4, pf);
       cb++;
-      pf = load(cb + CJ_RING_WORDS / 4);
+      pf = load(cb + WORDS / 4);
+      if (WORDS == 8) nn = word(2);  // read before its chunk was there, after 3 crossings
     }
   }
   __device__ __forceinline__ uint32_t peek() const { return __funnelshift_l(nxt, cur, pos); }
@@ -238,66 +259,6 @@ struct CJWin {
     nn = word(2);
   }
 };
-
-// Bit reader of the decode loops: the current and the next big-endian word
-// and a bit offset; a 32-bit window is one funnel shift, and a word boundary
-// is crossed at most once per symbol (a symbol consumes at most 31 bits).
-// One more word is loaded a crossing ahead and kept as read from memory
-// (byte-swapped only when it becomes the next word), so a load has several
-// symbols to arrive before the window needs it.
-// Bytes at or past `end_byte` read as 0xFF (the padding the reference's bit
-// reader supplies).
-struct CJFBits {
-  const uint32_t* words;
-  uint32_t wfull, end_byte, cur, nxt, raw2, wi, off;
-
-  __device__ __forceinline__ uint32_t word(uint32_t i) const {
-    return i < wfull ? cj_bswap(words[i]) : cj_word(words, i, end_byte);
-  }
-  // word i as stored (cj_bswap of it is word(i))
-  __device__ __forceinline__ uint32_t word_raw(uint32_t i) const {
-    return i < wfull ? words[i] : cj_bswap(cj_word(words, i, end_byte));
-  }
-  __device__ __forceinline__ void init(const uint32_t* w, uint64_t eb, uint64_t p) {
-    words = w;
-    end_byte = (uint32_t)eb;
-    wfull = (uint32_t)(eb >> 2);
-    const uint32_t w0 = (uint32_t)(p >> 5);
-    off = (uint32_t)(p & 31);
-    cur = word(w0);
-    wi = w0 + 1;
-    nxt = word(wi);
-    raw2 = word_raw(wi + 1);
-  }
-  __device__ __forceinline__ uint32_t peek() const { return __funnelshift_l(nxt, cur, off); }
-  __device__ __forceinline__ void skip(uint32_t u) {
-    off += u;
-    if (off >= 32) {
-      off -= 32;
-      cur = nxt;
-      nxt = cj_bswap(raw2);
-      wi++;
-      raw2 = word_raw(wi + 1);
-    }
-  }
-  __device__ __forceinline__ uint64_t pos() const { return ((uint64_t)(wi - 1) << 5) + off; }
-};
-
-// Component, DC slot and AC slot of MCU phase m (from the packed phase
-// table; the per-phase arrays for MCUs of more than 10 blocks).
-__device__ __forceinline__ void cj_phase(const CJScanParams& sp, int bpm, uint64_t pack, uint32_t m, int& c,
-                                         uint32_t& dslot, uint32_t& aslot) {
-  if (bpm <= 10) {
-    const uint32_t f = (uint32_t)(pack >> (6 * m)) & 63;
-    c = (int)(f & 3);
-    dslot = (f >> 2) & 3;
-    aslot = f >> 4;
-  } else {
-    c = sp.phase_comp[m];
-    dslot = sp.comp_dc[c];
-    aslot = sp.comp_ac[c];
-  }
-}
 
 // Checkpoints of a subsequence decode: the decoder state at the first block
 // boundary at or after each of CJ_CKPTS thresholds (1/4, 1/2, 3/4 of the
@@ -324,9 +285,9 @@ struct CJJoin {
 // The loop is straight-line code over the tables of CJSpecTab: a divergent
 // branch costs some 40 cycles whether one lane takes it or all, and with 32
 // lanes at different symbols every branch is taken by some lane in almost
-// every step (measured: 870 cycles per symbol with branches for word
-// crossings, long codes and block ends, against about 60 for the symbol's
-// dependent instructions alone).  So word crossings are selects, a long code
+// every step (measured on 4:2:0 photos: 870 cycles per symbol step with branches
+// for word crossings, long codes and block ends, 280 as here; the sync phase of
+// the 1024-image mix 0.88 -> 0.42 ms, of 48 1080p frames 1.05 -> 0.33 ms).  So word crossings are selects, a long code
 // is two steps (its prefix entry makes its subtable the next step's table), a
 // lane whose block has ended consumes nothing, and the end of blocks is one
 // branch per round of three steps.  The DC entry and window are kept and the
@@ -347,9 +308,27 @@ struct CJJoin {
 // the totals of all joined lanes are taken together after the loop: lanes
 // reach their checkpoints at different steps, so a global load there would
 // stall the warp once per lane and checkpoint.
-// A warp's shared memory in the speculative decode: its ring, and per MCU
-// phase the shared addresses of the phase's tables (x: dc | acm << 16), then
-// ac1, the component << 16 and the next phase << 24 (y).
+// Phase entries: per MCU phase the shared addresses of the phase's tables
+// (x: dc | acm << 16), then ac1, the component << 16 and the next phase << 24
+// (y).  Written by the whole warp for an image and its tables at `tab`.
+__device__ __forceinline__ void cj_phase_entries(const CJScanParams& sp, uint32_t tab, uint32_t phases) {
+  const int i = threadIdx.x & 31, bpm = sp.bpm;
+  __syncwarp();
+  if (i < bpm) {
+    const uint32_t c = sp.phase_comp[i], d = sp.comp_dc[c], a = sp.comp_ac[c] - 2u;
+    const uint32_t dc = tab + (uint32_t)offsetof(CJSpecTab, dc) + d * (uint32_t)sizeof(CJSpecTab::dc[0]);
+    const uint32_t ac1 = tab + (uint32_t)offsetof(CJSpecTab, ac1) + a * (uint32_t)sizeof(CJSpecTab::ac1[0]);
+    const uint32_t acm = tab + a * (uint32_t)sizeof(CJSpecTab::acm[0]);
+    cj_sts32(phases + 8 * i, dc | (acm << 16));
+    cj_sts32(phases + 8 * i + 4, ac1 | (c << 16) | ((i + 1 == bpm ? 0u : (uint32_t)i + 1) << 24));
+  }
+  __syncwarp();
+}
+// from an ac1 table to the subtables of its long codes
+static_assert(sizeof(CJSpecTab::sub[0]) == sizeof(CJSpecTab::ac1[0]), "sub follows ac1 at one distance");
+#define CJ_SPEC_SUB ((uint32_t)(offsetof(CJSpecTab, sub) - offsetof(CJSpecTab, ac1)))
+
+// A warp's shared memory in the speculative decode.
 struct CJSpecWarp {
   uint32_t ring[CJ_RING_WORDS][32];
   uint2 phase[CJ_MAX_BPM];
@@ -370,11 +349,11 @@ struct CJSpecJob {
   CJSubRec r;
 };
 __device__ __forceinline__ void cj_spec_job(CJSpecJob& x, const CJScanParams& sp, const CJScanParams& tp,
-                                            const CJSpecTab& tab, const void* data, const CJLane& ln, CJCkpt* ck,
+                                            uint32_t tab, const void* data, const CJLane& ln, CJCkpt* ck,
                                             uint32_t cstep, const CJSpecWarp& sw) {
   x.sp = &sp;
   x.tp = &tp;
-  x.tab = (uint32_t)__cvta_generic_to_shared(&tab);
+  x.tab = tab;
   x.data = reinterpret_cast<const uint4*>(data);
   x.begin = (uint32_t)ln.begin;
   x.end = (uint32_t)ln.end;
@@ -394,25 +373,11 @@ __device__ __forceinline__ void cj_spec_job(CJSpecJob& x, const CJScanParams& sp
 template <bool HYP>
 __device__ __noinline__ void cj_spec_warp(CJSpecJob* job, bool run, uint64_t start) {
   CJSpecJob& x = *job;
-  CJWin br;
+  CJWin<CJ_RING_WORDS> br;
   const uint32_t begin = x.begin, end = x.end, cstep = x.cstep, phases = x.phase;
   CJCkpt* const ck = x.ck;
   const int bpm = x.sp->bpm;
-  {  // the phase entries of this image and these tables
-    const int i = threadIdx.x & 31;
-    __syncwarp();
-    if (i < bpm) {
-      const uint32_t c = x.sp->phase_comp[i], d = x.sp->comp_dc[c], a = x.sp->comp_ac[c] - 2u;
-      const uint32_t dc = x.tab + (uint32_t)offsetof(CJSpecTab, dc) + d * (uint32_t)sizeof(CJSpecTab::dc[0]);
-      const uint32_t ac1 = x.tab + (uint32_t)offsetof(CJSpecTab, ac1) + a * (uint32_t)sizeof(CJSpecTab::ac1[0]);
-      const uint32_t acm = x.tab + a * (uint32_t)sizeof(CJSpecTab::acm[0]);
-      cj_sts32(phases + 8 * i, dc | (acm << 16));
-      cj_sts32(phases + 8 * i + 4, ac1 | (c << 16) | ((i + 1 == bpm ? 0u : (uint32_t)i + 1) << 24));
-    }
-    __syncwarp();
-  }
-  static_assert(sizeof(CJSpecTab::sub[0]) == sizeof(CJSpecTab::ac1[0]), "sub follows ac1 at one distance");
-  constexpr uint32_t SUB = (uint32_t)(offsetof(CJSpecTab, sub) - offsetof(CJSpecTab, ac1));
+  cj_phase_entries(*x.sp, x.tab, phases);
   int c = 0, k = -1, nb = 0, d0 = 0, d1 = 0, d2 = 0, j = 0;
   uint32_t dcv = 0, dce = 0, thresh = cstep;
   uint32_t next = cj_state_phase(start);  // phase of the block after the current one
@@ -477,7 +442,7 @@ __device__ __noinline__ void cj_spec_warp(CJSpecJob* job, bool run, uint64_t sta
     k += (int)(st >> 9);
     const bool prefix = st < (1u << 9);
     const bool high = k > CJ_MULTI_MAXK;
-    tab = prefix ? ac1 + SUB + ((st & 0x1E0u) << 2) : (high ? ac1 : acm);
+    tab = prefix ? ac1 + CJ_SPEC_SUB + ((st & 0x1E0u) << 2) : (high ? ac1 : acm);
     sh = prefix ? 26 : (high ? 32 - CJ_FAST_BITS : 32 - CJ_MULTI_BITS);
   };
   uint32_t p = br.pos;  // the last block boundary
@@ -666,133 +631,185 @@ __device__ __forceinline__ int64_t cj_lane_write_end(const CJLane& ln, const CJS
   return end > bend ? bend : end;
 }
 
+// A warp's shared memory in the write-out.
+struct CJWriteWarp {
+  uint32_t ring[CJ_WRITE_WORDS][32];
+  uint2 phase[CJ_MAX_BPM];
+  uint32_t order[32];  // completed blocks of a round
+};
+
+// One lane's unit of the write-out (sp .. coef agree over the warp).
+struct CJWriteJob {
+  const CJScanParams *sp, *tp;
+  CJStatus* st;
+  const uint4* data;
+  int16_t* coef;  // of block `base`
+  int64_t base;   // blk and bend count from here
+  uint32_t tab, ring, phase, order, wbuf, zz;  // shared addresses (wbuf: the warp's 32 blocks; zz: 2 x zig-zag index)
+  uint32_t end_byte, end, stop, seg_end;       // bits: of the subsequence, of the unit, of the segment
+  uint32_t pos, m;                             // the unit's first block
+  int blk, bend, dc[3];
+  bool last, marker;  // the segment's last subsequence; an RSTn follows the segment
+  bool cut;           // out: stopped inside block blk at an error
+};
+
 // Warp-cooperative write-out of 32 units (one per lane; `active` = false for
 // lanes without one), symbol for symbol the serial block decode with the
-// same structural checks.  Each lane builds its current block in its own
-// 64-entry int16 buffer in shared memory (`wbuf` + lane * 64, all zero on
-// entry and on return).  After every symbol the warp stores the blocks its
-// lanes completed in that step: 8 lanes per block, 4 blocks per round, one
+// same structural checks, as straight-line rounds of three symbols (see
+// cj_spec_warp).  Each lane builds its current block in its own 64-entry int16
+// buffer in shared memory (all zero on entry and on return; the 16-byte chunks
+// of lane l are permuted by l mod 8, so equal positions of different lanes fall
+// into different banks).  After every round the warp stores the blocks its
+// lanes completed: 8 lanes per block, 4 blocks at a time, one
 // 16-byte store each -- a whole 128-byte line per block instead of one
 // scattered 2-byte store per coefficient -- and clears those buffers.  Blocks
 // go to memory whole, so the range needs no zero fill; a unit that stops at
-// an error stores its partial block (as the serial decode leaves it) and zeroes
-// the rest of its range, up to `zero_end`.
-__device__ __forceinline__ void cj_write_units_warp(const CJScanParams& sp, const CJScanParams& tp, const uint32_t* words,
-                                                    const CJLane& ln, const CJSegment& seg, uint64_t start,
-                                                    int64_t first_block, int dc0, int dc1, int dc2,
-                                                    int16_t* __restrict__ coef, CJStatus* st, const uint8_t* zz,
-                                                    uint64_t stop, int64_t zero_end, bool active, int16_t* wbuf) {
+// an error stores its partial block (as the serial decode leaves it).
+// Measured on the 1024-image mix: 1.05 ms with a branch per event, tables in
+// global memory and a store loop per symbol; 0.72 ms as here (48 1080p frames
+// 0.35 -> 0.23, 512 thumbnails 0.25 -> 0.12).
+static __device__ __noinline__ void cj_write_warp(CJWriteJob* job, bool active) {
+  CJWriteJob& x = *job;
   const int lane = threadIdx.x & 31;
-  int16_t* mine = wbuf + lane * 64;
-  int64_t b = first_block;
-  const int64_t bend = seg.first_block + seg.nblocks;
-  const uint64_t seg_end = seg.bit_end;
-  const int bpm = sp.bpm;
-  const uint64_t pack = sp.phase_pack;
-  CJFBits br;
-  uint32_t m = 0, aslot = 0, slot = 0;
-  int c = 0;
-  if (active) {
-    br.init(words, ln.end_byte, cj_state_bit(start));
-    m = cj_state_phase(start);
-    cj_phase(sp, bpm, pack, m, c, slot, aslot);
-  }
-  int k = -1;
-  int32_t dd = 0;
-  bool cut = false;  // stopped inside block b at an error
-  // the structural checks made before every block; false = stop here
-  auto block_start = [&]() -> bool {
-    const uint64_t p = br.pos();
-    if (p >= stop) return false;  // the next unit's first block
-    if (!ln.last && p >= ln.end) return false;
-    if (b >= bend) {
-      if (!ln.last) cj_raise_dec(st, b, CJ_DEV_EXTRA);
-      else if (seg.marker_follows) {
-        if (((p + 7) >> 3) != ln.end_byte) cj_raise_dec(st, b, CJ_DEV_TRAILING);
-      } else if (ln.end_byte > ((p + 7) >> 3) + 2) {
-        cj_raise_dec(st, b, CJ_DEV_TRAILING);
-      }
-      return false;
-    }
-    if (seg.marker_follows && p >= seg_end) {
-      cj_raise_dec(st, b, CJ_DEV_OVERRUN);
-      return false;
-    }
-    return true;
+  cj_phase_entries(*x.sp, x.tab, x.phase);
+  CJWin<CJ_WRITE_WORDS> br;
+  const uint32_t mine = x.wbuf + 128 * lane, swz = (uint32_t)(lane & 7) << 4, zz = x.zz;
+  // (copies: the compiler reads a job's fields from local memory again after
+  // every shared-memory store of the loop)
+  const uint32_t phases = x.phase, seg_end = x.marker ? x.seg_end : 0xFFFFFFFFu, order = x.order;
+  const uint32_t wsrc = x.wbuf;
+  uint4* const out = reinterpret_cast<uint4*>(x.coef) + (lane & 7);
+  // a block does not start here by itself: the unit's or lane's end, or past the marker
+  uint32_t lim = min(x.stop, x.last ? 0xFFFFFFFFu : x.end);
+  lim = min(lim, seg_end);
+  int b = x.blk, dc0 = x.dc[0], dc1 = x.dc[1], dc2 = x.dc[2];
+  const int bend = x.bend;
+  bool cut = false;
+  uint32_t next = x.m;
+  uint2 ph = make_uint2(cj_lds32(phases + 8 * next), cj_lds32(phases + 8 * next + 4));
+  uint32_t tab, sh, ac1;
+  int c, k = -1, dd = 0;
+  auto begin_block = [&]() {
+    tab = ph.x & 0xFFFFu;
+    sh = 32 - CJ_MULTI_DC_BITS;
+    ac1 = ph.y & 0xFFFFu;
+    c = (int)((ph.y >> 16) & 255);
+    next = ph.y >> 24;
+    ph.x = cj_lds32(phases + 8 * next);
+    ph.y = cj_lds32(phases + 8 * next + 4);
+    k = -1;
   };
-  bool run = active && block_start();
-  for (;;) {
-    int done = -1;  // block (of this image) to store after this step
-    if (run) {
-      const uint32_t v = br.peek();
-      const uint32_t stp = cj_step(tp, slot, v);
-      const uint32_t dk = (stp >> 5) & 127, size = stp >> 12, total = stp & 31;
-      const int kn = k + (int)dk;
-      const uint32_t len = total - size;
-      const int32_t val = size ? cj_extend((v << len) >> (32 - size), size) : 0;
-      if (k < 0) dd = val;
-      else if (size && kn <= 63) mine[zz[kn]] = (int16_t)val;
-      br.skip(total - (kn > 63 ? size : 0u));
-      slot = aslot;
-      if (kn < 63) {
-        k = kn;
-      } else if (kn > 63 && dk != CJ_STEP_EOB) {  // failing symbol: the block is cut here
-        cj_raise_dec(st, b, dk == CJ_STEP_NO_CODE ? CJ_DEV_BAD_CODE : CJ_DEV_BAD_AC);
-        done = (int)b;
-        cut = true;
-        run = false;
-      } else if (seg.marker_follows && br.pos() > seg_end) {
-        cj_raise_dec(st, b, CJ_DEV_OVERRUN);
-        done = (int)b;
-        cut = true;
-        run = false;
-      } else {
-        int dcv;
-        if (c == 0) dcv = dc0 += dd;
-        else if (c == 1) dcv = dc1 += dd;
-        else dcv = dc2 += dd;
-        if (dcv < -32768 || dcv > 32767) {
-          cj_raise_dec(st, b, CJ_DEV_DC_RANGE);
-          cut = true;
-          run = false;
-        } else {
-          mine[0] = (int16_t)dcv;
-          b++;
-          m = (m + 1 == (uint32_t)bpm) ? 0 : m + 1;
-          cj_phase(sp, bpm, pack, m, c, slot, aslot);
-          k = -1;
-          run = block_start();
-        }
-        done = (int)(cut ? b : b - 1);
-      }
+  // why no block starts at bit p (once per unit)
+  auto stopped = [&](uint32_t p) {
+    if (p >= x.stop || (!x.last && p >= x.end)) return;
+    if (b >= bend) {
+      if (!x.last) cj_raise_dec(x.st, x.base + b, CJ_DEV_EXTRA);
+      else if (x.marker ? ((p + 7) >> 3) != x.end_byte : x.end_byte > ((p + 7) >> 3) + 2)
+        cj_raise_dec(x.st, x.base + b, CJ_DEV_TRAILING);
+    } else {
+      cj_raise_dec(x.st, x.base + b, CJ_DEV_OVERRUN);
     }
-    unsigned mask = __ballot_sync(CJ_FULL, done >= 0);
-    __syncwarp();
-    while (mask) {  // warp-uniform: up to 4 blocks per round, lanes 8j..8j+7 take the j-th
-      const int s0 = __ffs(mask) - 1;
-      mask &= mask - 1;
-      const int s1 = __ffs(mask) - 1;
-      mask &= mask - 1;
-      const int s2 = __ffs(mask) - 1;
-      mask &= mask - 1;
-      const int s3 = __ffs(mask) - 1;
-      mask &= mask - 1;
-      const int j = lane >> 3;
-      const int src = j == 0 ? s0 : (j == 1 ? s1 : (j == 2 ? s2 : s3));
-      const int bsrc = __shfl_sync(CJ_FULL, done, src < 0 ? 0 : src);
-      if (src >= 0) {
-        uint4* s = reinterpret_cast<uint4*>(wbuf + src * 64) + (lane & 7);
-        reinterpret_cast<uint4*>(coef + (int64_t)bsrc * 64)[lane & 7] = *s;
-        *s = make_uint4(0, 0, 0, 0);
-      }
-    }
-    __syncwarp();
-    if (!__any_sync(CJ_FULL, run)) break;
+  };
+  br.pos = x.pos;
+  br.col = x.ring;
+  br.cur = br.nxt = br.nn = 0;
+  bool live = active;
+  if (live && (br.pos >= lim || b >= bend)) {
+    stopped(br.pos);
+    live = false;
   }
-  // blocks of the range an early stop left undecoded read as zeros
-  for (int64_t x = cut ? b + 1 : b; active && x < zero_end; x++) {
-    uint4* p = reinterpret_cast<uint4*>(coef + x * 64);
+  if (live) br.init(x.data, x.ring, x.end_byte, br.pos);
+  begin_block();
+  if (!live) k = 63;
+  uint32_t lst = 0;  // the block's last entry
+  // One symbol of entry st at window v; DC only where `dc` says so.
+  auto symbol = [&](uint32_t st, uint32_t v, bool dc) {
+    const uint32_t size = (st >> 5) & 15, dk = st >> 9;
+    const uint32_t w = __funnelshift_l(0u, v, (st & 31) - size);
+    // (T.81 F.2.2.1: a magnitude whose first bit is 0 is negative)
+    int val = (int)__funnelshift_rc(w, 0u, 32 - size);
+    val -= (int)w >= 0 ? (int)((1u << size) - 1u) : 0;
+    const bool isdc = dc && k < 0;
+    if (dc) dd = isdc ? val : dd;
+    br.skip(st & 31);
+    k += (int)dk;
+    if (size && dk - 1u < 16u && k <= 63 && !isdc) cj_sts16(mine + (cj_tab8(zz + k) ^ swz), (uint32_t)val);
+    const bool prefix = dk == 0;
+    tab = prefix ? ac1 + CJ_SPEC_SUB + ((st & 0x1E0u) << 2) : ac1;
+    sh = prefix ? 26 : 32 - CJ_FAST_BITS;
+  };
+  while (__any_sync(CJ_FULL, live)) {
+    if (live) br.refill();
+    __syncwarp();
 #pragma unroll
-    for (int i = 0; i < 8; i++) p[i] = make_uint4(0, 0, 0, 0);
+    for (int q = 0; q < CJ_STEPS_PER_ROUND; q++) {
+      const uint32_t v = br.peek();
+      uint32_t st = cj_tab16(tab + 2 * (v >> sh));
+      lst = k < 63 ? st : lst;
+      st = k < 63 ? st : 0;
+      symbol(st, v, q == 0);
+    }
+    bool done = false;
+    if (live && k >= 63) {
+      if (k >= CJ_SPEC_FARK) {  // rare: through the steps in memory
+        k -= (int)(CJ_SPEC_FAR >> 9);
+        const uint32_t v = br.peek();
+        lst = cj_spec_entry(cj_step(*x.tp, k < 0 ? x.sp->comp_dc[c] : x.sp->comp_ac[c], v), 0, k < 0);
+        symbol(lst, v, true);
+      }
+      if (k >= 63) {
+        done = true;
+        const uint32_t adv = lst >> 9;
+        // an EOB, or a symbol that landed on 63
+        const bool ok = adv == CJ_SPEC_EOB ? (lst & 0x1E0u) == 0 : k == 63 && adv <= 16;
+        if (!ok || br.pos > seg_end) {
+          cj_raise_dec(x.st, x.base + b, ok ? CJ_DEV_OVERRUN : CJ_DEV_BAD_AC);
+          cut = true;
+        } else {
+          int v = c == 0 ? dc0 : (c == 1 ? dc1 : dc2);
+          v += dd;
+          if (c == 0) dc0 = v;
+          else if (c == 1) dc1 = v;
+          else dc2 = v;
+          if (v < -32768 || v > 32767) {
+            cj_raise_dec(x.st, x.base + b, CJ_DEV_DC_RANGE);
+            cut = true;
+          } else {
+            cj_sts16(mine + swz, (uint32_t)v);
+          }
+        }
+      }
+    }
+    const unsigned mask = __ballot_sync(CJ_FULL, done);
+    if (mask) {
+      if (done) cj_sts32(order + 4 * __popc(mask & ((1u << lane) - 1u)), ((uint32_t)b << 5) | (uint32_t)lane);
+      __syncwarp();
+      const int n = __popc(mask);
+      for (int r = lane >> 3; r < ((n + 3) & ~3); r += 4) {  // warp-uniform count
+        if (r < n) {
+          const uint32_t o = cj_lds32(order + 4 * r), src = o & 31;
+          const uint32_t at = wsrc + 128 * src + ((((uint32_t)lane ^ src) & 7u) << 4);
+          const uint4 z = cj_lds128(at);
+          out[(int64_t)((int32_t)o >> 5) * 8] = z;
+          cj_sts128_zero(at);
+        }
+      }
+      __syncwarp();
+      if (done) {
+        if (cut) {
+          live = false;
+        } else {
+          b++;
+          begin_block();
+          if (br.pos >= lim || b >= bend) {
+            stopped(br.pos);
+            live = false;
+          }
+        }
+        if (!live) k = 63;
+      }
+    }
   }
+  x.blk = b;
+  x.cut = cut;
 }
