@@ -46,8 +46,8 @@
 #define BT_THREADS 256
 // Default bits per speculative subsequence of a batch: with many images
 // decoding side by side, long subsequences (fewer lanes and settle chains)
-// win; the autotuner chooses 4096 on the mixed 1024-image workload.  The
-// single-image paths keep CJ_SUB_BITS_DEFAULT (more lanes per image).
+// win; the autotuner chooses 4096 on the mixed 1024-image workload.  A batch or
+// file that leaves the GPU unfilled takes shorter ones (bt_fill_bits).
 #define BT_SUB_BITS_DEFAULT 4096
 #define BT_WARPS (BT_THREADS / 32)
 // MCU-phase hypotheses per subsequence at most (the standard's largest MCU
@@ -1664,6 +1664,7 @@ struct CJBatch {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   // tuning (cjBatchSetTuning / cjBatchAutotune)
   int sub_bits = BT_SUB_BITS_DEFAULT;
+  bool sub_bits_auto = true;  // no size set: each stage picks one by the batch's fill (bt_fill_bits)
   int sub_bits_class[CJ_SAMPLING_CLASSES] = {0, 0, 0, 0, 0};  // 0: sub_bits
   int decode_ctas = BT_DECODE_CTAS_DEFAULT;  // decode-kernel CTAs per SM (3, 4 or 5)
   int tile_cap = 0;                          // max MCUs per pixel tile (0 = layout maximum)
@@ -1814,6 +1815,8 @@ static int bt_parse(CJBatch* b, const unsigned char* data, size_t size, CJImageH
   return 0;
 }
 
+static int bt_sub_cap(int64_t scan_len, int nseg, int sub_bits);
+
 // The plan of one image alone at the start of every buffer: destuff tiles,
 // markers, segments, subsequences of `sub_bits`, pixel tiles.
 static void bt_plan_one(const CJImageHeader& h, int64_t scan_len, int sub_bits, CJImageDesc* d) {
@@ -1825,7 +1828,7 @@ static void bt_plan_one(const CJImageHeader& h, int64_t scan_len, int sub_bits, 
   d->mark_cap = h.nseg_expected + 1;
   d->seg_cap = h.nseg_expected;
   d->sub_bits = sub_bits;
-  d->sub_cap = ((int)((scan_len * 8 + sub_bits - 1) / sub_bits) + h.nseg_expected + 1 + 31) & ~31;
+  d->sub_cap = bt_sub_cap(scan_len, h.nseg_expected, sub_bits);
   d->T = cj_pix_tile_mcus(h.hmax, bpm);
   d->nptiles = h.mcuy * ((h.mcux + d->T - 1) / d->T);
 }
@@ -1874,6 +1877,46 @@ static int bt_sub_bits_for(const CJBatch* b, const CJImageHeader& h) {
   return c ? c : b->sub_bits;
 }
 
+// Subsequences (a multiple of 32) an image may need at a size.
+static int bt_sub_cap(int64_t scan_len, int nseg, int sub_bits) {
+  return ((int)((scan_len * 8 + sub_bits - 1) / sub_bits) + nseg + 1 + 31) & ~31;
+}
+
+// The subsequence size of a decode for which none is set, and whether it runs
+// with MCU-phase hypotheses.  `warps(S)`: its warps at size S.
+//
+// Short subsequences shorten the serial chain (a decode of S bits takes
+// about 25 ns per bit), long ones repeat less work in the settle; which counts
+// depends on whether the SMs have warps to spare.  Up to 8 warps per SM a chain
+// runs at full speed, so the smallest size that stays within that is taken,
+// and the batch default beyond.  Device time at 4096 / 2048 / 1024 / 512 bits:
+// 40 mixed photos (222 warps at 1024) 0.66 / 0.34 / 0.34 / 0.35 ms, 512
+// thumbnails (857 at 1024) 0.44 / 0.39 / 0.39 / 0.44, 24 large photos (647 at
+// 2048) 0.94 / 0.87 / 0.94 / 1.00, 48 1080p frames (994 at 4096) 1.18 / 1.16 /
+// 1.38, one 24-megapixel 4:2:2 file (1106 at 1024) - / 0.44 / 0.43 / 0.48.
+//
+// Hypotheses (one image, or a batch small enough): only for MCUs of
+// 5 blocks and more, where a decode out of step with the MCU phase stays so for
+// thousands of bits, and up to 16 warps per SM of them.  One 4:2:0 file
+// with / without: 1024x768 0.22 / 0.30 ms, 4096x4096 0.44 / 0.70; 4:2:2
+// 1024x768 0.19 / 0.15, 4:4:4 0.17 / 0.13.
+#define BT_FILL_WARPS 8
+#define BT_FILL_HYP 16
+#define BT_HYP_MIN_BPM 5
+template <class F>
+static int bt_fill_bits(int from, int to, int sms, F warps) {
+  int bits = from;
+  while (bits < to && warps(bits) > (int64_t)BT_FILL_WARPS * sms) bits *= 2;
+  return bits;
+}
+// The same for one image with `nh` hypotheses; 0: they do not fit.
+template <class F>
+static int bt_fill_bits_hyp(int from, int to, int sms, int nh, F warps) {
+  for (int bits = from; bits <= to; bits *= 2)
+    if (warps(bits) * nh <= (int64_t)BT_FILL_HYP * sms) return bits;
+  return 0;
+}
+
 static bool bt_sub_bits_ok(int bits) { return bits >= 128 && bits <= 65536 && !(bits & 31); }
 
 extern "C" {
@@ -1891,9 +1934,11 @@ int cjBatchGetSubsequenceBitsFor(const CJBatch* b, int sampling_class) {
 }
 
 int cjBatchSetSubsequenceBits(CJBatch* b, int bits) {
-  if (bits == 0) bits = BT_SUB_BITS_DEFAULT;
+  const bool automatic = bits == 0;
+  if (automatic) bits = BT_SUB_BITS_DEFAULT;
   if (!b || !bt_sub_bits_ok(bits)) return PROGRAMMER_ERROR;
   b->sub_bits = bits;
+  b->sub_bits_auto = automatic;
   return 0;
 }
 
@@ -2119,11 +2164,9 @@ int cjBatchStage(CJBatch* b, int n, const unsigned char* blob, const int64_t* of
     d.seg_cap = h.nseg_expected;
     nseg += d.seg_cap;
     d.sub_bits = bt_sub_bits_for(b, h);
-    int sub_cap = (int)((sl * 8 + d.sub_bits - 1) / d.sub_bits) + h.nseg_expected + 1;
-    sub_cap = (sub_cap + 31) & ~31;
+    d.sub_cap = bt_sub_cap(sl, h.nseg_expected, d.sub_bits);
     d.sub0 = nsubw * 32;
-    d.sub_cap = sub_cap;
-    nsubw += sub_cap / 32;
+    nsubw += d.sub_cap / 32;
     int bpm = (int)(h.total_blocks / ((int64_t)h.mcux * h.mcuy));
     d.T = b->idct == CJ_PIX_IDCT_TC ? cj_pix_tile_mcus_tc(h.hmax, bpm) : cj_pix_tile_mcus(h.hmax, bpm);
     while (b->tile_cap > 0 && d.T > b->tile_cap && d.T > 1) d.T >>= 1;
@@ -2160,6 +2203,29 @@ int cjBatchStage(CJBatch* b, int n, const unsigned char* blob, const int64_t* of
     b->dims.push_back(h.nch == 3 ? (h.height * h.comp_sy[1] + h.vmax - 1) / h.vmax : 0);
     b->outoff.push_back(fancy ? d.rgb_off : d.out_off);
     nd++;
+  }
+  if (b->sub_bits_auto && nd) {  // the size by the batch's fill, for the classes that follow it
+    auto own = [&](int k) { return b->sub_bits_class[bt_sampling_class(hh[k])] != 0; };
+    auto warps = [&](int bits) {
+      int64_t w = 0;
+      for (int k = 0; k < nd; k++)
+        w += (own(k) ? dd[k].sub_cap : bt_sub_cap(dd[k].raw_len, hh[k].nseg_expected, bits)) / 32;
+      return w;
+    };
+    const int bpm = (int)(hh[0].total_blocks / ((int64_t)hh[0].mcux * hh[0].mcuy));
+    int bits = 0;
+    if (nd == 1 && b->hyp_enabled && bpm >= BT_HYP_MIN_BPM)
+      bits = bt_fill_bits_hyp(512, BT_SUB_BITS_DEFAULT, b->sm_count, std::min(bpm, BT_MAX_HYP), warps);
+    if (!bits) bits = bt_fill_bits(1024, BT_SUB_BITS_DEFAULT, b->sm_count, warps);
+    nsubw = 0;
+    for (int k = 0; k < nd; k++) {
+      if (!own(k)) {
+        dd[k].sub_bits = bits;
+        dd[k].sub_cap = bt_sub_cap(dd[k].raw_len, hh[k].nseg_expected, bits);
+      }
+      dd[k].sub0 = nsubw * 32;
+      nsubw += dd[k].sub_cap / 32;
+    }
   }
   b->n_dev = nd;
   // a colour image (both table pairs) can serve grey ones too
@@ -2220,9 +2286,8 @@ int cjBatchStage(CJBatch* b, int n, const unsigned char* blob, const int64_t* of
               CUDA_KERNEL_LAUNCH_ERROR);
   if (per_sm < 1) return UNSUPPORTED_ERROR;
   b->grid = std::min(per_sm, b->decode_ctas) * b->sm_count;
-  // MCU-phase hypotheses only where their decodes fit beside the batch's own
-  // warps in one round of the grid: a batch of a few images leaves most of
-  // the GPU idle while its settle chains run, a full batch has no room
+  // MCU-phase hypotheses where they pay and their decodes fit beside the
+  // batch's own warps (bt_fill_bits)
   b->nhyp = 1;
   if (b->hyp_enabled) {
     int maxbpm = 1;
@@ -2236,7 +2301,7 @@ int cjBatchStage(CJBatch* b, int n, const unsigned char* blob, const int64_t* of
     CJ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
                     &per_sm_hyp, (const void*)bt_decode_kernel(b->decode_ctas, true), BT_THREADS, bt_decode_smem(nh)),
                 CUDA_KERNEL_LAUNCH_ERROR);
-    if (nh > 1 && per_sm_hyp > 0 && (int64_t)nsubw * nh <= (int64_t)b->grid * BT_WARPS) {
+    if (nh >= BT_HYP_MIN_BPM && per_sm_hyp > 0 && (int64_t)nsubw * nh <= (int64_t)BT_FILL_HYP * b->sm_count) {
       const size_t nsub = (size_t)nsubw * 32, nrec = nsub * 2 * nh;  // hypotheses and probes
       if (bt_ensure(b, b->hrecs, nrec * sizeof(CJSubRec)) || bt_ensure(b, b->hckpt, nrec * CJ_CKPTS * sizeof(CJCkpt)) ||
           bt_ensure(b, b->hmap, nsub * 16))
@@ -2589,6 +2654,7 @@ int cjBatchAutotune(CJBatch* b, int n, const unsigned char* blob, const int64_t*
     if (trials_ms && trial < max_trials) trials_ms[trial] = ms;
     trial++;
   };
+  b->sub_bits_auto = false;  // from here on the size is the measured one
   // 1. subsequence size x decode-kernel occupancy (one size for every class)
   for (int k = 0; k < CJ_SAMPLING_CLASSES; k++) b->sub_bits_class[k] = 0;
   for (int sb : subs)
@@ -2689,13 +2755,11 @@ int cj_reader_decode(JPGReader* jpg, bool stage) {
     for (int c = 0; c < h.nch; c++) bpm += h.comp_sx[c] * h.comp_sy[c];
     const int nh = std::min(bpm, BT_MAX_HYP);
     CJImageDesc desc;
-    // the default size: 512-bit subsequences (more, shorter speculative
-    // decodes: the lowest latency) when their hypothesis decodes still fit
-    // in one round of the grid, else 1024 bits
     int sub = d->sub_bits;
     if (d->sub_bits_auto) {
-      bt_plan_one(h, n, 512, &desc);
-      sub = (int64_t)(desc.sub_cap / 32) * std::max(nh, 1) <= (int64_t)cap * BT_WARPS ? 512 : CJ_SUB_BITS_DEFAULT;
+      auto warps = [&](int bits) { return (int64_t)(bt_sub_cap(n, h.nseg_expected, bits) / 32); };
+      sub = bpm >= BT_HYP_MIN_BPM ? bt_fill_bits_hyp(512, BT_SUB_BITS_DEFAULT, sms, nh, warps) : 0;
+      if (!sub) sub = bt_fill_bits(512, BT_SUB_BITS_DEFAULT, sms, warps);
     }
     bt_plan_one(h, n, sub, &desc);
     const int nwarps = desc.sub_cap / 32;
@@ -2714,12 +2778,11 @@ int cj_reader_decode(JPGReader* jpg, bool stage) {
         cj_dev_ensure(d->coef, (size_t)h.total_blocks * 128 + 128) || cj_dev_ensure(d->bctl, sizeof(CJBatchCtl)))
       return CUDA_MEM_ERROR;
     if (cj_host_ensure(d->h_bctl, sizeof(CJBatchCtl))) return OOM_ERROR;
-    // MCU-phase hypotheses when their decodes fit in one round of the grid
-    // (one image leaves most of the GPU idle while its settle chains run)
+    // MCU-phase hypotheses where they pay and fit (bt_fill_bits)
     d->b_nhyp = 1;
     int cap_run = cap;  // co-resident CTAs of the variant that runs
     const int groups = (nwarps + BT_WARPS - 1) / BT_WARPS;
-    if (nh > 1 && (int64_t)nwarps * nh <= (int64_t)cap * BT_WARPS) {
+    if (nh >= BT_HYP_MIN_BPM && (int64_t)nwarps * nh <= (int64_t)BT_FILL_HYP * sms) {
       int per_hyp = 0;
       CJ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_hyp, (const void*)bt_decode_kernel(BT_HYP_CTAS, true),
                                                                 BT_THREADS, bt_decode_smem(nh)),

@@ -31,9 +31,8 @@ void cjReaderSetFlags(JPGReader *r, int flags);
 
 /* Bits per speculative subsequence of the parallel Huffman decode
  * (multiple of 32, 128..65536); 0 restores the default, which picks per
- * image: 512 bits where the MCU-phase hypothesis decodes of so many
- * subsequences still fit in one round of the GPU (small images, the lowest
- * latency), else 1024. */
+ * image: the smallest of 512, 1024, 2048 and 4096 bits whose decodes (with the
+ * MCU-phase hypotheses of a 4:2:0 image) leave the GPU's warps at full speed. */
 int cjReaderSetSubsequenceBits(JPGReader *r, int bits);
 
 /* Device time of the last decode split by stage, in milliseconds:
@@ -127,7 +126,8 @@ void cjBatchDestroy(CJBatch *b);
 int cjBatchSetSubsequenceBits(CJBatch *b, int bits);
 
 /* Tuning of later stages/runs: bits per speculative subsequence (0 =
- * default, 4096 for a batch; multiple of 32, 128..65536), decode-kernel CTAs per SM (3, 4 or 5,
+ * default: 4096 for a full batch, less for one that leaves the GPU unfilled;
+ * multiple of 32, 128..65536), decode-kernel CTAs per SM (3, 4 or 5,
  * 0 = 4: the register budget per thread of the entropy kernel, 80/64/48), and
  * the largest pixel tile in MCUs (power of two, 0 = the layout maximum:
  * 128 pixels across). */
@@ -182,7 +182,8 @@ int cjBatchSetOutput(CJBatch *b, int format, int idct);
 int cjBatchSetParse(CJBatch *b, int on_device);
 /* MCU-phase hypotheses of the entropy decode (on != 0, the default): when a
  * staged batch's speculative decodes leave most of the GPU idle (a few
- * images), each subsequence of a multi-component scan is also decoded from
+ * images) and its MCUs have 5 blocks or more (4:2:0), each subsequence is also
+ * decoded from
  * its first bit under every other MCU phase and then from each of its
  * predecessor's hypothesis exits; the settle takes those decodes instead of
  * re-decoding lane after lane.  Results are identical either way; only the
