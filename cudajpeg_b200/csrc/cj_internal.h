@@ -4,6 +4,8 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include <vector>
+
 #include "../../include/format.h"
 #include "cj_core.h"
 
@@ -34,7 +36,9 @@ struct CJReaderDevice {
   CJHostHuff huff[4];
   uint16_t dq16[4][64];   // quantisation tables as parsed (8- or 16-bit), zig-zag order
   bool progressive = false;  // the frame is SOF2
-  int prog_scans = 0;        // progressive scans queued for this frame
+  int prog_scans = 0;        // progressive scans noted for this frame, and their parameter blocks and byte spans
+  std::vector<uint8_t> prog_blocks;
+  std::vector<int64_t> prog_spans;
   // GPU resources, created on the first scan
   bool gpu_ready = false;
   int device = -1;
@@ -94,8 +98,8 @@ struct CJProgScan {
 };
 // Check a progressive frame's SOS header at jpg->pos (0 or a format.h code).
 int cj_parse_prog_sos(JPGReader* jpg, CJProgScan* s);
-// Progressive frames (progressive.cu): queue one SOS's scan; at EOI, the
-// pixel stage's parameters.
+// Progressive frames (progressive.cu): note one SOS's scan; at EOI, decode the
+// scans and queue the pixel stage's parameters.
 int cj_prog_scan(JPGReader* jpg);
 int cj_prog_finish(JPGReader* jpg);
 // The scan's entropy decode as one image of the batch decode kernel
