@@ -1592,53 +1592,61 @@ struct alignas(16) CJParseSummary {
 static_assert(sizeof(CJParseSummary) == 80, "summary size");
 static_assert(sizeof(CJImageHeader) % 16 == 0, "headers are copied in 16-byte words");
 
-#define BT_PARSE_THREADS 128
+#define BT_PARSE_WARPS 4
 
-// The batch's marker parse on the GPU: thread i walks file i's marker
+// The batch's marker parse on the GPU: a warp walks file i's marker
 // segments (cj_parse_header) in the blob already copied to the device and
 // leaves its header in `hdr` (device memory).  The CTA's summaries are
 // written to `sum`, pinned host memory mapped into the device's address
 // space, as one contiguous run of 16-byte stores: they reach the host
 // without a device-to-host copy (which would queue behind any other copy in
 // that direction).
-__global__ void __launch_bounds__(BT_PARSE_THREADS) k_parse_headers(const uint8_t* __restrict__ blob,
-                                                                   const int64_t* __restrict__ offsets,
-                                                                   const int64_t* __restrict__ sizes, int n,
-                                                                   CJImageHeader* hdr, CJParseSummary* sum) {
-  __shared__ CJParseSummary s_sum[BT_PARSE_THREADS];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(32 * BT_PARSE_WARPS) k_parse_headers(const uint8_t* __restrict__ blob,
+                                                                     const int64_t* __restrict__ offsets,
+                                                                     const int64_t* __restrict__ sizes, int n,
+                                                                     CJImageHeader* hdr, CJParseSummary* sum) {
+  __shared__ CJParseSummary s_sum[BT_PARSE_WARPS];
+  __shared__ alignas(16) CJImageHeader s_hdr[BT_PARSE_WARPS];
+  __shared__ uint32_t s_win[BT_PARSE_WARPS][CJ_PARSE_WINDOW / 4];
+  const int wp = threadIdx.x >> 5, i = blockIdx.x * BT_PARSE_WARPS + wp;
   if (i < n) {
     int64_t so = 0, sl = 0;
-    CJImageHeader* h = &hdr[i];
-    const int e = cj_parse_header(blob + offsets[i], sizes[i], h, &so, &sl);
-    CJParseSummary& q = s_sum[threadIdx.x];
-    q.scan_off = so;
-    q.scan_len = sl;
-    q.total_blocks = h->total_blocks;
-    q.err = e;
-    q.mcux = h->mcux;
-    q.mcuy = h->mcuy;
-    q.width = h->width;
-    q.height = h->height;
-    q.hmax = h->hmax;
-    q.vmax = h->vmax;
-    q.restart_interval = h->restart_interval;
-    q.nseg_expected = h->nseg_expected;
-    q.nch = h->nch;
-    q.huff_mask = h->huff_mask;
-    q.xshift = h->xshift;
-    q.yshift = h->yshift;
-    for (int c = 0; c < 3; c++) {
-      q.comp_dc[c] = h->comp_dc[c];
-      q.comp_ac[c] = h->comp_ac[c];
-      q.comp_q[c] = h->comp_q[c];
-      q.comp_sx[c] = h->comp_sx[c];
-      q.comp_sy[c] = h->comp_sy[c];
+    CJImageHeader* h = &s_hdr[wp];
+    const uint8_t* f = blob + offsets[i];
+    const int e = cj_parse_header(CJWarpBytes{f, s_win[wp], nullptr, f + sizes[i]}, sizes[i], h, &so, &sl);
+    __syncwarp();
+    for (int k = threadIdx.x & 31; k < (int)(sizeof(CJImageHeader) / 16); k += 32)
+      reinterpret_cast<uint4*>(&hdr[i])[k] = reinterpret_cast<const uint4*>(h)[k];
+    if ((threadIdx.x & 31) == 0) {
+      CJParseSummary& q = s_sum[wp];
+      q.scan_off = so;
+      q.scan_len = sl;
+      q.total_blocks = h->total_blocks;
+      q.err = e;
+      q.mcux = h->mcux;
+      q.mcuy = h->mcuy;
+      q.width = h->width;
+      q.height = h->height;
+      q.hmax = h->hmax;
+      q.vmax = h->vmax;
+      q.restart_interval = h->restart_interval;
+      q.nseg_expected = h->nseg_expected;
+      q.nch = h->nch;
+      q.huff_mask = h->huff_mask;
+      q.xshift = h->xshift;
+      q.yshift = h->yshift;
+      for (int c = 0; c < 3; c++) {
+        q.comp_dc[c] = h->comp_dc[c];
+        q.comp_ac[c] = h->comp_ac[c];
+        q.comp_q[c] = h->comp_q[c];
+        q.comp_sx[c] = h->comp_sx[c];
+        q.comp_sy[c] = h->comp_sy[c];
+      }
+      q.pad[0] = 0;
     }
-    q.pad[0] = 0;
   }
   __syncthreads();
-  const int first = blockIdx.x * blockDim.x, cnt = min((int)blockDim.x, n - first);
+  const int first = blockIdx.x * BT_PARSE_WARPS, cnt = min(BT_PARSE_WARPS, n - first);
   const uint4* src = reinterpret_cast<const uint4*>(s_sum);
   uint4* dst = reinterpret_cast<uint4*>(sum + first);
   const int words = cnt * (int)(sizeof(CJParseSummary) / 16);
@@ -2000,7 +2008,7 @@ int cjDebugParseCompare(const unsigned char* data, size_t size, int* err_host, i
     sl1 = (int64_t)(r->end - r->pos);
   }
   if (!e1 && (uint64_t)sl1 > CJ_MAX_SCAN_BYTES) e1 = UNSUPPORTED_ERROR;
-  const int e2 = cj_parse_header(data, (int64_t)size, h2, &so2, &sl2);
+  const int e2 = cj_parse_header(CJHostBytes{data}, (int64_t)size, h2, &so2, &sl2);
   *err_host = e1;
   *err_parse = e2;
   int diff = 0;
@@ -2091,7 +2099,7 @@ int cjBatchStage(CJBatch* b, int n, const unsigned char* blob, const int64_t* of
     CJ_CUDA_TRY(cudaMemcpyAsync(b->blob.p, blob, (size_t)blob_bytes, cudaMemcpyHostToDevice, s), CUDA_MEM_ERROR);
     CJ_CUDA_TRY(cudaMemcpyAsync(b->p_size.p, hs, nn * 16, cudaMemcpyHostToDevice, s), CUDA_MEM_ERROR);
     const int64_t* d_off = (const int64_t*)b->p_size.p;
-    k_parse_headers<<<(n + BT_PARSE_THREADS - 1) / BT_PARSE_THREADS, BT_PARSE_THREADS, 0, s>>>(
+    k_parse_headers<<<(n + BT_PARSE_WARPS - 1) / BT_PARSE_WARPS, 32 * BT_PARSE_WARPS, 0, s>>>(
         (const uint8_t*)b->blob.p, d_off, d_off + n, n, (CJImageHeader*)b->p_hdr.p, b->d_psum);
     CJ_CUDA_TRY(cudaGetLastError(), CUDA_KERNEL_LAUNCH_ERROR);
     b->launches++;

@@ -1,6 +1,6 @@
 // cj_parse.cuh -- the marker-segment parse of one JPEG file up to its scan,
 // as one function that runs on the host and on the device.  The batch
-// decoder runs it on the GPU, one thread per file (k_parse_headers in
+// decoder runs it on the GPU, one warp per file (k_parse_headers in
 // batch.cu), over the files it has already copied to the device; it yields
 // the same header, scan range and error code as the host marker loop of the
 // drop-in path (format.cu cj_marker_loop with stop_at_scan, scan.cu
@@ -25,7 +25,59 @@ struct CJImageHeader {
   int64_t total_blocks;
 };
 
-CJ_HD unsigned cj_rd16(const uint8_t* p) { return ((unsigned)p[0] << 8) | p[1]; }
+// The parse reads a file through a byte source B: an indexable position (b[i],
+// b + i) that also says how many threads run the same parse side by side
+// (table copies are shared out over them).  On the host that is a pointer and
+// one thread.
+struct CJHostBytes {
+  const uint8_t* p;
+  CJ_HD uint8_t operator[](int64_t i) const { return p[i]; }
+  CJ_HD CJHostBytes operator+(int64_t d) const { return CJHostBytes{p + d}; }
+  CJ_HD int lane() const { return 0; }
+  CJ_HD int lanes() const { return 1; }
+  CJ_HD bool any(bool x) const { return x; }
+  CJ_HD void sync() const {}
+  CJ_HD void seek(int64_t) {}
+};
+
+#ifdef __CUDACC__
+// On the device a warp parses one file: the bytes around the segment at hand lie
+// in shared memory (CJ_PARSE_WINDOW of them, moved along by seek()), the rest is
+// read from global memory.  Headers fit one window; one thread per file reading
+// global memory byte by byte took 430 us for 1024 files (a chain of some 600
+// L2 round trips), a warp per file 31 us.
+#define CJ_PARSE_WINDOW 2048
+struct CJWarpBytes {
+  const uint8_t* g;  // position 0 of the view
+  uint32_t* win;     // CJ_PARSE_WINDOW / 4 + 1 words of shared memory
+  const uint8_t* w0;  // global address of the window's first byte (4-byte aligned)
+  const uint8_t* lim;  // end of the file
+  __device__ uint8_t operator[](int64_t i) const {
+    const uint8_t* a = g + i;
+    const int64_t o = a - w0;
+    return o >= 0 && o < CJ_PARSE_WINDOW ? reinterpret_cast<const uint8_t*>(win)[o] : *a;
+  }
+  __device__ CJWarpBytes operator+(int64_t d) const { return CJWarpBytes{g + d, win, w0, lim}; }
+  __device__ int lane() const { return threadIdx.x & 31; }
+  __device__ int lanes() const { return 32; }
+  __device__ bool any(bool x) const { return __any_sync(0xFFFFFFFFu, x); }
+  __device__ void sync() const { __syncwarp(); }
+  // Every lane: make the window cover what follows position i.
+  __device__ void seek(int64_t i) {
+    const uint8_t* a = g + i;
+    if (w0 && a >= w0 && a + 768 <= w0 + CJ_PARSE_WINDOW) return;
+    __syncwarp();
+    w0 = reinterpret_cast<const uint8_t*>(reinterpret_cast<uintptr_t>(a) & ~(uintptr_t)3);
+    // (the words of the window stay inside the blob: its buffer has 64 bytes behind the last file)
+    for (int k = lane(); k < CJ_PARSE_WINDOW / 4; k += 32)
+      win[k] = w0 + 4 * k < lim ? reinterpret_cast<const uint32_t*>(w0)[k] : 0u;
+    __syncwarp();
+  }
+};
+#endif
+
+template <class B>
+CJ_HD unsigned cj_rd16(const B& p) { return ((unsigned)p[0] << 8) | p[1]; }
 
 // Frame state the segments build up (a fresh one per file).
 struct CJParseState {
@@ -36,9 +88,10 @@ struct CJParseState {
 
 // SOF0 / SOF2 (src/format.cu:242-354): precision, size, components,
 // power-of-two sampling, the geometry the decoder supports.
-CJ_HD int cj_ps_sof(const uint8_t* buf, int64_t& pos, int64_t end, CJParseState& s) {
+template <class B>
+CJ_HD int cj_ps_sof(const B& buf, int64_t& pos, int64_t end, CJParseState& s) {
   if (pos > end) return SYNTAX_ERROR;
-  const uint8_t* block = buf + pos;
+  const B block = buf + pos;
   const unsigned block_len = cj_rd16(block);
   if (block_len < 9 || pos + block_len >= end) return SYNTAX_ERROR;
   if (block[2] != 8) return UNSUPPORTED_ERROR;
@@ -50,7 +103,7 @@ CJ_HD int cj_ps_sof(const uint8_t* buf, int64_t& pos, int64_t end, CJParseState&
   if (block_len < 8u + s.nch * 3u) return SYNTAX_ERROR;
   int sxm = 0, sym = 0;
   for (int i = 0; i < s.nch; i++) {
-    const uint8_t* c = block + 8 + 3 * i;
+    const B c = block + (8 + 3 * i);
     s.ids[i] = c[0];
     s.sx[i] = c[1] >> 4;
     s.sy[i] = c[1] & 0xF;
@@ -83,7 +136,8 @@ CJ_HD int cj_ps_sof(const uint8_t* buf, int64_t& pos, int64_t end, CJParseState&
 // DHT (src/format.cu:357-400): table class and id, code-space overflow, at
 // most 256 symbols; kept in canonical (BITS, HUFFVAL) form per slot
 // (DC0, DC1, AC0, AC1).
-CJ_HD int cj_ps_dht(const uint8_t* buf, int64_t& pos, int64_t end, CJParseState& s, CJImageHeader* h) {
+template <class B>
+CJ_HD int cj_ps_dht(const B& buf, int64_t& pos, int64_t end, CJParseState& s, CJImageHeader* h) {
   if (pos > end) return SYNTAX_ERROR;
   const int64_t block_end = pos + cj_rd16(buf + pos);
   if (block_end > end) return SYNTAX_ERROR;
@@ -105,8 +159,8 @@ CJ_HD int cj_ps_dht(const uint8_t* buf, int64_t& pos, int64_t end, CJParseState&
       nsym += count;
     }
     if (nsym > 256) return UNSUPPORTED_ERROR;
-    for (int l = 0; l < 16; l++) h->counts[slot][l] = buf[p + 1 + l];
-    for (int k = 0; k < nsym; k++) h->symbols[slot][k] = buf[sym + k];
+    for (int l = buf.lane(); l < 16; l += buf.lanes()) h->counts[slot][l] = buf[p + 1 + l];
+    for (int k = buf.lane(); k < nsym; k += buf.lanes()) h->symbols[slot][k] = buf[sym + k];
     s.huff_defined |= 1 << slot;
     p = sym + nsym;
   }
@@ -117,7 +171,8 @@ CJ_HD int cj_ps_dht(const uint8_t* buf, int64_t& pos, int64_t end, CJParseState&
 
 // DQT (src/format.cu:424-442; 16-bit tables, Pq = 1, as the host parser
 // reads them, steps below 2^15).
-CJ_HD int cj_ps_dqt(const uint8_t* buf, int64_t& pos, int64_t end, CJImageHeader* h) {
+template <class B>
+CJ_HD int cj_ps_dqt(const B& buf, int64_t& pos, int64_t end, CJImageHeader* h) {
   if (pos > end) return SYNTAX_ERROR;
   const int64_t block_end = pos + cj_rd16(buf + pos);
   if (block_end > end) return SYNTAX_ERROR;
@@ -126,11 +181,13 @@ CJ_HD int cj_ps_dqt(const uint8_t* buf, int64_t& pos, int64_t end, CJImageHeader
     const int pq = buf[p] >> 4, id = buf[p] & 15;
     const int n = pq ? 129 : 65;
     if (pq > 1 || id > 3 || p + n > block_end) return SYNTAX_ERROR;
-    for (int k = 0; k < 64; k++) {
-      const unsigned v = pq ? cj_rd16(buf + p + 1 + 2 * k) : buf[p + 1 + k];
-      if (v > 32767) return UNSUPPORTED_ERROR;
+    bool big = false;
+    for (int k = buf.lane(); k < 64; k += buf.lanes()) {
+      const unsigned v = pq ? cj_rd16(buf + (p + 1 + 2 * k)) : buf[p + 1 + k];
+      big = big || v > 32767;
       h->dq[id][k] = (uint16_t)v;
     }
+    if (buf.any(big)) return UNSUPPORTED_ERROR;
     p += n;
   }
   if (p != block_end) return SYNTAX_ERROR;
@@ -139,12 +196,13 @@ CJ_HD int cj_ps_dqt(const uint8_t* buf, int64_t& pos, int64_t end, CJImageHeader
 }
 
 // DRI (src/format.cu:404-421).
-CJ_HD int cj_ps_dri(const uint8_t* buf, int64_t& pos, int64_t end, CJParseState& s) {
+template <class B>
+CJ_HD int cj_ps_dri(const B& buf, int64_t& pos, int64_t end, CJParseState& s) {
   if (pos > end) return SYNTAX_ERROR;
   const unsigned block_len = cj_rd16(buf + pos);
   if (block_len < 2 || pos + block_len > end) return SYNTAX_ERROR;
   if (block_len < 4) return SYNTAX_ERROR;
-  s.restart = (int)cj_rd16(buf + pos + 2);
+  s.restart = (int)cj_rd16(buf + (pos + 2));
   pos += block_len;
   return 0;
 }
@@ -152,9 +210,10 @@ CJ_HD int cj_ps_dri(const uint8_t* buf, int64_t& pos, int64_t end, CJParseState&
 // SOS of a progressive frame: only checked (the batch decoder takes
 // baseline frames): a valid header is UNSUPPORTED_ERROR, an invalid one a
 // SYNTAX_ERROR, as progressive.cu cj_parse_prog_sos decides.
-CJ_HD int cj_ps_prog_sos(const uint8_t* buf, int64_t pos, int64_t end, const CJParseState& s) {
+template <class B>
+CJ_HD int cj_ps_prog_sos(const B& buf, int64_t pos, int64_t end, const CJParseState& s) {
   if (pos + 2 > end) return SYNTAX_ERROR;
-  const uint8_t* p = buf + pos;
+  const B p = buf + pos;
   const unsigned hlen = cj_rd16(p);
   if (hlen < 6 || pos + hlen > end) return SYNTAX_ERROR;
   if (!s.nch) return SYNTAX_ERROR;
@@ -162,7 +221,7 @@ CJ_HD int cj_ps_prog_sos(const uint8_t* buf, int64_t pos, int64_t end, const CJP
   if (ns < 1 || ns > s.nch || hlen != 6u + 2u * ns) return SYNTAX_ERROR;
   int prev = -1, dc[3] = {0, 0, 0}, ac[3] = {0, 0, 0};
   for (int j = 0; j < ns; j++) {
-    const uint8_t* d = p + 3 + 2 * j;
+    const B d = p + (3 + 2 * j);
     int c = 0;
     while (c < s.nch && s.ids[c] != d[0]) c++;
     if (c == s.nch || c <= prev || (d[1] & 0xEE)) return SYNTAX_ERROR;
@@ -170,7 +229,7 @@ CJ_HD int cj_ps_prog_sos(const uint8_t* buf, int64_t pos, int64_t end, const CJP
     dc[j] = d[1] >> 4;
     ac[j] = (d[1] & 1) | 2;
   }
-  const uint8_t* t = p + 3 + 2 * ns;
+  const B t = p + (3 + 2 * ns);
   const int ss = t[0], se = t[1], ah = t[2] >> 4, al = t[2] & 15;
   if ((ss == 0) != (se == 0) || se > 63 || ss > se || (ss && ns != 1) || al > 13 || (ah && ah != al + 1))
     return SYNTAX_ERROR;
@@ -187,10 +246,13 @@ CJ_HD int cj_ps_prog_sos(const uint8_t* buf, int64_t pos, int64_t end, const CJP
 // component list, Ss/Se/Ah/Al; each component's own tables must be
 // defined), then the header of the batch decoder.  *scan_off / *scan_len:
 // the entropy-coded bytes (from after the SOS header to before the EOI).
-CJ_HD int cj_parse_header(const uint8_t* buf, int64_t size, CJImageHeader* h, int64_t* scan_off,
+template <class B>
+CJ_HD int cj_parse_header(B buf, int64_t size, CJImageHeader* h, int64_t* scan_off,
                           int64_t* scan_len) {
-  for (int k = 0; k < (int)sizeof(CJImageHeader); k++) reinterpret_cast<uint8_t*>(h)[k] = 0;
+  for (int k = buf.lane(); k < (int)sizeof(CJImageHeader); k += buf.lanes()) reinterpret_cast<uint8_t*>(h)[k] = 0;
+  buf.sync();  // the lanes' stores above precede those below
   *scan_off = *scan_len = 0;
+  if (size >= 4) buf.seek(0);
   if (size < 4 || buf[0] != 0xFF || buf[1] != 0xD8 || buf[size - 2] != 0xFF || buf[size - 1] != 0xD9)
     return FILE_ERROR;
   if (size < 6) return SYNTAX_ERROR;
@@ -203,7 +265,9 @@ CJ_HD int cj_parse_header(const uint8_t* buf, int64_t size, CJImageHeader* h, in
   s.progressive = 0;
   s.width = s.height = s.mcux = s.mcuy = s.sxmax = s.symax = 0;
   for (;;) {
-    if (pos > end || buf[pos] != 0xFF) return SYNTAX_ERROR;
+    if (pos > end) return SYNTAX_ERROR;
+    buf.seek(pos);
+    if (buf[pos] != 0xFF) return SYNTAX_ERROR;
     const int marker = buf[pos + 1];
     pos += 2;
     int e = 0;
@@ -223,15 +287,16 @@ CJ_HD int cj_parse_header(const uint8_t* buf, int64_t size, CJImageHeader* h, in
         if (pos + hlen > end) return SYNTAX_ERROR;
         if (!s.nch) return SYNTAX_ERROR;
         if (hlen < 4u + 2u * s.nch) return SYNTAX_ERROR;
-        const uint8_t* p = buf + pos + 2;
-        if (*(p++) != s.nch) return UNSUPPORTED_ERROR;
-        for (int i = 0; i < s.nch; i++, p += 2) {
+        B p = buf + (pos + 2);
+        if (p[0] != s.nch) return UNSUPPORTED_ERROR;
+        p = p + 1;
+        for (int i = 0; i < s.nch; i++, p = p + 2) {
           if (p[0] != s.ids[i]) return SYNTAX_ERROR;
           if (p[1] & 0xEE) return SYNTAX_ERROR;
-          h->comp_dc[i] = (uint8_t)(p[1] >> 4);
-          h->comp_ac[i] = (uint8_t)((p[1] & 1) | 2);
-          if (!(s.huff_defined & (1 << h->comp_dc[i])) || !(s.huff_defined & (1 << h->comp_ac[i])))
-            return SYNTAX_ERROR;
+          const int dc = p[1] >> 4, ac = (p[1] & 1) | 2;
+          h->comp_dc[i] = (uint8_t)dc;
+          h->comp_ac[i] = (uint8_t)ac;
+          if (!(s.huff_defined & (1 << dc)) || !(s.huff_defined & (1 << ac))) return SYNTAX_ERROR;
         }
         if (p[0] || p[1] != 63 || p[2]) return UNSUPPORTED_ERROR;
         pos += hlen;
@@ -266,9 +331,8 @@ CJ_HD int cj_parse_header(const uint8_t* buf, int64_t size, CJImageHeader* h, in
         h->nseg_expected = s.restart ? (int)((mcus + s.restart - 1) / s.restart) : 1;
         h->total_blocks = mcus * bpm;
         // the pixel tile layout's geometry condition (cj_pix_check)
-        if (h->comp_sx[0] != h->hmax || h->comp_sy[0] != h->vmax) return UNSUPPORTED_ERROR;
-        if (h->nch == 3 && ((h->comp_sx[1] << xs) != h->hmax || (h->comp_sy[1] << ys) != h->vmax))
-          return UNSUPPORTED_ERROR;
+        if (s.sx[0] != s.sxmax || s.sy[0] != s.symax) return UNSUPPORTED_ERROR;
+        if (s.nch == 3 && ((s.sx[1] << xs) != s.sxmax || (s.sy[1] << ys) != s.symax)) return UNSUPPORTED_ERROR;
         return 0;
       }
       case 0xFE: e = pos > end ? SYNTAX_ERROR : (pos += cj_rd16(buf + pos), 0); break;

@@ -172,7 +172,7 @@ int cjBatchGetSubsequenceBitsFor(const CJBatch *b, int sampling_class);
 int cjBatchSetOutput(CJBatch *b, int format, int idct);
 /* Where a batch staged from now on has its files' marker segments parsed:
  * on the GPU (on_device != 0, the default: the files are copied to the
- * device first and one thread per file walks its segments there, the reference's
+ * device first and one warp per file walks its segments there, the reference's
  * marker loop src/format.cu:159-215 with the segment checks of
  * src/format.cu:242-442 and the scan-header check of
  * src/decodeScanGPU.cu:124-144) or on the host (on_device == 0: the marker
