@@ -27,6 +27,7 @@
 #define CJ_DEV_DC_RANGE 6        // DC predictor outside int16 (UNSUPPORTED_ERROR)
 #define CJ_DEV_EXTRA 7           // more entropy data than MCUs
 #define CJ_DEV_CAPACITY 8        // more markers / subsequences than buffers allow
+#define CJ_DEV_TIMEOUT 9         // a wait for another scan's blocks ran out (progressive.cu)
 
 // One Huffman table in canonical form.
 //   fast[w >> (16 - CJ_FAST_BITS)] = (len << 8) | symbol for codes of length

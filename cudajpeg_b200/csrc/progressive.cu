@@ -9,11 +9,12 @@
 // (interleaved or not), DC refinement (one bit per block), AC first with
 // end-of-band runs, and AC refinement with correction bits.
 //
-// Scans that touch the same coefficients run one after another, the others
-// side by side: a scan's level is one more than that of the scans before it
-// with a common component and band, and one launch runs a level, one CTA per
-// restart interval of its scans (the 10 scans of the IJG encoder's script make
-// 3 launches).
+// One CTA per restart interval of a scan.  A scan that touches coefficients of
+// scans before it follows them: all scans run in one launch, and a chunk of
+// blocks is decoded once the scans it follows have published that they are past
+// these blocks (the refinements of a component run a chunk behind one another).
+// If there are more intervals than CTAs fit on the GPU at once, a launch takes one
+// level of scans, those whose predecessors all ran in the launches before.
 #include <stdio.h>
 #include <string.h>
 
@@ -25,10 +26,16 @@
 #include "cj_internal.h"
 #include "cj_tables.h"
 
-// A scan's parameter block: the scan, its four Huffman tables.
+#define PG_DEPS 16  // scans that one scan follows (64 bands at the most; more take the launch per level)
+
+// A scan's parameter block: the scan, its four Huffman tables, the scans it
+// follows in the same launch (block by block, or after their last: whole).
 struct CJProgBlock {
   CJProgScan s;
   CJHuff huff[4];
+  int32_t ndep, dep[PG_DEPS];
+  uint32_t whole;  // bit per dependency
+  int32_t blocks;  // of the scan in all
 };
 
 // One CTA's work: a restart interval of a scan, its stuffed bytes [begin, end).
@@ -46,10 +53,12 @@ struct CJProgWork {
 // zero-history positions of every block are listed (zpos); after it, the
 // coefficients of the symbols found (evt) are read and written.  The walk itself,
 // one thread, is then two dependent shared-memory loads per refinement symbol and
-// one per symbol otherwise (about 130 and 70 cycles).
+// one per symbol otherwise.
 // Measured on a 1024x768 4:2:0 q80 file of 115 KB, 213 thousand symbols: 254 ms with
-// one thread decoding each scan from global memory, 17.4 ms in this form (10.5 of
-// them the last luma refinement's 129 thousand symbols).
+// one thread decoding each scan from global memory; in chunks, a launch per level
+// of scans 17.4 ms with a walk of 132 cycles a symbol, 13.1 ms with the present one
+// (1.5 + 3.8 + 7.6, the last luma refinement's 129 thousand symbols); in one launch
+// 8.1 ms; with a refinement's blocks staged in shared memory 7.6 ms.
 #define PG_THREADS 512
 #define PG_BITS 16384        // bit positions of a chunk
 #define PG_BLOCK_BITS 2048   // no block takes more bits than this (63 symbols of 31 bits and an EOB)
@@ -57,20 +66,23 @@ struct CJProgWork {
 #define PG_SEQ 2048          // blocks of a chunk (first scans)
 #define PG_REF_BLOCKS 256    // blocks of a chunk (AC refinement)
 #define PG_EVENTS 4096
-#define PG_ZPOS 80           // 64 positions, and the 16 a run may reach behind them
+#define PG_ZPOS 128          // 63 positions, and the 64 a symbol may step behind them
+#define PG_ZEND 252          // behind a block's last zero-history position
 #define PG_RAW 9             // stuffed bytes a thread looks at per chunk
 
 struct PGShared {
   CJHuff huff[2];                       // DC: slots 0 and 1; AC: [0]
+  alignas(16) uint32_t ahead[64];       // the refinement walk may load up to 63 entries before sym (and not use them)
   union {
     alignas(16) uint32_t sym[PG_BITS];      // AC scans
     alignas(16) uint16_t dcsym[2][PG_BITS];  // DC scans: by Huffman table
   };
-  alignas(16) uint8_t zpos[PG_REF_BLOCKS][PG_ZPOS];  // zero-history positions of each block, then 255
+  alignas(16) uint8_t zpos[PG_REF_BLOCKS][PG_ZPOS];  // 4 x the zero-history positions of each block, then PG_ZEND
   alignas(16) uint32_t words[PG_BYTES / 4 + 4];  // destuffed bytes as stored, zeros behind them
   uint16_t raw[PG_BYTES + 1];           // offset of each destuffed byte from the chunk's first stuffed byte
   uint32_t evt[PG_EVENTS];
   uint32_t ev0[PG_SEQ];
+  uint32_t coef[PG_REF_BLOCKS][33];     // the blocks before the scan (33: a thread per block, each in a bank of its own)
   uint64_t hist[PG_REF_BLOCKS];         // nonzero coefficients of the band, bit = zig-zag position - ss
   uint8_t nz[PG_REF_BLOCKS];
   uint8_t zz[64];
@@ -84,13 +96,16 @@ struct PGShared {
 };
 
 // Symbol entries.  DC (16 bits): bits 0-4 bits consumed, 5-8 magnitude size, 15
-// invalid.  AC (32 bits): byte 0 bits consumed; byte 1 run + 1; byte 2 first
-// scans: magnitude size, refinement: 1 newly nonzero, 3 and negative; byte 3
-// PG_EOB: an end-of-band run (byte 1: its number of extra bits, which count as
-// consumed), PG_BAD: invalid.  (ZRL is a run of 15 with byte 2 zero.)
+// invalid.  AC (32 bits): byte 0 four times the bits consumed (sym's bytes to the
+// next entry); byte 1 run + 1, or PG_STEP_OUT, which leaves the band, for an
+// end-of-band run (PG_EOB; bits 16-30: the further blocks it covers; its extra
+// bits count as consumed) and for an invalid code (PG_BAD); byte 2 first scans:
+// magnitude size, refinement: 1 newly nonzero, 3 and negative.  (ZRL is a run of
+// 15 with byte 2 zero.)
 #define PG_DC_BAD 0x8000u
-#define PG_EOB 0x01000000u
-#define PG_BAD 0x02000000u
+#define PG_EOB 0x80000000u
+#define PG_BAD 0x40000000u
+#define PG_STEP_OUT 64u
 __device__ __forceinline__ uint32_t pg_dc_symbol(const CJHuff& t, uint32_t win) {
   const uint32_t e = cj_huff_decode(t, win >> 16), s = e & 255;
   return !e || s > 11 ? PG_DC_BAD : ((e >> 8) + s) | (s << 5);
@@ -98,9 +113,12 @@ __device__ __forceinline__ uint32_t pg_dc_symbol(const CJHuff& t, uint32_t win) 
 __device__ __forceinline__ uint32_t pg_ac_symbol(const CJHuff& t, uint32_t win, bool refine) {
   const uint32_t e = cj_huff_decode(t, win >> 16);
   const uint32_t len = e >> 8, r = (e >> 4) & 15, s = e & 15;
-  if (!e || (refine && s > 1)) return PG_BAD;
-  if (s == 0 && r < 15) return (len + r) | (r << 8) | PG_EOB;
-  const uint32_t low = (len + s) | ((r + 1) << 8);
+  if (!e || (refine && s > 1)) return PG_BAD | (PG_STEP_OUT << 8);
+  if (s == 0 && r < 15) {
+    const uint32_t more = (1u << r) - 1u + __funnelshift_rc(win << len, 0u, 32 - r);
+    return (4 * (len + r)) | (PG_STEP_OUT << 8) | (more << 16) | PG_EOB;
+  }
+  const uint32_t low = (4 * (len + s)) | ((r + 1) << 8);
   if (!refine) return low | (s << 16);
   return low | (s ? ((win >> (31 - len)) & 1u ? 1u : 3u) << 16 : 0u);
 }
@@ -210,9 +228,24 @@ __device__ __forceinline__ void pg_walk_dc(PGShared& S, int nb, int bps) {
   S.done = b;
 }
 
-// Event: position of a symbol, its zig-zag position << 16.
+// The AC walks keep positions as byte offsets into sym (four times the bit), load
+// the next entry before they test whether the block ends, and leave the band by
+// the same test at its last coefficient, an end-of-band run and an invalid code.
+__device__ __forceinline__ uint32_t pg_lds32(uint32_t a) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ uint32_t pg_lds8(uint32_t a) {
+  uint32_t v;
+  asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(a));
+  return v;
+}
+
+// Event: offset of a symbol, its zig-zag position << 16.
 __device__ __forceinline__ void pg_walk_first(PGShared& S, int nb, int ss, int se) {
-  uint32_t pos = S.bit;
+  const uint32_t sym = (uint32_t)__cvta_generic_to_shared(S.sym);
+  uint32_t pos = 4 * S.bit, e = pg_lds32(sym + pos);
   int b = 0, eob = S.eob, ne = 0;
   for (;;) {
     if (eob) {
@@ -220,33 +253,31 @@ __device__ __forceinline__ void pg_walk_first(PGShared& S, int nb, int ss, int s
       b += skip;
       eob -= skip;
     }
-    if (b >= nb || pos >= PG_BITS - PG_BLOCK_BITS || ne >= PG_EVENTS - 64) break;
+    if (b >= nb || pos >= 4 * (PG_BITS - PG_BLOCK_BITS) || ne >= PG_EVENTS - 64) break;
     const int st = ne;
     int k = ss - 1;
-    uint32_t e;
     for (;;) {
-      e = S.sym[pos];
-      if (e & (PG_EOB | PG_BAD)) break;
       k += (int)((e >> 8) & 255);
       S.evt[ne++] = pos | ((uint32_t)k << 16);
       pos += e & 255;
-      if (k >= se) break;
-    }
-    if (e & PG_EOB) {
-      const uint32_t r = (e >> 8) & 255;
-      pos += e & 255;
-      eob = (1 << r) - 1 + (int)pg_bits(S, pos - r, r);
-    } else if (e & PG_BAD) {
-      S.err = CJ_DEV_BAD_CODE;
-    } else if (k > se) {  // a coefficient past the band, or a ZRL that ends the block
-      ne--;
-      if (e & 0xFF0000u) S.err = CJ_DEV_BAD_AC;
+      const uint32_t next = pg_lds32(sym + pos);
+      if (k >= se) {
+        if (k > se) {  // an end-of-band run, an invalid code, a coefficient past the band, a ZRL that ends the block
+          ne--;
+          if (e & PG_EOB) eob = (int)((e >> 16) & 0x7FFF);
+          else if (e & PG_BAD) S.err = CJ_DEV_BAD_CODE;
+          else if (e & 0xFF0000u) S.err = CJ_DEV_BAD_AC;
+        }
+        e = next;
+        break;
+      }
+      e = next;
     }
     S.ev0[b] = (uint32_t)st | ((uint32_t)(ne - st) << 16);
     if (S.err) break;
     b++;
   }
-  S.pos = (int)pos;
+  S.pos = (int)(pos >> 2);
   S.done = b;
   S.eob = eob;
 }
@@ -256,50 +287,54 @@ __device__ __forceinline__ void pg_walk_first(PGShared& S, int nb, int ss, int s
 // has met k - (z + r) nonzero ones, whose correction bits lie behind the
 // symbols: with q the bits of the block's symbols alone, the next symbol is at
 // q + k - (z + r).  Every block takes one correction bit per nonzero coefficient
-// in all.  Event: position of a symbol, z + r << 16 (PG_AT_EOB: an end-of-band
+// in all.  Event: offset of a symbol, z + r << 16 (PG_AT_EOB: an end-of-band
 // symbol; PG_IN_RUN: a block inside a run, position of its correction bits).
 #define PG_AT_EOB 0xFFu
 #define PG_IN_RUN 0xFEu
 __device__ __forceinline__ void pg_walk_refine(PGShared& S, int nb, int width) {
-  uint32_t pos = S.bit;
+  const uint32_t sym = (uint32_t)__cvta_generic_to_shared(S.sym), zpos = (uint32_t)__cvta_generic_to_shared(S.zpos);
+  const uint32_t last = 4 * (uint32_t)(width - 1);
+  uint32_t pos = 4 * S.bit;
   int b = 0, eob = S.eob, ne = 0;
-  while (b < nb && pos < PG_BITS - PG_BLOCK_BITS && ne < PG_EVENTS - 64) {
+  while (b < nb && pos < 4 * (PG_BITS - PG_BLOCK_BITS) && ne < PG_EVENTS - 64) {
+    const uint32_t nz4 = 4u * S.nz[b];
     S.ev0[b] = ne;
     if (eob) {
       S.evt[ne++] = pos | (PG_IN_RUN << 16);
-      pos += S.nz[b];
+      pos += nz4;
       eob--;
       b++;
       continue;
     }
-    const uint8_t* zp = S.zpos[b];
-    uint32_t q = pos, e, k;
-    int z = -1;
+    uint32_t e = pg_lds32(sym + pos), q = pos, z = zpos + b * PG_ZPOS - 1, k4, next;
+    const uint32_t z0 = z + 1;
     for (;;) {
-      e = S.sym[pos];
-      if (e & (PG_EOB | PG_BAD)) break;
-      z += (int)((e >> 8) & 255);
-      k = zp[z];
+      z += (e >> 8) & 255;
+      k4 = pg_lds8(z);
       q += e & 255;
-      S.evt[ne++] = pos | ((uint32_t)z << 16);
-      pos = q + k - (uint32_t)z;
-      if ((int)k >= width - 1) break;
+      S.evt[ne++] = pos | ((z - z0) << 16);
+      const uint32_t at = q - 4 * (z - z0) + k4;
+      next = pg_lds32(sym + at);
+      if (k4 >= last) {
+        if (k4 < PG_ZEND) pos = at;
+        break;
+      }
+      pos = at;
+      e = next;
     }
-    if (e & PG_EOB) {
-      const uint32_t r = (e >> 8) & 255;
-      S.evt[ne++] = pos | (PG_AT_EOB << 16);
-      eob = (1 << r) - 1 + (int)pg_bits(S, pos + (e & 255) - r, r);
-      pos = q + (e & 255) + S.nz[b];
-    } else if (e & PG_BAD) {
-      S.err = CJ_DEV_BAD_AC;
-    } else if (k == 255) {  // past the band: an error, or a ZRL that ends the block
-      pos = q + S.nz[b];
-      if (e & 0xFF0000u) S.err = CJ_DEV_BAD_AC;
+    if (k4 >= PG_ZEND) {  // past the band: an end-of-band run, an error, or a ZRL that ends the block
+      if (e & PG_EOB) {
+        S.evt[ne - 1] = pos | (PG_AT_EOB << 16);
+        eob = (int)((e >> 16) & 0x7FFF);
+      } else if (e & (PG_BAD | 0xFF0000u)) {
+        S.err = CJ_DEV_BAD_AC;
+        break;
+      }
+      pos = q + nz4;
     }
-    if (S.err) break;
     b++;
   }
-  S.pos = (int)pos;
+  S.pos = (int)(pos >> 2);
   S.done = b;
   S.eob = eob;
   if (!S.err) S.ev0[b] = ne;  // the end of the last block's events (an error's block is left out)
@@ -307,10 +342,47 @@ __device__ __forceinline__ void pg_walk_refine(PGShared& S, int nb, int width) {
 
 __constant__ uint8_t c_prog_zz[64] = CJ_ZIGZAG_INIT;
 
+// Waits (one thread) until the scans that `b` follows are past `need` blocks of
+// theirs, which of a dependency marked whole are all.  progress[i]: blocks of scan i
+// done and written, progress[nscans]: chunks done by any CTA.  The wait is given up
+// when no CTA of the launch finished a chunk for PG_WAIT_POLLS polls (seconds; a
+// chunk takes a fraction of a millisecond, and the CTAs are all resident).
+// Polls are relaxed loads, which leave the SM's L1 alone; the fence behind them
+// orders the reads of the coefficients.
+#define PG_WAIT_POLLS (1u << 23)
+__device__ __forceinline__ int pg_load_relaxed(const int* p) {
+  int v;
+  asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __noinline__ bool pg_await(const CJProgBlock* __restrict__ scans, const CJProgBlock& b, const int* progress,
+                                      int nscans, int need) {
+  for (int j = 0; j < b.ndep; j++) {
+    const int want = (b.whole >> j) & 1 ? scans[b.dep[j]].blocks : need;
+    int seen = -1;
+    unsigned polls = 0;
+    while (pg_load_relaxed(&progress[b.dep[j]]) < want) {
+      const int any = pg_load_relaxed(&progress[nscans]);
+      if (any != seen) polls = 0;
+      seen = any;
+      if (++polls > PG_WAIT_POLLS) return false;
+      __nanosleep(256);
+    }
+  }
+  __threadfence();
+  return true;
+}
+// A CTA's chunk is written (its threads are past a barrier): blocks more of `scan` done.
+__device__ __forceinline__ void pg_publish(int* progress, int nscans, int scan, int blocks) {
+  __threadfence();
+  atomicAdd(&progress[scan], blocks);
+  atomicAdd(&progress[nscans], 1);
+}
+
 __global__ void __launch_bounds__(PG_THREADS) k_prog_scans(const CJProgBlock* __restrict__ scans,
                                                            const CJProgWork* __restrict__ work,
                                                            const uint8_t* __restrict__ file, int16_t* coef,
-                                                           CJStatus* st) {
+                                                           CJStatus* st, int* progress, int nscans) {
   extern __shared__ __align__(16) uint8_t pg_smem[];
   PGShared& S = *reinterpret_cast<PGShared*>(pg_smem);
   const CJProgWork wk = work[blockIdx.x];
@@ -346,6 +418,15 @@ __global__ void __launch_bounds__(PG_THREADS) k_prog_scans(const CJProgBlock* __
   while (S.blk < nseq && !S.err) {  // CTA-uniform: written only between barriers below
     const int blk0 = S.blk;
     const int64_t raw0 = S.rawpos;
+    if (progress && scans[wk.scan].ndep) {
+      if (tid == 0 && !pg_await(scans, scans[wk.scan], progress, nscans, min(nseq, blk0 + PG_REF_BLOCKS)))
+        S.err = CJ_DEV_TIMEOUT;
+      __syncthreads();
+      if (S.err) {
+        if (tid == 0) cj_raise(st, 0, S.err);
+        break;
+      }
+    }
     pg_stage_bytes(S, file, raw0, wk.end);
     const int nbits = S.done;
     int nb = nseq - blk0;
@@ -371,19 +452,28 @@ __global__ void __launch_bounds__(PG_THREADS) k_prog_scans(const CJProgBlock* __
         pg_stage_symbols<false>(S, 0, S.huff[0], refine, nbits);
       }
       if (dc) {
-      } else if (refine) {  // history: a warp per block, two zig-zag positions per lane
+      } else if (refine) {  // the blocks, then their history: a warp per block, two zig-zag positions per lane
         const int lane = tid & 31;
+        for (int i = tid; i < nb * 8; i += PG_THREADS) {
+          const uint4 v = reinterpret_cast<const uint4*>(coef + pg_block(s, S, u0, bps, blk0 + (i >> 3)) * 64)[i & 7];
+          uint32_t* to = &S.coef[i >> 3][4 * (i & 7)];
+          to[0] = v.x;
+          to[1] = v.y;
+          to[2] = v.z;
+          to[3] = v.w;
+        }
+        __syncthreads();
         const uint32_t lt = (1u << lane) - 1u;
         for (int b = tid >> 5; b < nb; b += PG_THREADS / 32) {
-          const int16_t* blk = coef + pg_block(s, S, u0, bps, blk0 + b) * 64;
+          const int16_t* blk = reinterpret_cast<const int16_t*>(S.coef[b]);
           const bool in0 = lane < width, in1 = lane + 32 < width;
           const bool n0 = in0 && blk[S.zz[s.ss + lane]] != 0, n1 = in1 && blk[S.zz[min(63, s.ss + lane + 32)]] != 0;
           const uint32_t h0 = __ballot_sync(CJ_FULL, n0), h1 = __ballot_sync(CJ_FULL, n1);
           const uint32_t z0 = __ballot_sync(CJ_FULL, in0 && !n0), z1 = __ballot_sync(CJ_FULL, in1 && !n1);
-          if (lane < PG_ZPOS / 4) reinterpret_cast<uint32_t*>(S.zpos[b])[lane] = 0xFFFFFFFFu;
+          if (lane < PG_ZPOS / 4) reinterpret_cast<uint32_t*>(S.zpos[b])[lane] = PG_ZEND * 0x01010101u;
           __syncwarp();
-          if (in0 && !n0) S.zpos[b][__popc(z0 & lt)] = (uint8_t)lane;
-          if (in1 && !n1) S.zpos[b][__popc(z0) + __popc(z1 & lt)] = (uint8_t)(lane + 32);
+          if (in0 && !n0) S.zpos[b][__popc(z0 & lt)] = (uint8_t)(4 * lane);
+          if (in1 && !n1) S.zpos[b][__popc(z0) + __popc(z1 & lt)] = (uint8_t)(4 * (lane + 32));
           if (lane == 0) {
             S.nz[b] = (uint8_t)(__popc(h0) + __popc(h1));
             S.hist[b] = (uint64_t)h0 | ((uint64_t)h1 << 32);
@@ -439,9 +529,9 @@ __global__ void __launch_bounds__(PG_THREADS) k_prog_scans(const CJProgBlock* __
           const int64_t at = pg_block(s, S, u0, bps, blk0 + b);
           int16_t* blk = coef + at * 64;
           for (uint32_t i = 0; i < (v0 >> 16); i++) {
-            const uint32_t ev = S.evt[(v0 & 0xFFFFu) + i], e = S.sym[ev & 0xFFFFu], size = (e >> 16) & 255;
+            const uint32_t ev = S.evt[(v0 & 0xFFFFu) + i], e = S.sym[(ev & 0xFFFFu) >> 2], size = (e >> 16) & 255;
             if (!size) continue;  // ZRL
-            const int v = cj_extend(pg_bits(S, (ev & 0xFFFFu) + (e & 255) - size, size), size) * (1 << al);
+            const int v = cj_extend(pg_bits(S, (((ev & 0xFFFFu) + (e & 255)) >> 2) - size, size), size) * (1 << al);
             if (v < -32768 || v > 32767) {
               cj_raise(st, at, CJ_DEV_DC_RANGE);
               break;
@@ -458,16 +548,17 @@ __global__ void __launch_bounds__(PG_THREADS) k_prog_scans(const CJProgBlock* __
           const int e1 = (int)S.ev0[b + 1];
           int c = 0;  // corrections made
           for (int i = (int)S.ev0[b]; i < e1; i++) {
-            const uint32_t ev = S.evt[i], z = ev >> 16, e = S.sym[ev & 0xFFFFu];
-            const uint32_t k = z < PG_IN_RUN ? S.zpos[b][z] : 255;
-            const int c1 = k < 255 ? (int)(k - z) : nz;
-            uint32_t at = (ev & 0xFFFFu) + (z == PG_IN_RUN ? 0u : e & 255);
+            const uint32_t ev = S.evt[i], z = ev >> 16, e = S.sym[(ev & 0xFFFFu) >> 2];
+            const uint32_t k4 = z < PG_IN_RUN ? S.zpos[b][z] : PG_ZEND, k = k4 >> 2;
+            const int c1 = k4 < PG_ZEND ? (int)(k - z) : nz;
+            uint32_t at = ((ev & 0xFFFFu) + (z == PG_IN_RUN ? 0u : e & 255)) >> 2;
             for (; c < c1; c++, at++) {
-              int16_t* q = &blk[S.zz[s.ss + __ffsll((long long)h) - 1]];
+              const int zz = S.zz[s.ss + __ffsll((long long)h) - 1];
+              const int v = reinterpret_cast<const int16_t*>(S.coef[b])[zz];
               h &= h - 1;
-              if (pg_bits(S, at, 1) && !(*q & p1)) *q = (int16_t)(*q + (*q >= 0 ? p1 : m1));
+              if (pg_bits(S, at, 1) && !(v & p1)) blk[zz] = (int16_t)(v + (v >= 0 ? p1 : m1));
             }
-            if (k < 255 && (e & 0x10000u)) blk[S.zz[s.ss + k]] = (int16_t)(e & 0x20000u ? m1 : p1);
+            if (k4 < PG_ZEND && (e & 0x10000u)) blk[S.zz[s.ss + k]] = (int16_t)(e & 0x20000u ? m1 : p1);
           }
         }
       }
@@ -476,11 +567,13 @@ __global__ void __launch_bounds__(PG_THREADS) k_prog_scans(const CJProgBlock* __
     if (tid == 0) {
       if (S.err) cj_raise(st, pg_block(s, S, u0, bps, blk0 + S.done), S.err);
       S.blk = blk0 + S.done;
+      if (progress) pg_publish(progress, nscans, wk.scan, S.done);
       S.rawpos = raw0 + min((int)S.raw[min(S.pos >> 3, PG_BYTES)], (int)min((int64_t)65535, wk.end - raw0));
       S.bit = S.pos & 7;
     }
     __syncthreads();
   }
+  if (progress && tid == 0) pg_publish(progress, nscans, wk.scan, nseq - S.blk);  // an error's blocks: none waits for them
 }
 
 // ---------------------------------------------------------------- host side
@@ -624,26 +717,48 @@ int cj_prog_scan(JPGReader* jpg) {
   return 0;
 }
 
-// Decode the noted scans, a level per launch, and queue the pixel stage's
-// parameters (geometry and the quantisation tables; the Huffman tables are not
-// needed after the scans).
+// Decode the noted scans and queue the pixel stage's parameters (geometry and the
+// quantisation tables; the Huffman tables are not needed after the scans).
 int cj_prog_finish(JPGReader* jpg) {
   CJReaderDevice* d = jpg->dev;
   const int n = d->prog_scans;
-  const CJProgBlock* blocks = reinterpret_cast<const CJProgBlock*>(d->prog_blocks.data());
-  // levels: a scan waits for those before it that touch a common coefficient
+  CJProgBlock* blocks = reinterpret_cast<CJProgBlock*>(d->prog_blocks.data());
+  // a scan follows the last ones before it that touch a coefficient of its; its level
+  // is one more than theirs
   std::vector<int> level(n);
-  int levels = 0, last[CJ_MAX_BPM][64];  // by the component's first block in an MCU
+  int levels = 0, last[CJ_MAX_BPM][64];  // scan + 1, by the component's first block in an MCU
+  bool one_launch = true;
   memset(last, 0, sizeof(last));
   for (int i = 0; i < n; i++) {
-    const CJProgScan& s = blocks[i].s;
+    CJProgBlock& b = blocks[i];
+    const CJProgScan& s = b.s;
+    b.blocks = s.nunits;
+    if (s.ns > 1) {
+      int bps = 0;
+      for (int j = 0; j < s.ns; j++) bps += s.sx[j] * s.sy[j];
+      b.blocks *= bps;
+    }
+    b.ndep = 0;
+    b.whole = 0;
     int l = 0;
     for (int j = 0; j < s.ns; j++)
-      for (int k = s.ss; k <= s.se; k++) l = std::max(l, last[s.first[j]][k]);
-    level[i] = l++;
-    for (int j = 0; j < s.ns; j++)
-      for (int k = s.ss; k <= s.se; k++) last[s.first[j]][k] = l;
-    levels = std::max(levels, l);
+      for (int k = s.ss; k <= s.se; k++) {
+        const int p = last[s.first[j]][k] - 1;
+        last[s.first[j]][k] = i + 1;
+        if (p < 0 || std::find(b.dep, b.dep + b.ndep, p) != b.dep + b.ndep) continue;
+        if (p == i) continue;
+        l = std::max(l, level[p] + 1);
+        if (b.ndep == PG_DEPS) {
+          one_launch = false;
+          continue;
+        }
+        // block by block: refinements of one component's AC band, whose chunks are of PG_REF_BLOCKS
+        const CJProgScan& q = blocks[p].s;
+        if (!(s.ss > 0 && s.ah && q.ss > 0 && q.nint == 1 && s.nint == 1)) b.whole |= 1u << b.ndep;
+        b.dep[b.ndep++] = p;
+      }
+    level[i] = l;
+    levels = std::max(levels, l + 1);
   }
   std::vector<CJProgWork> work;
   std::vector<size_t> from(levels + 1, 0);
@@ -657,23 +772,42 @@ int cj_prog_finish(JPGReader* jpg) {
     }
     from[l + 1] = work.size();
   }
+  CJ_CUDA_TRY(cudaFuncSetAttribute(k_prog_scans, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PGShared)),
+              CUDA_KERNEL_LAUNCH_ERROR);
+  int sms = 0, per = 0;
+  CJ_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d->device), CUDA_MEM_ERROR);
+  CJ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_prog_scans, PG_THREADS, sizeof(PGShared)),
+              CUDA_KERNEL_LAUNCH_ERROR);
+  one_launch = one_launch && levels > 1 && work.size() <= (size_t)sms * per;
+  // copied together: the scans' blocks, the work items, the progress counters' zeros
   const size_t pbytes = ((size_t)n * sizeof(CJProgBlock) + 15) & ~(size_t)15;
-  const size_t bytes = pbytes + work.size() * sizeof(CJProgWork);
-  d->prog_blocks.resize(bytes);  // the copy's source: blocks, then work items
-  memcpy(d->prog_blocks.data() + pbytes, work.data(), work.size() * sizeof(CJProgWork));
+  const size_t wbytes = work.size() * sizeof(CJProgWork), bytes = pbytes + wbytes + (n + 1) * sizeof(int);
+  d->prog_blocks.resize(bytes);
+  memcpy(d->prog_blocks.data() + pbytes, work.data(), wbytes);
+  memset(d->prog_blocks.data() + pbytes + wbytes, 0, (n + 1) * sizeof(int));
   if (cj_dev_ensure(d->pscan, bytes)) return CUDA_MEM_ERROR;
   CJ_CUDA_TRY(cudaMemcpyAsync(d->pscan.p, d->prog_blocks.data(), bytes, cudaMemcpyHostToDevice, d->stream),
               CUDA_MEM_ERROR);
   d->param_bytes += bytes;
-  CJ_CUDA_TRY(cudaFuncSetAttribute(k_prog_scans, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PGShared)),
-              CUDA_KERNEL_LAUNCH_ERROR);
   cj_profile_begin(d);
-  for (int l = 0; l < levels; l++) {
-    k_prog_scans<<<(unsigned)(from[l + 1] - from[l]), PG_THREADS, sizeof(PGShared), d->stream>>>(
-        (const CJProgBlock*)d->pscan.p, (const CJProgWork*)((const uint8_t*)d->pscan.p + pbytes) + from[l],
-        (const uint8_t*)d->raw.p, (int16_t*)d->coef.p, (CJStatus*)d->status.p);
+  uint8_t* dev = (uint8_t*)d->pscan.p;
+  for (int l = 0; l < (one_launch ? 1 : levels); l++) {
+    const CJProgBlock* a_scans = (const CJProgBlock*)dev;
+    const CJProgWork* a_work = (const CJProgWork*)(dev + pbytes) + from[l];
+    const uint8_t* a_file = (const uint8_t*)d->raw.p;
+    int16_t* a_coef = (int16_t*)d->coef.p;
+    CJStatus* a_st = (CJStatus*)d->status.p;
+    int* a_progress = one_launch ? (int*)(dev + pbytes + wbytes) : nullptr;
+    int a_n = n;
+    void* args[] = {&a_scans, &a_work, &a_file, &a_coef, &a_st, &a_progress, &a_n};
+    const unsigned grid = (unsigned)((one_launch ? work.size() : from[l + 1]) - from[l]);
+    // CTAs that wait for one another are all resident (cooperative); levels need not be
+    CJ_CUDA_TRY(one_launch ? cudaLaunchCooperativeKernel((const void*)k_prog_scans, dim3(grid), dim3(PG_THREADS), args,
+                                                         sizeof(PGShared), d->stream)
+                           : cudaLaunchKernel((const void*)k_prog_scans, dim3(grid), dim3(PG_THREADS), args,
+                                              sizeof(PGShared), d->stream),
+                CUDA_KERNEL_LAUNCH_ERROR);
     cj_after_launch(d, CJ_K_PROG_SCAN);
-    CJ_CUDA_TRY(cudaGetLastError(), CUDA_KERNEL_LAUNCH_ERROR);
   }
   CJScanParams* hp = (CJScanParams*)d->h_params.p;
   cj_fill_params(jpg, hp);

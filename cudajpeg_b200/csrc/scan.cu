@@ -123,6 +123,7 @@ int cj_status_error(const CJStatus* st) {
   int code = (int)(key & 0xFF);
   if (code == CJ_DEV_DC_RANGE) return UNSUPPORTED_ERROR;
   if (code == CJ_DEV_CAPACITY) return PROGRAMMER_ERROR;
+  if (code == CJ_DEV_TIMEOUT) return CUDA_KERNEL_LAUNCH_ERROR;
   return SYNTAX_ERROR;
 }
 
