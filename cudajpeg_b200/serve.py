@@ -92,7 +92,7 @@ class Server:
         p = self.lib.cjServerDLPack(self.ptr, ticket)
         if not p:
             raise DecodeError(PROGRAMMER_ERROR, f"request {ticket} has no device pixels")
-        return torch.from_dlpack(DLPackView(p, self.lib))
+        return torch.from_dlpack(DLPackView(p, self.lib).__dlpack__())
 
     def set_tuning(self, sub_bits: int = 0, decode_ctas_per_sm: int = 0, pixel_tile_cap: int = 0):
         err = self.lib.cjServerSetTuning(self.ptr, sub_bits, decode_ctas_per_sm, pixel_tile_cap)
