@@ -363,18 +363,17 @@ __device__ __forceinline__ void cj_tc_build_a(int nblk, const int16_t* sc, uint8
     const uint4 raw = *reinterpret_cast<const uint4*>(sc + kb * 64 + v * 8);
     const uint4 qv = *reinterpret_cast<const uint4*>(&P.qh[P.bq[kb]][v * 8]);
     const uint32_t rw[4] = {raw.x, raw.y, raw.z, raw.w}, qw[4] = {qv.x, qv.y, qv.z, qv.w};
-    uint32_t p[4], acc = 0;
+    uint32_t p[4];
+    __half2 top = __float2half2_rn(0.f);
 #pragma unroll
     for (int j = 0; j < 4; j++) {
       const __half2 c2 = __halves2half2(__short2half_rn((short)(rw[j] & 0xFFFFu)), __short2half_rn((short)(rw[j] >> 16)));
       __half2 pr = __hmul2(c2, *reinterpret_cast<const __half2*>(&qw[j]));
       if (j == 0) pr = __hadd2(pr, bias);
       p[j] = *reinterpret_cast<const uint32_t*>(&pr);
-      // per half: |x| >= 2048 (0x6800, NaN and Inf above) sets bit 15 of
-      // (bits & 0x7FFF) + 0x1800; no carry crosses into the upper half
-      acc |= (p[j] & 0x7FFF7FFFu) + 0x18001800u;
+      top = __hmax2_nan(top, __habs2(pr));
     }
-    big[t] = (acc & 0x80008000u) != 0;
+    big[t] = tc_beyond(top);
     *reinterpret_cast<uint4*>(sA + tc_sw128_off(kb, v)) = make_uint4(p[0], p[1], p[2], p[3]);
   }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");

@@ -172,18 +172,15 @@ int cj_upload_basis() {
 #define TC_ROWS (8 / TC_GROUPS)
 static_assert(TC_THREADS == 256 || TC_THREADS == 512, "two or four threads per block in the epilogue");
 #ifndef TC_STAGES
-#define TC_STAGES 2                 // coefficient tiles in flight per CTA (TMA ring)
-#endif
-#ifndef TC_ABUF
-#define TC_ABUF 1                   // A tiles (with one, a tile's A build waits for the previous MMAs)
+#define TC_STAGES 2                 // tiles per CTA, each first the coefficients, then in place the A tile
 #endif
 #ifndef TC_MINB
-#define TC_MINB 3                   // CTAs per SM the kernel is compiled for
+#define TC_MINB 4                   // CTAs per SM the kernel is compiled for
 #endif
 #define TC_TILE_BYTES 16384         // 128 blocks x 64 int16
-// dynamic shared memory: 1 KiB of alignment slack, the TMA ring, the
-// swizzled A tile(s), the hi/lo basis, three slots of per-row range flags
-#define TC_SMEM (1024 + TC_STAGES * TC_TILE_BYTES + TC_ABUF * 16384 + 16384 + 3 * 1024)
+// dynamic shared memory: 1 KiB of alignment slack, the tiles, the hi/lo basis,
+// three slots of per-row range flags
+#define TC_SMEM (1024 + TC_STAGES * TC_TILE_BYTES + 16384 + 3 * 1024)
 
 // per device: Khi then Klo, core-matrix layout
 #define CJ_MAX_DEVICES 64
@@ -211,18 +208,25 @@ __device__ __forceinline__ void tc_tile_load(void* dst, const CUtensorMap* map, 
 //
 // A persistent CTA runs its tiles k = 0, 1, ... (tile blockIdx.x + k *
 // gridDim.x) through a software pipeline with one barrier per tile:
-//   - TC_STAGES - 1 tiles ahead, thread 0 has TMA copies in flight into a
-//     ring of shared-memory stages (mbarrier per stage);
+//   - thread 0 has TMA copies in flight into the tiles that no MMA reads any
+//     more (mbarrier per tile);
 //   - iteration k: every thread dequantises 4 coefficient rows of tile k
-//     into the FP16 A tile (TC_ABUF of them, 128-byte swizzled; with one,
-//     after tile k-1's MMAs have read it; for pixels the DC is biased by
-//     TC_DC_BIAS; a row FP16 cannot hold exactly sets its range flag)
+//     into FP16 in place (a block's 8 rows are one warp's; 128-byte swizzled;
+//     for pixels the DC is biased by TC_DC_BIAS; a row FP16 cannot hold exactly
+//     sets its range flag)
 //     -- barrier -- thread 0 issues tile k's 8 MMAs into one of two
-//     64-column accumulators and the next copy, while every thread runs tile
-//     k-1's epilogue: wait for its MMAs, read its block's half row of D (32
+//     64-column accumulators, while every thread runs tile k-1's epilogue: wait
+//     for its MMAs (after which thread 0 starts the copy that takes the tile's
+//     place), read its block's half row of D (32
 //     values) with tcgen05.ld, floor (the bias did the rounding), level-
 //     shift and clip, store.  A thread whose block has a range flag computes
 //     its 32 outputs in FP32 from the coefficients in global memory instead.
+// Bound by instruction issue and the chain copy - convert - MMA - read of each
+// CTA, not by memory: 8192 x 8192 samples (201 MB, 31 us at the measured copy
+// rate) took 63 us with a copy ring beside the A tile (three CTAs per SM), the
+// float -> int32 conversions of the epilogue in the quarter-rate unit that also
+// converts int16 -> half (59% busy), and an index division per block and tile;
+// 56 us with four CTAs, floor by addition (tc_level4) and no division.
 // Range flags keep three slots, so a thread still in tile k-1's epilogue
 // never sees tile k+1's flags.  A wait that runs out marks `status` and the
 // tile's output is not written; the pipeline keeps its barriers.
@@ -237,8 +241,7 @@ __global__ void __launch_bounds__(TC_THREADS, TC_MINB) k_idct_tc(const __grid_co
   __shared__ float sbasis[64];
   uint8_t* smem = smem_raw + ((1024u - (cj_smem_addr(smem_raw) & 1023u)) & 1023u);
   uint8_t* stages = smem;
-  uint8_t* sA = smem + TC_STAGES * TC_TILE_BYTES;  // A tile(s), 1024-byte aligned
-  uint8_t* sB = sA + TC_ABUF * 16384;
+  uint8_t* sB = stages + TC_STAGES * TC_TILE_BYTES;
   uint8_t* flags = sB + 16384;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   for (int k = tid; k < 16384 / 16; k += TC_THREADS)
@@ -259,16 +262,16 @@ __global__ void __launch_bounds__(TC_THREADS, TC_MINB) k_idct_tc(const __grid_co
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_base;
   const int64_t ntiles = (a.nblocks + TC_M - 1) / TC_M;
-  const int64_t K = (int64_t)blockIdx.x < ntiles ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
+  const int K = (int64_t)blockIdx.x < ntiles ? (int)((ntiles - 1 - blockIdx.x) / gridDim.x) + 1 : 0;
   const int per = a.sx * a.sy, per_shift = __ffs(per) - 1;  // a power of two
   const int mcus_per_tile = TC_M / per;
-  auto issue = [&](int64_t k) {
-    const int64_t tile = blockIdx.x + k * gridDim.x;
-    const int s = (int)(k % TC_STAGES);
+  auto issue = [&](int k) {
+    const int64_t tile = blockIdx.x + (int64_t)k * gridDim.x;
+    const int s = k % TC_STAGES;
     tc_tile_load(stages + s * TC_TILE_BYTES, &tmap, (int)(tile * mcus_per_tile), &full[s]);
   };
   if (tid == 0)
-    for (int64_t k = 0; k < K && k < TC_STAGES - 1; k++) issue(k);
+    for (int k = 0; k < K && k < TC_STAGES; k++) issue(k);
   // this thread always converts coefficient row v = tid & 7 of its blocks:
   // the row's 8 quantisation steps as FP16 pairs, once
   const int v = tid & 7;
@@ -282,67 +285,60 @@ __global__ void __launch_bounds__(TC_THREADS, TC_MINB) k_idct_tc(const __grid_co
   // are left unbiased
   const __half2 bias = __floats2half2_rn(!RAW && v == 0 ? TC_DC_BIAS : 0.f, 0.f);
   bool bad = false;
-  for (int64_t k = 0; k <= K; k++) {
+  // the block whose outputs this thread has: block m of each tile, followed from
+  // tile to tile by its MCU's row and column (no division per tile; the launcher
+  // bounds the MCU count below 2^31)
+  const int quad = warp & 3, h = warp >> 2, m = 32 * quad + lane;
+  const uint32_t loc = (uint32_t)m & (uint32_t)(per - 1), lx = loc % (uint32_t)a.sx, ly = loc / (uint32_t)a.sx;
+  const uint32_t mcux = (uint32_t)a.mcux, mcu0 = (uint32_t)(((int64_t)blockIdx.x * TC_M + m) >> per_shift);
+  const uint32_t step_row = (gridDim.x * mcus_per_tile) / mcux, step_col = gridDim.x * mcus_per_tile - step_row * mcux;
+  uint32_t mrow = mcu0 / mcux, mcol = mcu0 - mrow * mcux;
+  int64_t kb = (int64_t)blockIdx.x * TC_M + m;
+  uint8_t* fl = flags;  // of tile k, and of tile k - 1
+  uint8_t* fl_prev = flags;
+  for (int k = 0; k <= K; k++) {
     if (k < K) {  // ---- A tile of local tile k
-      const int s = (int)(k % TC_STAGES);
-      if (!cj_mbar_wait(&full[s], (uint32_t)((k / TC_STAGES) & 1))) bad = true;
-      const uint8_t* st = stages + s * TC_TILE_BYTES;
-      uint8_t* a_k = sA + (k % TC_ABUF) * 16384;
-      // with one A tile, tile k - 1's MMAs must have read it (bounded wait;
-      // the epilogue below waits for the same phase)
-      if (TC_ABUF == 1 && k >= 1 && !cj_mbar_wait(&mma_done[(k - 1) & 1], (uint32_t)(((k - 1) >> 1) & 1)))
-        bad = true;
-      uint8_t* fl = flags + (k % 3) * 1024;
+      const int s = k % TC_STAGES;
+      if (!cj_mbar_wait(&full[s], (uint32_t)(k / TC_STAGES) & 1u)) bad = true;
+      uint8_t* st = stages + s * TC_TILE_BYTES;
 #pragma unroll
       for (int j = 0; j < 1024 / TC_THREADS; j++) {
         const int t = tid + TC_THREADS * j, kb = t >> 3;  // row (kb, v) sits at t * 16
         const uint4 raw = *reinterpret_cast<const uint4*>(st + t * 16);
+        __syncwarp();  // block kb's 8 rows are this warp's: read before they are overwritten
         const uint32_t rw[4] = {raw.x, raw.y, raw.z, raw.w};
-        uint32_t p[4], acc = 0;
+        uint32_t p[4];
+        __half2 top = __float2half2_rn(0.f);
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-          const __half2 c2 = __halves2half2(__short2half_rn((short)(rw[i] & 0xFFFFu)),
-                                            __short2half_rn((short)(rw[i] >> 16)));
+          const __half2 c2 = __halves2half2(__short2half_rn((short)(rw[i] & 0xFFFFu)), __short2half_rn((short)(rw[i] >> 16)));
           __half2 pr = __hmul2(c2, *reinterpret_cast<const __half2*>(&qh[i]));
           if (i == 0) pr = __hadd2(pr, bias);
           p[i] = *reinterpret_cast<const uint32_t*>(&pr);
-          // per half: |x| >= 2048 (0x6800, NaN and Inf above) sets bit 15 of
-          // (bits & 0x7FFF) + 0x1800; no carry crosses into the upper half
-          acc |= (p[i] & 0x7FFF7FFFu) + 0x18001800u;
+          top = __hmax2_nan(top, __habs2(pr));
         }
-        fl[t] = (acc & 0x80008000u) != 0;
-        *reinterpret_cast<uint4*>(a_k + tc_sw128_off(kb, v)) = make_uint4(p[0], p[1], p[2], p[3]);
+        fl[t] = tc_beyond(top);
+        *reinterpret_cast<uint4*>(st + tc_sw128_off(kb, v)) = make_uint4(p[0], p[1], p[2], p[3]);
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (k < K && tid == 0) {  // ---- tile k's MMAs, then the copy TC_STAGES - 1 tiles ahead
-      tc_idct_mmas_asw(tmem + (uint32_t)(k & 1) * 64u, cj_smem_addr(sA + (k % TC_ABUF) * 16384), cj_smem_addr(sB),
-                       cj_smem_addr(&mma_done[k & 1]));
-      if (k + TC_STAGES - 1 < K) issue(k + TC_STAGES - 1);
-    }
+    if (k < K && tid == 0)  // ---- tile k's MMAs
+      tc_idct_mmas_asw(tmem + (uint32_t)(k & 1) * 64u, cj_smem_addr(stages + (k % TC_STAGES) * TC_TILE_BYTES),
+                       cj_smem_addr(sB), cj_smem_addr(&mma_done[k & 1]));
     if (k >= 1) {  // ---- epilogue of local tile k - 1
-      const int64_t kk = k - 1;
+      const int kk = k - 1;
       const bool ok = cj_mbar_wait(&mma_done[kk & 1], (uint32_t)((kk >> 1) & 1));
       if (!ok) bad = true;
+      // tile k - 1's MMAs have read it: the next copy into its place
+      if (tid == 0 && ok && kk + TC_STAGES < K) issue(kk + TC_STAGES);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const int quad = warp & 3, h = warp >> 2, m = 32 * quad + lane;
-      const int64_t kb = (blockIdx.x + kk * gridDim.x) * TC_M + m;
       const bool live = ok && kb < a.nblocks;
-      const bool flagged = live && *reinterpret_cast<const uint64_t*>(flags + (kk % 3) * 1024 + m * 8) != 0;
-      int bx = 0, by = 0;
-      int64_t gb = 0;
-      if (live && RAW) {
-        gb = kb;
-      } else if (live) {  // cj_plane_src in 32-bit arithmetic (the launcher bounds the MCU count below 2^31)
-        const uint32_t mcu = (uint32_t)kb >> per_shift, loc = (uint32_t)kb & (uint32_t)(per - 1);
-        const uint32_t mrow = mcu / (uint32_t)a.mcux, mcol = mcu - mrow * (uint32_t)a.mcux;
-        bx = (int)(mcol * a.sx + loc % (uint32_t)a.sx);
-        by = (int)(mrow * a.sy + loc / (uint32_t)a.sx);
-        gb = (int64_t)mcu * a.bpm + a.first + loc;
-      }
+      const bool flagged = live && *reinterpret_cast<const uint64_t*>(fl_prev + m * 8) != 0;
+      const uint32_t bx = mcol * (uint32_t)a.sx + lx, by = mrow * (uint32_t)a.sy + ly;
+      uint8_t* px = a.plane + ((int64_t)(by * 8u) + TC_ROWS * h) * a.stride + (int64_t)bx * 8;
       const uint32_t ta = tmem + (uint32_t)(kk & 1) * 64u + ((uint32_t)(32 * quad) << 16) + (uint32_t)(TC_COLS * h);
 #pragma unroll
       for (int j = 0; j < TC_COLS / 16; j++) {
@@ -350,18 +346,19 @@ __global__ void __launch_bounds__(TC_THREADS, TC_MINB) k_idct_tc(const __grid_co
         tc_ld16(ta + 16u * j, d);
         if (!live || flagged) continue;
         if (RAW) {
-          float4* o = reinterpret_cast<float4*>(raw_out + (gb * 64 + TC_COLS * h + 16 * j));
+          float4* o = reinterpret_cast<float4*>(raw_out + (kb * 64 + TC_COLS * h + 16 * j));
 #pragma unroll
           for (int i = 0; i < 4; i++) o[i] = make_float4(d[4 * i], d[4 * i + 1], d[4 * i + 2], d[4 * i + 3]);
         } else {
 #pragma unroll
           for (int y = 0; y < 2; y++)
-            *reinterpret_cast<uint2*>(a.plane + (int64_t)(by * 8 + TC_ROWS * h + 2 * j + y) * a.stride + bx * 8) =
+            *reinterpret_cast<uint2*>(px + (2 * j + y) * (int64_t)a.stride) =
                 make_uint2(tc_level4(d[8 * y], d[8 * y + 1], d[8 * y + 2], d[8 * y + 3]),
                            tc_level4(d[8 * y + 4], d[8 * y + 5], d[8 * y + 6], d[8 * y + 7]));
         }
       }
       if (flagged) {  // rare: this thread's TC_COLS outputs (its TC_ROWS pixel rows) in FP32
+        const int64_t gb = RAW ? kb : ((int64_t)mrow * mcux + mcol) * a.bpm + a.first + loc;
         const int16_t* blk = a.coef + gb * 64;
 #pragma unroll 1
         for (int x = 0; x < 8; x++) {
@@ -377,11 +374,17 @@ __global__ void __launch_bounds__(TC_THREADS, TC_MINB) k_idct_tc(const __grid_co
             float s = 0.f;
             for (int vv = 0; vv < 8; vv++) s = fmaf(col[vv], sbasis[vv * 8 + y], s);
             if (RAW) raw_out[gb * 64 + y * 8 + x] = s;
-            else a.plane[(int64_t)(by * 8 + y) * a.stride + bx * 8 + x] = (uint8_t)cj_clip8(tc_round(s) + 128);
+            else px[(int64_t)(y - TC_ROWS * h) * a.stride + x] = (uint8_t)cj_clip8(tc_round(s) + 128);
           }
         }
       }
+      kb += (int64_t)gridDim.x * TC_M;
+      mrow += step_row;
+      mcol += step_col;
+      if (mcol >= mcux) mcol -= mcux, mrow++;
     }
+    fl_prev = fl;
+    fl = fl == flags + 2048 ? flags : fl + 1024;
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
