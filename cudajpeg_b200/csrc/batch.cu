@@ -1240,13 +1240,11 @@ __global__ void __launch_bounds__(MODE == CJ_PIX_IDCT_TC ? CJ_TC_THREADS : CJ_PI
   }
   CJTcState tc;
   if (MODE == CJ_PIX_IDCT_TC) {
-    // the swizzled A tile starts on the first 1024-byte boundary of its
-    // region (the dynamic shared memory itself need not be so aligned)
-    uint8_t* a_region = smem + CJ_TC_A_OFF;
-    tc.a_tile = a_region + ((1024u - (cj_smem_addr(a_region) & 1023u)) & 1023u);
-    // the A tile starts zeroed (rows past a tile's blocks are never written)
-    for (int k = threadIdx.x; k < 16384 / 16; k += blockDim.x)
-      reinterpret_cast<uint4*>(tc.a_tile)[k] = make_uint4(0, 0, 0, 0);
+    // (the dynamic shared memory itself need not be aligned; rows of a tile past
+    // its blocks hold what they hold: only their own outputs, which nothing reads,
+    // depend on them)
+    uint8_t* region = smem + CJ_TC_SC_OFF;
+    tc.tiles = region + ((1024u - (cj_smem_addr(region) & 1023u)) & 1023u);
     // the hi/lo Kronecker basis, built once per device, into the B operand
     const uint4* gb = reinterpret_cast<const uint4*>(a.tc_basis);
     for (int k = threadIdx.x; k < 16384 / 16; k += blockDim.x)
@@ -1375,10 +1373,9 @@ __device__ __forceinline__ void bt_pixel_tiles(const CJBatchArgs& a, int t0, int
 // holds up to CJ_TC_MAXB blocks (cj_pix_tile_mcus_tc) and costs two
 // barrier-separated phases:
 //   1. thread 0 issues the tile's 8 MMAs (its A tile was built in the
-//      previous phase) and the bulk copy of the coefficients of the tile
-//      CJ_TC_NBUF ahead (into the buffer this tile's A was built from);
-//      every thread waits for the MMAs and runs the epilogue into the plane
-//      tiles -- barrier -- (rare: the FP32 redo of range-flagged blocks);
+//      previous phase); every thread waits for them, thread 0 starts the bulk
+//      copy of the coefficients of the tile CJ_TC_NBUF ahead into this one's
+//      place, and every thread runs the epilogue into the plane tiles -- barrier -- (rare: the FP32 redo of range-flagged blocks);
 //   2. the output of the tile from the plane tiles, then the A tile of the
 //      next tile from its copied coefficients -- barrier.
 // The output and the next A build share a phase, so no warp idles through
@@ -1397,9 +1394,7 @@ __device__ __forceinline__ void bt_pixel_tiles_tc(const CJBatchArgs& a, int t0, 
   };
   // tile u's coefficient buffer, and the wait for its copy (each buffer's
   // barrier completes one phase per tile it receives)
-  auto sc_of = [&](int u) {
-    return reinterpret_cast<int16_t*>(smem + CJ_TC_SC_OFF + ((u - t0) % CJ_TC_NBUF) * CJ_TC_COEF_BYTES);
-  };
+  auto tile_of = [&](int u) { return tc->tiles + ((u - t0) % CJ_TC_NBUF) * CJ_TC_COEF_BYTES; };
   auto wait_copy = [&](int u) {
     return cj_mbar_wait(&bar2[(u - t0) % CJ_TC_NBUF], (uint32_t)(((u - t0) / CJ_TC_NBUF) & 1));
   };
@@ -1415,8 +1410,8 @@ __device__ __forceinline__ void bt_pixel_tiles_tc(const CJBatchArgs& a, int t0, 
       s_pimg = nimg;
     }
     const int local = u - a.desc[nimg].ptile0, gx = (s_pg.mcux + s_pg.T - 1) / s_pg.T;
-    cj_pixel_issue(a.coef + a.desc[nimg].coef0 * 64, s_pg, local / gx, (local % gx) * s_pg.T, sc_of(u),
-                   &bar2[(u - t0) % CJ_TC_NBUF]);
+    cj_pixel_issue(a.coef + a.desc[nimg].coef0 * 64, s_pg, local / gx, (local % gx) * s_pg.T,
+                   reinterpret_cast<int16_t*>(tile_of(u)), &bar2[(u - t0) % CJ_TC_NBUF]);
   };
   int img = bt_find(a.n, t0, [&](int k) { return a.desc[k].ptile0; });
   int issued_to = min(t0 + CJ_TC_NBUF, t1);  // copies of tiles [.., issued_to) are issued
@@ -1443,7 +1438,7 @@ __device__ __forceinline__ void bt_pixel_tiles_tc(const CJBatchArgs& a, int t0, 
   __syncthreads();  // the setup before the first A build
   if (!wait_copy(t0)) cj_tile_fail = 1;
   waited_to = t0 + 1;
-  cj_tc_build_a(nblk, sc_of(t0), tc->a_tile, big, P);
+  cj_tc_build_a(nblk, tile_of(t0), big, P);
   __syncthreads();
   if (cj_pixel_failed(&a.st[img])) {
     leave();
@@ -1452,14 +1447,15 @@ __device__ __forceinline__ void bt_pixel_tiles_tc(const CJBatchArgs& a, int t0, 
   for (int t = t0; t < t1; t++) {
     // ---- phase 1: the tile's MMAs, the copy CJ_TC_NBUF tiles ahead, the epilogue
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (threadIdx.x == 0) {
-      tc_idct_mmas_asw(tc->tmem, cj_smem_addr(tc->a_tile), cj_smem_addr(smem + CJ_TC_B_OFF), cj_smem_addr(tc->bar));
-      if (t + CJ_TC_NBUF < t1) issue(t + CJ_TC_NBUF);
-    }
-    if (t + CJ_TC_NBUF < t1) issued_to = t + CJ_TC_NBUF + 1;
+    if (threadIdx.x == 0)
+      tc_idct_mmas_asw(tc->tmem, cj_smem_addr(tile_of(t)), cj_smem_addr(smem + CJ_TC_B_OFF), cj_smem_addr(tc->bar));
     const bool ok = cj_mbar_wait(tc->bar, tc->parity);
     tc->parity ^= 1u;
     if (!ok) cj_tile_fail = 1;
+    if (ok && t + CJ_TC_NBUF < t1) {  // the MMAs have read the tile: the copy that takes its place
+      if (threadIdx.x == 0) issue(t + CJ_TC_NBUF);
+      issued_to = t + CJ_TC_NBUF + 1;
+    }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const bool flagged = cj_tc_epilogue(g, nblk, smem, big, P, *tc, ok);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -1495,7 +1491,7 @@ __device__ __forceinline__ void bt_pixel_tiles_tc(const CJBatchArgs& a, int t0, 
       nblk = min(g.T, g.mcux - tcol * g.T) * g.bpm;
       if (!wait_copy(t + 1)) cj_tile_fail = 1;
       waited_to = t + 2;
-      cj_tc_build_a(nblk, sc_of(t + 1), tc->a_tile, big, P);
+      cj_tc_build_a(nblk, tile_of(t + 1), big, P);
     }
     __syncthreads();  // the output is written, the next A tile is complete
     if (cj_pixel_failed(&a.st[img])) {

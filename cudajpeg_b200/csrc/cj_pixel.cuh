@@ -82,14 +82,15 @@ struct CJPixGeom {
 #endif
 // Coefficient buffers of a tensor-core tile (TMA bulk copies in flight) and
 // the CTAs per SM its kernel is compiled for (its register cap).  Measured on
-// the 1024-image mix: one buffer at 3 CTAs/SM (60 KB of shared memory each)
-// runs the pixel stage in 1.04 ms, two buffers at 2 CTAs/SM in 1.24 ms, and
-// 64-block tiles at 4 CTAs/SM in 1.42-1.48 ms.
+// the 1024-image mix, pixel stage: one buffer at 4 CTAs/SM (43 KB of shared memory
+// each, 64 registers) 1.00 ms, at 3 CTAs/SM 1.09, two buffers at 3 CTAs/SM 1.13;
+// with an A tile of its own beside the coefficient buffer (60 KB, 3 CTAs/SM) 1.05.
+// What bounds it is instruction issue (58%, 32 warps) and the two barriers a tile.
 #ifndef CJ_TC_NBUF
 #define CJ_TC_NBUF 1
 #endif
 #ifndef CJ_TC_MINB
-#define CJ_TC_MINB 3
+#define CJ_TC_MINB 4
 #endif
 // Threads of a tensor-core pixel CTA: the epilogue splits each block's 64
 // outputs over CJ_TC_THREADS / 128 threads (warps w, w + 4, ... share TMEM
@@ -144,16 +145,14 @@ CJ_HD int cj_pix_check(const CJScanParams* hp) {
 // a batch CTA may come from different images -- never overlap the current
 // tile's working space.  The tensor-core form (tc) has a layout of its own
 // whose regions do not depend on the geometry either: the plane tiles first
-// (64 bytes per block: at most CJ_TC_SC_OFF), then CJ_TC_NBUF coefficient
-// buffers of CJ_TC_MAXB blocks, the 128-row FP16 A tile (16 KiB, in the
-// 128-byte swizzled layout, which must start on a 1024-byte boundary: the
-// region holds 1 KiB of slack and the kernel aligns the tile inside it), the
-// hi/lo Kronecker basis (16 KiB) and one range flag per block row.
+// (64 bytes per block: at most CJ_TC_SC_OFF), then CJ_TC_NBUF buffers of
+// CJ_TC_MAXB blocks, each first a tile's coefficients and then, in place, its
+// FP16 A tile (16 KiB, in the 128-byte swizzled layout, which must start on a
+// 1024-byte boundary: the region holds 1 KiB of slack and the kernel aligns the
+// buffers inside it), the hi/lo Kronecker basis (16 KiB) and one range flag per block row.
 #define CJ_TC_COEF_BYTES (CJ_TC_MAXB * 128)
 #define CJ_TC_SC_OFF (CJ_TC_MAXB * 64)
-#define CJ_TC_A_OFF (CJ_TC_SC_OFF + CJ_TC_NBUF * CJ_TC_COEF_BYTES)
-#define CJ_TC_A_BYTES (16384 + 1024)
-#define CJ_TC_B_OFF (CJ_TC_A_OFF + CJ_TC_A_BYTES)
+#define CJ_TC_B_OFF (CJ_TC_SC_OFF + CJ_TC_NBUF * CJ_TC_COEF_BYTES + 1024)
 #define CJ_TC_BIG_OFF (CJ_TC_B_OFF + 16384)
 #define CJ_TC_SMEM_BYTES (CJ_TC_BIG_OFF + CJ_TC_MAXB * 8)
 CJ_HD size_t cj_pix_layout(CJPixGeom* g, int csx, int csy, int nbuf = 1, bool tc = false) {
@@ -168,7 +167,7 @@ CJ_HD size_t cj_pix_layout(CJPixGeom* g, int csx, int csy, int nbuf = 1, bool tc
     g->cr_off = g->cb_off + csz_tc;
     g->sc1_off = CJ_TC_COEF_BYTES;  // from one coefficient buffer to the next
     g->tmp_off = 0;                 // unused
-    g->a_off = CJ_TC_A_OFF;
+    g->a_off = CJ_TC_SC_OFF;
     g->b_off = CJ_TC_B_OFF;
     g->big_off = CJ_TC_BIG_OFF;
     return CJ_TC_SMEM_BYTES;
@@ -341,7 +340,7 @@ struct CJTcState {
   uint64_t* bar;
   uint32_t parity;
   const float* basis;
-  uint8_t* a_tile;  // the swizzled A tile: inside the A region, on a 1024-byte boundary
+  uint8_t* tiles;  // the CJ_TC_NBUF coefficient / A tiles, on a 1024-byte boundary
 };
 
 // Tensor-core iDCT of a tile's blocks (at most CJ_TC_MAXB, rows of the
@@ -352,15 +351,17 @@ struct CJTcState {
 // the DC biased by TC_DC_BIAS (exact below 2048; a block row at or above it
 // sets the row's range flag),
 // in the 128-byte swizzled layout (conflict-free stores of a block's 8 rows),
-// then the proxy fence that makes the rows visible to the MMAs.
-__device__ __forceinline__ void cj_tc_build_a(int nblk, const int16_t* sc, uint8_t* sA, uint8_t* big,
-                                              const CJPixSmemParams& P) {
+// in place of the coefficients (a block's 8 rows are one warp's), then the proxy
+// fence that makes the rows visible to the MMAs.
+__device__ __forceinline__ void cj_tc_build_a(int nblk, uint8_t* tile, uint8_t* big, const CJPixSmemParams& P) {
   // a thread always builds row v = threadIdx.x & 7 (blockDim.x is a multiple
   // of 8); row 0's DC gets the rounding bias (TC_DC_BIAS)
   const __half2 bias = __halves2half2(__float2half_rn((threadIdx.x & 7) ? 0.f : TC_DC_BIAS), __float2half_rn(0.f));
-  for (int t = threadIdx.x; t < nblk * 8; t += blockDim.x) {
-    const int kb = t >> 3, v = t & 7;
-    const uint4 raw = *reinterpret_cast<const uint4*>(sc + kb * 64 + v * 8);
+  for (int t = threadIdx.x; (t & ~31) < nblk * 8; t += blockDim.x) {  // warp-uniform
+    const int kb = min(t >> 3, nblk - 1), v = t & 7;
+    const uint4 raw = *reinterpret_cast<const uint4*>(tile + kb * 128 + v * 16);
+    __syncwarp();  // read before they are overwritten
+    if (t >= nblk * 8) continue;
     const uint4 qv = *reinterpret_cast<const uint4*>(&P.qh[P.bq[kb]][v * 8]);
     const uint32_t rw[4] = {raw.x, raw.y, raw.z, raw.w}, qw[4] = {qv.x, qv.y, qv.z, qv.w};
     uint32_t p[4];
@@ -374,7 +375,7 @@ __device__ __forceinline__ void cj_tc_build_a(int nblk, const int16_t* sc, uint8
       top = __hmax2_nan(top, __habs2(pr));
     }
     big[t] = tc_beyond(top);
-    *reinterpret_cast<uint4*>(sA + tc_sw128_off(kb, v)) = make_uint4(p[0], p[1], p[2], p[3]);
+    *reinterpret_cast<uint4*>(tile + tc_sw128_off(kb, v)) = make_uint4(p[0], p[1], p[2], p[3]);
   }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
