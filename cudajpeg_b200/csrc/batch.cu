@@ -234,10 +234,24 @@ __device__ __forceinline__ uint64_t bt_map_compose(uint64_t f, uint64_t g, int n
   return o;
 }
 
+// Index of the first of the records h[0 .. last] whose exit is `exit`, 15 if none.
+// The loads go out together: one after another, ten of them were 4 us on the way of
+// every probe and settle round.
+__device__ __forceinline__ uint32_t bt_exit_index(const CJSubRec* h, int last, uint64_t exit) {
+  uint64_t e[BT_MAX_HYP];
+#pragma unroll
+  for (int p = 0; p < BT_MAX_HYP; p++) e[p] = p <= last ? __ldcg(&h[p].exit) : 0;
+  uint32_t q = 15;
+#pragma unroll
+  for (int p = BT_MAX_HYP - 1; p >= 0; p--)
+    if (p <= last && e[p] == exit) q = (uint32_t)p;
+  return q;
+}
+
 // The settle of the hypothesis variant: cj_warp_settle's loop and fixed
 // point, with the probe decodes as shortcuts.  Each round the first lane u
 // whose input moved has a final input (every lane before it is consistent).
-// If that input is one of its predecessor's hypothesis exits, the lanes from
+// If that input is one of its predecessor's hypothesis exits (bt_exit_index), the lanes from
 // u on follow the maps (a warp-wide prefix composition) to the hypothesis
 // each predecessor ends on, and every lane with a known predecessor
 // hypothesis takes the probe decode from that hypothesis's exit (record and
@@ -277,15 +291,7 @@ __device__ __forceinline__ bool bt_settle_map(const CJBatchArgs& a, CJSpecJob& x
     if (!cb) break;
     const int u = __ffs(cb) - 1;
     uint32_t q = 15;  // lane u: its input as a predecessor hypothesis
-    if (lane == u) {
-      const CJSubRec* ph = a.hrecs + (gs - 1) * 2 * NH;
-      const int pmax = pred_head ? 0 : nhi;
-      for (int p = 0; p <= pmax; p++)
-        if (__ldcg(&ph[p].exit) == want) {
-          q = (uint32_t)p;
-          break;
-        }
-    }
+    if (lane == u) q = bt_exit_index(a.hrecs + (gs - 1) * 2 * NH, pred_head ? 0 : nhi, want);
     uint64_t v = lane < u ? BT_MAP_ID : (lane == u ? bt_map_const(bt_map_at(M, q)) : M);
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
@@ -296,13 +302,17 @@ __device__ __forceinline__ bool bt_settle_map(const CJBatchArgs& a, CJSpecJob& x
     if (lane == u) pidx = q;
     const bool probe = ln.active && !ln.head && lane >= u && pidx < 15, redo = change && !probe;
     if (probe) {
-      const CJSubRec* pr = hrec + NH + pidx;
-      if (__ldcg(&pr->start) != r.start) {
-        r = bt_load_rec(pr);
-        const CJCkpt* pc = cj_lane_ckpts(a.hckpt, hb + NH + pidx);
-        for (int k = 0; k < CJ_CKPTS; k++)
-          ck[k] = CJCkpt{__ldcg(&pc[k].pp), __ldcg(&pc[k].nb), __ldcg(&pc[k].d0), __ldcg(&pc[k].d1),
-                         __ldcg(&pc[k].d2)};
+      // (the checkpoints' loads do not wait for the comparison)
+      const CJSubRec pr = bt_load_rec(hrec + NH + pidx);
+      const CJCkpt* pc = cj_lane_ckpts(a.hckpt, hb + NH + pidx);
+      CJCkpt c[CJ_CKPTS];
+#pragma unroll
+      for (int k = 0; k < CJ_CKPTS; k++)
+        c[k] = CJCkpt{__ldcg(&pc[k].pp), __ldcg(&pc[k].nb), __ldcg(&pc[k].d0), __ldcg(&pc[k].d1), __ldcg(&pc[k].d2)};
+      if (pr.start != r.start) {
+        r = pr;
+#pragma unroll
+        for (int k = 0; k < CJ_CKPTS; k++) ck[k] = c[k];
         dirty = true;
       }
     }
@@ -891,11 +901,7 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) k_decode_batch(CJBatchArgs a
         cj_spec_warp<true>(&x, run, from);
         if (run) {
           a.hrecs[hb + (nh + 1) + p] = x.r;
-          for (int k = 0; k <= nhi; k++)
-            if (__ldcg(&a.hrecs[hb + k].exit) == x.r.exit) {
-              mk = (uint8_t)k;
-              break;
-            }
+          mk = (uint8_t)bt_exit_index(a.hrecs + hb, nhi, x.r.exit);
         }
         if (ln.active) a.hmap[gs * 16 + p] = mk;
       });
