@@ -72,11 +72,10 @@ int cjReaderRedecodeDevice(JPGReader* r) {
 int cjReaderSync(JPGReader* r) {
   CJReaderDevice* d = r->dev;
   if (!d->gpu_ready) return PROGRAMMER_ERROR;
-  CJ_CUDA_TRY(cudaMemcpyAsync(d->h_status.p, d->status.p, sizeof(CJStatus), cudaMemcpyDeviceToHost,
-                              d->stream),
-              CUDA_MEM_ERROR);
+  int err = cj_reader_copy_status(d);
+  if (err) return err;
   CJ_CUDA_TRY(cudaStreamSynchronize(d->stream), CUDA_KERNEL_LAUNCH_ERROR);
-  int err = cj_reader_decode_status(r);
+  err = cj_reader_decode_status(r);
   return err ? err : cj_status_error((const CJStatus*)d->h_status.p);
 }
 

@@ -2780,8 +2780,18 @@ int cjBatchAutotune(CJBatch* b, int n, const unsigned char* blob, const int64_t*
 // decode kernel on the reader's one image, in the reader's grow-only
 // buffers -- one cooperative launch, Huffman tables built on the device,
 // fix-up passes looped on the device.  The grid is the co-resident maximum,
-// cut to the image's work (destuff tiles, warp groups) for small images so
-// that idle CTAs do not lengthen the grid barriers.
+// cut to the image's work (destuff tiles, warp groups; at least a CTA per SM) for
+// small images so that idle CTAs do not lengthen the grid barriers.
+//
+// Header, plan and the zeroed control block go to the device in one copy, and
+// nothing comes back between the decode and the pixel kernel: a copy of the control
+// block there held the pixel
+// kernel up by 12 us.
+struct BTReaderBlock {
+  CJImageHeader hdr;
+  alignas(16) CJImageDesc desc;
+  alignas(16) CJBatchCtl ctl;
+};
 int cj_reader_decode(JPGReader* jpg, bool stage) {
   CJReaderDevice* d = jpg->dev;
   cudaStream_t s = d->stream;
@@ -2814,7 +2824,7 @@ int cj_reader_decode(JPGReader* jpg, bool stage) {
     }
     bt_plan_one(h, n, sub, &desc);
     const int nwarps = desc.sub_cap / 32;
-    if (cj_dev_ensure(d->bhdr, sizeof(CJImageHeader)) || cj_dev_ensure(d->bdesc, sizeof(CJImageDesc)) ||
+    if (cj_dev_ensure(d->bhdr, sizeof(BTReaderBlock)) ||
         cj_dev_ensure(d->params, sizeof(CJScanParams)) || cj_dev_ensure(d->spec, sizeof(CJSpecTab)) ||
         cj_dev_ensure(d->status, sizeof(CJStatus)) ||
         cj_dev_ensure(d->raw, (size_t)n + 64) || cj_dev_ensure(d->data, (size_t)n + 64) ||
@@ -2826,7 +2836,7 @@ int cj_reader_decode(JPGReader* jpg, bool stage) {
         cj_dev_ensure(d->snap, (size_t)2 * nwarps * sizeof(uint64_t)) ||
         cj_dev_ensure(d->wagg, (size_t)nwarps * sizeof(CJWarpAgg)) ||
         cj_dev_ensure(d->carry, (size_t)nwarps * sizeof(CJWarpAgg)) ||
-        cj_dev_ensure(d->coef, (size_t)h.total_blocks * 128 + 128) || cj_dev_ensure(d->bctl, sizeof(CJBatchCtl)))
+        cj_dev_ensure(d->coef, (size_t)h.total_blocks * 128 + 128))
       return CUDA_MEM_ERROR;
     if (cj_host_ensure(d->h_bctl, sizeof(CJBatchCtl))) return OOM_ERROR;
     // MCU-phase hypotheses where they pay and fit (bt_fill_bits)
@@ -2857,18 +2867,23 @@ int cj_reader_decode(JPGReader* jpg, bool stage) {
     d->total_blocks = h.total_blocks;
     d->param_bytes = sizeof(CJImageHeader) + sizeof(CJImageDesc);
     CJ_CUDA_TRY(cudaEventRecord(d->ev_begin, s), CUDA_KERNEL_LAUNCH_ERROR);
-    CJ_CUDA_TRY(cudaMemcpyAsync(d->bhdr.p, &h, sizeof(h), cudaMemcpyHostToDevice, s), CUDA_MEM_ERROR);
-    CJ_CUDA_TRY(cudaMemcpyAsync(d->bdesc.p, &desc, sizeof(desc), cudaMemcpyHostToDevice, s), CUDA_MEM_ERROR);
+    BTReaderBlock blk;
+    memset(&blk, 0, sizeof(blk));
+    blk.hdr = h;
+    blk.desc = desc;
     // (a copy from pageable memory returns once its source has been staged,
-    // so the header and plan may live on this stack frame)
+    // so the block may live on this stack frame)
+    CJ_CUDA_TRY(cudaMemcpyAsync(d->bhdr.p, &blk, sizeof(blk), cudaMemcpyHostToDevice, s), CUDA_MEM_ERROR);
     if (n) CJ_CUDA_TRY(cudaMemcpyAsync(d->raw.p, jpg->pos, (size_t)n, cudaMemcpyHostToDevice, s), CUDA_MEM_ERROR);
   } else {
     CJ_CUDA_TRY(cudaEventRecord(d->ev_begin, s), CUDA_KERNEL_LAUNCH_ERROR);
+    CJ_CUDA_TRY(cudaMemsetAsync(&((BTReaderBlock*)d->bhdr.p)->ctl, 0, sizeof(CJBatchCtl), s), CUDA_MEM_ERROR);
   }
+  BTReaderBlock* const block = (BTReaderBlock*)d->bhdr.p;  // (device addresses)
   CJBatchArgs a;
   memset(&a, 0, sizeof(a));
-  a.hdr = (const CJImageHeader*)d->bhdr.p;
-  a.desc = (const CJImageDesc*)d->bdesc.p;
+  a.hdr = &block->hdr;
+  a.desc = &block->desc;
   a.prm = (CJScanParams*)d->params.p;
   a.spec = (CJSpecTab*)d->spec.p;
   a.st = (CJStatus*)d->status.p;
@@ -2886,7 +2901,7 @@ int cj_reader_decode(JPGReader* jpg, bool stage) {
   a.wagg = (CJWarpAgg*)d->wagg.p;
   a.carry = (CJWarpAgg*)d->carry.p;
   a.coef = (int16_t*)d->coef.p;
-  a.ctl = (CJBatchCtl*)d->bctl.p;
+  a.ctl = &block->ctl;
   a.n = 1;
   a.ntiles = d->b_ntiles;
   a.nwarps = d->b_nwarps;
@@ -2897,7 +2912,6 @@ int cj_reader_decode(JPGReader* jpg, bool stage) {
   a.hckpt = (CJCkpt*)d->hckpt.p;
   a.hmap = (uint8_t*)d->hmap.p;
   cj_profile_begin(d);
-  CJ_CUDA_TRY(cudaMemsetAsync(d->bctl.p, 0, sizeof(CJBatchCtl), s), CUDA_MEM_ERROR);
   void* args[] = {&a};
   CJ_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)bt_decode_kernel(BT_DECODE_CTAS_DEFAULT, d->b_nhyp > 1),
                                           dim3(d->b_grid),
@@ -2905,8 +2919,16 @@ int cj_reader_decode(JPGReader* jpg, bool stage) {
               CUDA_KERNEL_LAUNCH_ERROR);
   cj_after_launch(d, CJ_K_DECODE_BATCH);
   CJ_CUDA_TRY(cudaEventRecord(d->ev_scan, s), CUDA_KERNEL_LAUNCH_ERROR);
-  CJ_CUDA_TRY(cudaMemcpyAsync(d->h_bctl.p, d->bctl.p, sizeof(CJBatchCtl), cudaMemcpyDeviceToHost, s),
+  return 0;
+}
+
+int cj_reader_copy_status(CJReaderDevice* d) {
+  CJ_CUDA_TRY(cudaMemcpyAsync(d->h_status.p, d->status.p, sizeof(CJStatus), cudaMemcpyDeviceToHost, d->stream),
               CUDA_MEM_ERROR);
+  if (d->bhdr.p && d->h_bctl.p && !d->progressive)
+    CJ_CUDA_TRY(cudaMemcpyAsync(d->h_bctl.p, &((BTReaderBlock*)d->bhdr.p)->ctl, sizeof(CJBatchCtl),
+                                cudaMemcpyDeviceToHost, d->stream),
+                CUDA_MEM_ERROR);
   return 0;
 }
 

@@ -45,7 +45,7 @@ struct CJReaderDevice {
   cudaStream_t stream = nullptr;
   cudaEvent_t ev_begin = nullptr, ev_scan = nullptr, ev_end = nullptr;
   CJDevBuf raw, data, tile_keep, tile_mark, mpos, mcode, segs, recs, ckpt, snap, wagg, carry, coef,
-      pix, params, spec, status, wcoef, bhdr, bdesc, bctl, pscan, hrecs, hckpt, hmap;
+      pix, params, spec, status, wcoef, bhdr, pscan, hrecs, hckpt, hmap;
   CJHostBuf h_params, h_status, h_pixels, h_file, h_bctl;
   // per-scan bookkeeping
   int sub_bits = CJ_SUB_BITS_DEFAULT;
@@ -108,6 +108,8 @@ int cj_prog_finish(JPGReader* jpg);
 // re-run the decode over what is already there.  Asynchronous on the
 // reader's stream.
 int cj_reader_decode(JPGReader* jpg, bool stage);
+// Enqueue the copies of the decode's status to the host.
+int cj_reader_copy_status(CJReaderDevice* d);
 // After the reader's stream has been synchronised: CUDA_KERNEL_LAUNCH_ERROR
 // when a grid-barrier wait of the last decode timed out, else 0.
 int cj_reader_decode_status(const JPGReader* jpg);

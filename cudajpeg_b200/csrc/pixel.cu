@@ -102,10 +102,7 @@ int cj_pixel_launch(JPGReader* jpg, bool copy_out) {
   if (!copy_out) return 0;
   CJ_CUDA_TRY(cudaMemcpyAsync(d->h_pixels.p, d->pix.p, npix, cudaMemcpyDeviceToHost, d->stream),
               CUDA_MEM_ERROR);
-  CJ_CUDA_TRY(cudaMemcpyAsync(d->h_status.p, d->status.p, sizeof(CJStatus), cudaMemcpyDeviceToHost,
-                              d->stream),
-              CUDA_MEM_ERROR);
-  return 0;
+  return cj_reader_copy_status(d);
 }
 
 int cj_export_coefficients(JPGReader* jpg) {
