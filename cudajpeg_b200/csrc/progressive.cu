@@ -58,7 +58,10 @@ struct CJProgWork {
 // one thread decoding each scan from global memory; in chunks, a launch per level
 // of scans 17.4 ms with a walk of 132 cycles a symbol, 13.1 ms with the present one
 // (1.5 + 3.8 + 7.6, the last luma refinement's 129 thousand symbols); in one launch
-// 8.1 ms; with a refinement's blocks staged in shared memory 7.6 ms.
+// 8.1 ms; with a refinement's blocks staged in shared memory 7.6 ms, and with no more in
+// its walk than the next position takes 6.7 ms (about 95 cycles a symbol in all; loading
+// the four nearest entries ahead, to save the second load's latency, 9.3 ms: the
+// instructions count too).
 #define PG_THREADS 512
 #define PG_BITS 16384        // bit positions of a chunk
 #define PG_BLOCK_BITS 2048   // no block takes more bits than this (63 symbols of 31 bits and an EOB)
@@ -84,7 +87,7 @@ struct PGShared {
   uint32_t ev0[PG_SEQ];
   uint32_t coef[PG_REF_BLOCKS][33];     // the blocks before the scan (33: a thread per block, each in a bank of its own)
   uint64_t hist[PG_REF_BLOCKS];         // nonzero coefficients of the band, bit = zig-zag position - ss
-  uint8_t nz[PG_REF_BLOCKS];
+  uint8_t nz[PG_REF_BLOCKS + 1];
   uint8_t zz[64];
   uint8_t pcomp[CJ_MAX_BPM], pslot[CJ_MAX_BPM];
   int32_t pofs[CJ_MAX_BPM];
@@ -287,57 +290,66 @@ __device__ __forceinline__ void pg_walk_first(PGShared& S, int nb, int ss, int s
 // has met k - (z + r) nonzero ones, whose correction bits lie behind the
 // symbols: with q the bits of the block's symbols alone, the next symbol is at
 // q + k - (z + r).  Every block takes one correction bit per nonzero coefficient
-// in all.  Event: offset of a symbol, z + r << 16 (PG_AT_EOB: an end-of-band
-// symbol; PG_IN_RUN: a block inside a run, position of its correction bits).
-#define PG_AT_EOB 0xFFu
-#define PG_IN_RUN 0xFEu
+// in all.  Event: shared address of a symbol's entry; PG_IN_RUN: a block inside a run,
+// of its correction bits (by position).
+// One thread issues an instruction every 4 cycles or so: what the loop does not need
+// (z + r, the band position) is left to those who read the events.
+#define PG_IN_RUN 0x80000000u
 __device__ __forceinline__ void pg_walk_refine(PGShared& S, int nb, int width) {
   const uint32_t sym = (uint32_t)__cvta_generic_to_shared(S.sym), zpos = (uint32_t)__cvta_generic_to_shared(S.zpos);
-  const uint32_t last = 4 * (uint32_t)(width - 1);
-  uint32_t pos = 4 * S.bit;
-  int b = 0, eob = S.eob, ne = 0;
-  while (b < nb && pos < 4 * (PG_BITS - PG_BLOCK_BITS) && ne < PG_EVENTS - 64) {
-    const uint32_t nz4 = 4u * S.nz[b];
-    S.ev0[b] = ne;
+  const uint32_t last = 4 * (uint32_t)(width - 1), stop = sym + 4 * (PG_BITS - PG_BLOCK_BITS);
+  uint32_t pos = sym + 4 * S.bit, e = pg_lds32(pos), nz_next = 4u * S.nz[0];
+  int b = 0, eob = S.eob;
+  uint32_t* evt = S.evt;
+  while (b < nb && pos < stop && evt < S.evt + PG_EVENTS - 64) {
+    const uint32_t nz4 = nz_next;
+    nz_next = 4u * S.nz[b + 1];
+    S.ev0[b] = (uint32_t)(evt - S.evt);
     if (eob) {
-      S.evt[ne++] = pos | (PG_IN_RUN << 16);
+      *evt++ = pos | PG_IN_RUN;
       pos += nz4;
+      e = pg_lds32(pos);
       eob--;
       b++;
       continue;
     }
-    uint32_t e = pg_lds32(sym + pos), q = pos, z = zpos + b * PG_ZPOS - 1, k4, next;
-    const uint32_t z0 = z + 1;
+    const uint32_t z0 = zpos + b * PG_ZPOS;
+    uint32_t q = pos + 4, z = z0 - 1, k4, next;  // q: behind the block's symbols alone, less 4 (z + r); z + r = -1
     for (;;) {
-      z += (e >> 8) & 255;
+      const uint32_t run = (e >> 8) & 255;
+      z += run;
       k4 = pg_lds8(z);
-      q += e & 255;
-      S.evt[ne++] = pos | ((z - z0) << 16);
-      const uint32_t at = q - 4 * (z - z0) + k4;
-      next = pg_lds32(sym + at);
+      q = q + (e & 255) - 4 * run;
+      *evt++ = pos;
+      const uint32_t at = q + k4;
+      next = pg_lds32(at);
       if (k4 >= last) {
-        if (k4 < PG_ZEND) pos = at;
+        if (k4 < PG_ZEND) {
+          pos = at;
+          e = next;
+        }
         break;
       }
       pos = at;
       e = next;
     }
     if (k4 >= PG_ZEND) {  // past the band: an end-of-band run, an error, or a ZRL that ends the block
+      pos = q + 4 * (z - z0) + nz4;
+      next = pg_lds32(pos);
       if (e & PG_EOB) {
-        S.evt[ne - 1] = pos | (PG_AT_EOB << 16);
         eob = (int)((e >> 16) & 0x7FFF);
       } else if (e & (PG_BAD | 0xFF0000u)) {
         S.err = CJ_DEV_BAD_AC;
         break;
       }
-      pos = q + nz4;
+      e = next;
     }
     b++;
   }
-  S.pos = (int)(pos >> 2);
+  S.pos = (int)((pos - sym) >> 2);
   S.done = b;
   S.eob = eob;
-  if (!S.err) S.ev0[b] = ne;  // the end of the last block's events (an error's block is left out)
+  if (!S.err) S.ev0[b] = (uint32_t)(evt - S.evt);  // the end of the last block's events (an error's block is left out)
 }
 
 __constant__ uint8_t c_prog_zz[64] = CJ_ZIGZAG_INIT;
@@ -541,17 +553,21 @@ __global__ void __launch_bounds__(PG_THREADS) k_prog_scans(const CJProgBlock* __
         }
       } else {
         const int p1 = 1 << al, m1 = -(1 << al);
+        const uint32_t sym = (uint32_t)__cvta_generic_to_shared(S.sym);
         for (int b = tid; b < done; b += PG_THREADS) {
           int16_t* blk = coef + pg_block(s, S, u0, bps, blk0 + b) * 64;
           uint64_t h = S.hist[b];
           const int nz = S.nz[b];
           const int e1 = (int)S.ev0[b + 1];
-          int c = 0;  // corrections made
+          int c = 0;          // corrections made
+          uint32_t z = ~0u;  // zero-history coefficients passed, less 1
           for (int i = (int)S.ev0[b]; i < e1; i++) {
-            const uint32_t ev = S.evt[i], z = ev >> 16, e = S.sym[(ev & 0xFFFFu) >> 2];
-            const uint32_t k4 = z < PG_IN_RUN ? S.zpos[b][z] : PG_ZEND, k = k4 >> 2;
+            const uint32_t ev = S.evt[i], off = (ev & ~PG_IN_RUN) - sym, e = S.sym[off >> 2];
+            const bool in_run = (ev & PG_IN_RUN) != 0;
+            z += (e >> 8) & 255;
+            const uint32_t k4 = in_run ? PG_ZEND : S.zpos[b][z], k = k4 >> 2;
             const int c1 = k4 < PG_ZEND ? (int)(k - z) : nz;
-            uint32_t at = ((ev & 0xFFFFu) + (z == PG_IN_RUN ? 0u : e & 255)) >> 2;
+            uint32_t at = (off + (in_run ? 0u : e & 255)) >> 2;
             for (; c < c1; c++, at++) {
               const int zz = S.zz[s.ss + __ffsll((long long)h) - 1];
               const int v = reinterpret_cast<const int16_t*>(S.coef[b])[zz];
