@@ -2102,7 +2102,7 @@ int cjBatchStage(CJBatch* b, int n, const unsigned char* blob, const int64_t* of
     return OOM_ERROR;
   CJImageHeader* hh = (CJImageHeader*)b->h_hdr.p;
   CJImageDesc* dd = (CJImageDesc*)b->h_desc.p;
-  // Marker parse on the GPU: the files go to the device first, one thread per
+  // Marker parse on the GPU: the files go to the device first, one warp per
   // file parses its segments there (k_parse_headers); the headers stay on
   // the device and only the summaries the plan needs come back, through
   // mapped pinned memory.  The same parse runs on the host with
