@@ -140,6 +140,19 @@ struct CJSegment {
   int32_t pad;
 };
 
+// A block completed by a lane of a write-out warp.  The block counts from the
+// first block of the warp's first unit and takes a word of its own: another
+// lane's unit may lie anywhere in the image before or behind it (the next
+// restart interval begins at its own first block, however many blocks the data of
+// the one before it holds, and a truncated scan's padding decodes to the image's end).
+struct alignas(8) CJDone {
+  int32_t block;
+  uint32_t lane;
+};
+CJ_HD CJDone cj_done(int32_t block, uint32_t lane) { return CJDone{block, lane}; }
+// Its first 16-byte chunk in the coefficient buffer, from the same origin.
+CJ_HD int64_t cj_done_chunk(const CJDone& d) { return (int64_t)d.block * 8; }
+
 // Decoder state at a block boundary: bit position and MCU phase.
 CJ_HD uint64_t cj_state(uint64_t bit, uint32_t phase) { return (bit << 8) | phase; }
 CJ_HD uint64_t cj_state_bit(uint64_t s) { return s >> 8; }

@@ -158,6 +158,14 @@ __device__ __forceinline__ uint32_t cj_tab8(uint32_t a) {
   asm("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(a));
   return v;
 }
+__device__ __forceinline__ CJDone cj_lds_done(uint32_t a) {
+  CJDone v;
+  asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.block), "=r"(v.lane) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void cj_sts_done(uint32_t a, CJDone v) {
+  asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(a), "r"(v.block), "r"(v.lane) : "memory");
+}
 __device__ __forceinline__ uint4 cj_lds128(uint32_t a) {
   uint4 v;
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
@@ -635,7 +643,7 @@ __device__ __forceinline__ int64_t cj_lane_write_end(const CJLane& ln, const CJS
 struct CJWriteWarp {
   uint32_t ring[CJ_WRITE_WORDS][32];
   uint2 phase[CJ_MAX_BPM];
-  uint32_t order[32];  // completed blocks of a round
+  CJDone order[32];  // completed blocks of a round
 };
 
 // One lane's unit of the write-out (sp .. coef agree over the warp).
@@ -782,15 +790,15 @@ static __device__ __noinline__ void cj_write_warp(CJWriteJob* job, bool active) 
     }
     const unsigned mask = __ballot_sync(CJ_FULL, done);
     if (mask) {
-      if (done) cj_sts32(order + 4 * __popc(mask & ((1u << lane) - 1u)), ((uint32_t)b << 5) | (uint32_t)lane);
+      if (done) cj_sts_done(order + 8 * __popc(mask & ((1u << lane) - 1u)), cj_done(b, (uint32_t)lane));
       __syncwarp();
       const int n = __popc(mask);
       for (int r = lane >> 3; r < ((n + 3) & ~3); r += 4) {  // warp-uniform count
         if (r < n) {
-          const uint32_t o = cj_lds32(order + 4 * r), src = o & 31;
-          const uint32_t at = wsrc + 128 * src + ((((uint32_t)lane ^ src) & 7u) << 4);
+          const CJDone o = cj_lds_done(order + 8 * r);
+          const uint32_t at = wsrc + 128 * o.lane + ((((uint32_t)lane ^ o.lane) & 7u) << 4);
           const uint4 z = cj_lds128(at);
-          out[(int64_t)((int32_t)o >> 5) * 8] = z;
+          out[cj_done_chunk(o)] = z;
           cj_sts128_zero(at);
         }
       }
