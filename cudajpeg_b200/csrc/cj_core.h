@@ -153,6 +153,20 @@ CJ_HD CJDone cj_done(int32_t block, uint32_t lane) { return CJDone{block, lane};
 // Its first 16-byte chunk in the coefficient buffer, from the same origin.
 CJ_HD int64_t cj_done_chunk(const CJDone& d) { return (int64_t)d.block * 8; }
 
+// Positions of the write-out.  They are 32-bit and the data end at bit 2^31 at
+// the latest (CJ_MAX_SCAN_BYTES), but the last unit of a truncated scan decodes
+// on in 1-bits until its image's last block, which may take more than 2^32 of
+// them.  A position this far behind the data and its chunk index are put back by
+// whole rings of the bit window, to where there is still nothing but 1-bits.
+#define CJ_POS_FOLD 0xC0000000u
+#define CJ_POS_BACK (1u << 30)
+CJ_HD void cj_fold_position(uint32_t& pos, uint32_t& chunk) {
+  if (pos >= CJ_POS_FOLD) {
+    pos -= CJ_POS_BACK;
+    chunk -= CJ_POS_BACK / 128;
+  }
+}
+
 // Decoder state at a block boundary: bit position and MCU phase.
 CJ_HD uint64_t cj_state(uint64_t bit, uint32_t phase) { return (bit << 8) | phase; }
 CJ_HD uint64_t cj_state_bit(uint64_t s) { return s >> 8; }

@@ -255,6 +255,7 @@ struct CJWin {
       pf = load(cb + WORDS / 4);
       if (WORDS == 8) nn = word(2);  // read before its chunk was there, after 3 crossings
     }
+    if (WORDS == 8) cj_fold_position(pos, cb);  // (the write-out's)
   }
   __device__ __forceinline__ uint32_t peek() const { return __funnelshift_l(nxt, cur, pos); }
   // u <= 31: at most one word is crossed

@@ -26,3 +26,25 @@ def test_any_block_of_an_image_is_stored_at_its_place(tmp_path):
           }
       printf("done\\n");""")
     assert out == "done\n"
+
+
+def test_positions_in_a_truncated_scans_padding_do_not_wrap(tmp_path):
+    """2^34 bits of padding: the position stays behind the data, keeps its place in the window's ring of 8
+    words, and its chunk index keeps up with it."""
+    out = run_host(tmp_path, """
+      const uint32_t data_end = 8u * CJ_MAX_SCAN_BYTES;
+      uint32_t pos = data_end, cb = pos >> 7;
+      uint64_t full = pos;
+      for (uint32_t k = 0; full < 1ull << 34; k++) {
+        const uint32_t step = 3 * (k % 32);  // a round of three symbols
+        pos += step;
+        full += step;
+        cb = pos >> 7;
+        cj_fold_position(pos, cb);
+        if (pos < data_end || (pos & 255) != (full & 255) || cb != pos >> 7) {
+          printf("%u %llu\\n", pos, (unsigned long long)full);
+          break;
+        }
+      }
+      printf("done\\n");""")
+    assert out == "done\n"
