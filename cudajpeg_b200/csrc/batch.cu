@@ -38,6 +38,7 @@
 #include "cj_entropy.cuh"
 #include "cj_idct.cuh"
 #include "cj_internal.h"
+#include "cj_once.h"
 #include "cj_parse.cuh"
 #include "cj_pixel.cuh"
 #include "cj_scan_util.cuh"
@@ -2800,11 +2801,8 @@ int cj_reader_decode(JPGReader* jpg, bool stage) {
     int e = bt_fill_header(jpg, &h);
     if (e) return e;
     const int64_t n = (int64_t)(jpg->end - jpg->pos);
-    static bool attrs = false;  // per process: the attribute is per function, not per device
-    if (!attrs) {
-      CJ_CUDA_TRY(bt_decode_attrs(), CUDA_MEM_ERROR);
-      attrs = true;
-    }
+    static CJOncePerDevice attrs;
+    CJ_CUDA_TRY(attrs.run(d->device, bt_decode_attrs), CUDA_MEM_ERROR);
     int sms = 0, per_sm = 0;
     CJ_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d->device), CUDA_MEM_ERROR);
     CJ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(

@@ -18,6 +18,7 @@
 
 #include "../../include/pixelTransformGPU.h"
 #include "cj_internal.h"
+#include "cj_once.h"
 #include "cj_idct.cuh"
 #include "cj_pixel.cuh"
 
@@ -84,11 +85,10 @@ int cj_pixel_launch(JPGReader* jpg, bool copy_out) {
   size_t smem;
   int err = cj_pixel_geom(jpg, &g, &smem);
   if (err) return err;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaFuncSetAttribute(k_pixel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    attr_set = true;
-  }
+  static CJOncePerDevice attrs;
+  CJ_CUDA_TRY(attrs.run(d->device, [] {
+                return cudaFuncSetAttribute(k_pixel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+              }), CUDA_KERNEL_LAUNCH_ERROR);
   const size_t npix = (size_t)g.width * g.height * (g.nch == 3 ? 3 : 1);
   if (cj_dev_ensure(d->pix, npix + 16)) return CUDA_MEM_ERROR;
   if (cj_host_ensure(d->h_pixels, npix + 16)) return OOM_ERROR;
