@@ -47,7 +47,7 @@ EXPORTED = [
     "decodeScanGPU", "iDCT_resample_colourTransform", "cjIDCTPlane", "cjIDCTBlocksRaw",
     "cjReaderInfo", "cjReaderPixels", "cjReaderSetFlags", "cjReaderSetSubsequenceBits",
     "cjReaderStageTimes", "cjReaderDeviceCoefficients", "cjReaderDeviceQuantTable",
-    "cjReaderStream", "cjDebugHuffDecode", "cjReaderRedecodeDevice", "cjReaderSync",
+    "cjReaderSetWaitLimit", "cjReaderStream", "cjDebugHuffDecode", "cjReaderRedecodeDevice", "cjReaderSync",
     "cjReaderDevicePixels", "cjReaderSetProfile", "cjReaderKernelTimes", "cjReaderLaunchCount",
     "cjBatchCreate", "cjBatchDestroy", "cjBatchSetSubsequenceBits", "cjBatchStage", "cjBatchRun",
     "cjBatchFetch", "cjBatchWait", "cjBatchDecode", "cjBatchImage", "cjBatchDeviceImage",
@@ -103,6 +103,7 @@ def load(build_if_missing: bool = True):
     lib.cjReaderPixels.argtypes = [vp]
     lib.cjReaderSetFlags.argtypes = [vp, C.c_int]
     lib.cjReaderSetSubsequenceBits.argtypes = [vp, C.c_int]
+    lib.cjReaderSetWaitLimit.argtypes = [vp, C.c_uint]
     lib.cjReaderStageTimes.argtypes = [vp, C.POINTER(C.c_float)]
     lib.cjReaderDeviceCoefficients.restype = vp
     lib.cjReaderDeviceCoefficients.argtypes = [vp, i64p]
@@ -219,6 +220,11 @@ class Reader:
             raise ValueError(f"bad subsequence size {bits}")
 
     # ---- decode
+    def set_wait_limit(self, polls: int):
+        err = self.lib.cjReaderSetWaitLimit(self.ptr, polls)
+        if err:
+            raise DecodeError(err)
+
     def open(self, path: str, check: bool = True) -> int:
         err = self.lib.openJPG(self.ptr, os.fsencode(path))
         if check and err:

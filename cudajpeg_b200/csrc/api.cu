@@ -40,6 +40,12 @@ int cjReaderSetSubsequenceBits(JPGReader* r, int bits) {
   return 0;
 }
 
+int cjReaderSetWaitLimit(JPGReader* r, unsigned polls) {
+  if (!r) return PROGRAMMER_ERROR;
+  r->dev->wait_limit = polls;
+  return 0;
+}
+
 void cjReaderStageTimes(const JPGReader* r, float* ms) {
   const CJReaderDevice* d = r->dev;
   ms[0] = ms[1] = 0.f;

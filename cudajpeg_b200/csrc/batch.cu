@@ -2909,6 +2909,7 @@ int cj_reader_decode(JPGReader* jpg, bool stage) {
   a.hrecs = (CJSubRec*)d->hrecs.p;
   a.hckpt = (CJCkpt*)d->hckpt.p;
   a.hmap = (uint8_t*)d->hmap.p;
+  a.wait_limit = d->wait_limit;
   cj_profile_begin(d);
   void* args[] = {&a};
   CJ_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)bt_decode_kernel(BT_DECODE_CTAS_DEFAULT, d->b_nhyp > 1),

@@ -47,6 +47,7 @@ struct CJReaderDevice {
   CJDevBuf raw, data, tile_keep, tile_mark, mpos, mcode, segs, recs, ckpt, snap, wagg, carry, coef,
       pix, params, spec, status, wcoef, bhdr, pscan, hrecs, hckpt, hmap;
   CJHostBuf h_params, h_status, h_pixels, h_file, h_bctl;
+  unsigned wait_limit = 0;  // polls of a wait between CTAs before it is given up (0 = default)
   // per-scan bookkeeping
   int sub_bits = CJ_SUB_BITS_DEFAULT;
   bool sub_bits_auto = true;  // no size set: the decode picks 512 or 1024 bits per image

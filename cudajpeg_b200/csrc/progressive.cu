@@ -96,6 +96,7 @@ struct PGShared {
   int64_t rawpos;
   int bit, blk, eob, err, dc[3];
   int pos, done;  // after the walk: bits and blocks of this chunk
+  int ready;      // the scans before it are past this chunk's blocks
 };
 
 // Symbol entries.  DC (16 bits): bits 0-4 bits consumed, 5-8 magnitude size, 15
@@ -357,7 +358,7 @@ __constant__ uint8_t c_prog_zz[64] = CJ_ZIGZAG_INIT;
 // Waits (one thread) until the scans that `b` follows are past `need` blocks of
 // theirs, which of a dependency marked whole are all.  progress[i]: blocks of scan i
 // done and written, progress[nscans]: chunks done by any CTA.  The wait is given up
-// when no CTA of the launch finished a chunk for PG_WAIT_POLLS polls (seconds; a
+// when no CTA of the launch finished a chunk for `limit` polls (by default seconds; a
 // chunk takes a fraction of a millisecond, and the CTAs are all resident).
 // Polls are relaxed loads, which leave the SM's L1 alone; the fence behind them
 // orders the reads of the coefficients.
@@ -368,7 +369,7 @@ __device__ __forceinline__ int pg_load_relaxed(const int* p) {
   return v;
 }
 __device__ __noinline__ bool pg_await(const CJProgBlock* __restrict__ scans, const CJProgBlock& b, const int* progress,
-                                      int nscans, int need) {
+                                      int nscans, int need, unsigned limit) {
   for (int j = 0; j < b.ndep; j++) {
     const int want = (b.whole >> j) & 1 ? scans[b.dep[j]].blocks : need;
     int seen = -1;
@@ -377,7 +378,7 @@ __device__ __noinline__ bool pg_await(const CJProgBlock* __restrict__ scans, con
       const int any = pg_load_relaxed(&progress[nscans]);
       if (any != seen) polls = 0;
       seen = any;
-      if (++polls > PG_WAIT_POLLS) return false;
+      if (++polls >= limit) return false;
       __nanosleep(256);
     }
   }
@@ -394,7 +395,8 @@ __device__ __forceinline__ void pg_publish(int* progress, int nscans, int scan, 
 __global__ void __launch_bounds__(PG_THREADS) k_prog_scans(const CJProgBlock* __restrict__ scans,
                                                            const CJProgWork* __restrict__ work,
                                                            const uint8_t* __restrict__ file, int16_t* coef,
-                                                           CJStatus* st, int* progress, int nscans) {
+                                                           CJStatus* st, int* progress, int nscans,
+                                                           unsigned wait_limit) {
   extern __shared__ __align__(16) uint8_t pg_smem[];
   PGShared& S = *reinterpret_cast<PGShared*>(pg_smem);
   const CJProgWork wk = work[blockIdx.x];
@@ -431,11 +433,12 @@ __global__ void __launch_bounds__(PG_THREADS) k_prog_scans(const CJProgBlock* __
     const int blk0 = S.blk;
     const int64_t raw0 = S.rawpos;
     if (progress && scans[wk.scan].ndep) {
-      if (tid == 0 && !pg_await(scans, scans[wk.scan], progress, nscans, min(nseq, blk0 + PG_REF_BLOCKS)))
-        S.err = CJ_DEV_TIMEOUT;
+      // (a word of its own: S.err, which the loop's test reads, does not change before the next barrier)
+      if (tid == 0)
+        S.ready = pg_await(scans, scans[wk.scan], progress, nscans, min(nseq, blk0 + PG_REF_BLOCKS), wait_limit);
       __syncthreads();
-      if (S.err) {
-        if (tid == 0) cj_raise(st, 0, S.err);
+      if (!S.ready) {
+        if (tid == 0) cj_raise(st, 0, CJ_DEV_TIMEOUT);
         break;
       }
     }
@@ -815,7 +818,8 @@ int cj_prog_finish(JPGReader* jpg) {
     CJStatus* a_st = (CJStatus*)d->status.p;
     int* a_progress = one_launch ? (int*)(dev + pbytes + wbytes) : nullptr;
     int a_n = n;
-    void* args[] = {&a_scans, &a_work, &a_file, &a_coef, &a_st, &a_progress, &a_n};
+    unsigned a_limit = d->wait_limit ? d->wait_limit : PG_WAIT_POLLS;
+    void* args[] = {&a_scans, &a_work, &a_file, &a_coef, &a_st, &a_progress, &a_n, &a_limit};
     const unsigned grid = (unsigned)((one_launch ? work.size() : from[l + 1]) - from[l]);
     // CTAs that wait for one another are all resident (cooperative); levels need not be
     CJ_CUDA_TRY(one_launch ? cudaLaunchCooperativeKernel((const void*)k_prog_scans, dim3(grid), dim3(PG_THREADS), args,

@@ -35,6 +35,13 @@ void cjReaderSetFlags(JPGReader *r, int flags);
  * MCU-phase hypotheses of a 4:2:0 image) leave the GPU's warps at full speed. */
 int cjReaderSetSubsequenceBits(JPGReader *r, int bits);
 
+/* Bound on each wait between thread blocks of the reader's decode kernels, in
+ * polls (0 = the default, some seconds): the grid barriers of a baseline decode
+ * and a progressive scan's wait for the scans before it.  A wait that runs out
+ * ends the decode with CUDA_KERNEL_LAUNCH_ERROR; the reader stays usable.  A
+ * tiny limit is a way to test that path (see cjBatchSetWaitLimit). */
+int cjReaderSetWaitLimit(JPGReader *r, unsigned polls);
+
 /* Device time of the last decode split by stage, in milliseconds:
  * [0] entropy stages (destuff .. coefficient write), [1] pixel kernel. */
 void cjReaderStageTimes(const JPGReader *r, float *ms);
