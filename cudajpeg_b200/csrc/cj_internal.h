@@ -36,7 +36,8 @@ struct CJReaderDevice {
   CJHostHuff huff[4];
   uint16_t dq16[4][64];   // quantisation tables as parsed (8- or 16-bit), zig-zag order
   bool progressive = false;  // the frame is SOF2
-  int prog_scans = 0;        // progressive scans noted for this frame, and their parameter blocks and byte spans
+  int prog_scans = 0;        // progressive scans of this frame so far
+  int prog_noted = 0;        // of them not yet decoded; their parameter blocks and byte spans
   std::vector<uint8_t> prog_blocks;
   std::vector<int64_t> prog_spans;
   // GPU resources, created on the first scan
@@ -99,8 +100,8 @@ struct CJProgScan {
 };
 // Check a progressive frame's SOS header at jpg->pos (0 or a format.h code).
 int cj_parse_prog_sos(JPGReader* jpg, CJProgScan* s);
-// Progressive frames (progressive.cu): note one SOS's scan; at EOI, decode the
-// scans and queue the pixel stage's parameters.
+// Progressive frames (progressive.cu): note one SOS's scan (and decode what is
+// noted when that is much); at EOI, decode the rest and queue the pixel stage's parameters.
 int cj_prog_scan(JPGReader* jpg);
 int cj_prog_finish(JPGReader* jpg);
 // The scan's entropy decode as one image of the batch decode kernel

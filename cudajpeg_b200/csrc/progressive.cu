@@ -15,10 +15,14 @@
 // these blocks (the refinements of a component run a chunk behind one another).
 // If there are more intervals than CTAs fit on the GPU at once, a launch takes one
 // level of scans, those whose predecessors all ran in the launches before.
+// Noted scans take memory (some 10 KB each, for as little as ten bytes of file), so
+// a frame's are decoded whenever PG_NOTE_SCANS of them, or PG_NOTE_INTERVALS
+// intervals, have been noted; the usual script of ten scans never gets there.
 #include <stdio.h>
 #include <string.h>
 
 #include <algorithm>
+#include <new>
 #include <vector>
 
 #include "../../include/decodeScanGPU.h"
@@ -26,6 +30,8 @@
 #include "cj_internal.h"
 #include "cj_tables.h"
 
+#define PG_NOTE_SCANS 64
+#define PG_NOTE_INTERVALS (1u << 16)
 #define PG_DEPS 16  // scans that one scan follows (64 bands at the most; more take the launch per level)
 
 // A scan's parameter block: the scan, its four Huffman tables, the scans it
@@ -648,11 +654,14 @@ int cj_parse_prog_sos(JPGReader* jpg, CJProgScan* s) {
   return 0;
 }
 
+static int pg_decode_noted(JPGReader* jpg);
+
 // decodeScanGPU for a scan of a progressive frame: check the header, find the
 // scan's restart intervals and its end (the next marker that is not RSTn),
-// and note it for the frame's pixel stage (cj_prog_finish).  The first scan of
-// the frame copies the file to the device and clears the coefficients.
-int cj_prog_scan(JPGReader* jpg) {
+// and note it for the frame's pixel stage (cj_prog_finish), or for an earlier
+// launch when there are many.  The first scan of the frame copies the file to the
+// device and clears the coefficients.
+static int pg_note_scan(JPGReader* jpg) {
   CJReaderDevice* d = jpg->dev;
   // the header first (host only, so a malformed file fails the same way
   // with or without a GPU), then the device
@@ -681,7 +690,8 @@ int cj_prog_scan(JPGReader* jpg) {
   // restart intervals and the end of the scan, from the stuffed bytes
   const unsigned char* base = jpg->buf;
   std::vector<int64_t> spans;
-  spans.reserve(2 * (size_t)S.nint);
+  // (an interval costs two bytes of file at the least, whatever the header says)
+  spans.reserve(std::min(2 * (size_t)S.nint, (size_t)(jpg->end - jpg->pos) + 2));
   spans.push_back((int64_t)(jpg->pos - base));
   unsigned char* q = jpg->pos;
   const unsigned char* lim = jpg->end;  // the EOI marker lies past it
@@ -724,23 +734,26 @@ int cj_prog_scan(JPGReader* jpg) {
     d->param_bytes = 0;
     d->nkev = 0;
   }
-  if (!d->prog_scans) {
+  if (!d->prog_scans) {  // (a file that ended in an error may have left some)
     d->prog_blocks.clear();
     d->prog_spans.clear();
+    d->prog_noted = 0;
   }
   const uint8_t* pb = reinterpret_cast<const uint8_t*>(&blk);
   d->prog_blocks.insert(d->prog_blocks.end(), pb, pb + sizeof(blk));
   d->prog_spans.insert(d->prog_spans.end(), spans.begin(), spans.end());
   d->prog_scans++;
+  d->prog_noted++;
   jpg->pos = q;  // the marker that ends the scan
+  if (d->prog_noted >= PG_NOTE_SCANS || d->prog_spans.size() >= 2 * (size_t)PG_NOTE_INTERVALS) return pg_decode_noted(jpg);
   return 0;
 }
 
-// Decode the noted scans and queue the pixel stage's parameters (geometry and the
-// quantisation tables; the Huffman tables are not needed after the scans).
-int cj_prog_finish(JPGReader* jpg) {
+// Queue the decode of the noted scans, behind that of the scans before them.
+static int pg_decode_noted(JPGReader* jpg) {
   CJReaderDevice* d = jpg->dev;
-  const int n = d->prog_scans;
+  const int n = d->prog_noted;
+  if (!n) return 0;
   CJProgBlock* blocks = reinterpret_cast<CJProgBlock*>(d->prog_blocks.data());
   // a scan follows the last ones before it that touch a coefficient of its; its level
   // is one more than theirs
@@ -808,7 +821,7 @@ int cj_prog_finish(JPGReader* jpg) {
   CJ_CUDA_TRY(cudaMemcpyAsync(d->pscan.p, d->prog_blocks.data(), bytes, cudaMemcpyHostToDevice, d->stream),
               CUDA_MEM_ERROR);
   d->param_bytes += bytes;
-  cj_profile_begin(d);
+  if (!d->nkev) cj_profile_begin(d);
   uint8_t* dev = (uint8_t*)d->pscan.p;
   for (int l = 0; l < (one_launch ? 1 : levels); l++) {
     const CJProgBlock* a_scans = (const CJProgBlock*)dev;
@@ -829,10 +842,39 @@ int cj_prog_finish(JPGReader* jpg) {
                 CUDA_KERNEL_LAUNCH_ERROR);
     cj_after_launch(d, CJ_K_PROG_SCAN);
   }
+  d->prog_blocks.clear();
+  d->prog_spans.clear();
+  d->prog_noted = 0;
+  return 0;
+}
+
+// Decode the scans still noted and queue the pixel stage's parameters (geometry and
+// the quantisation tables; the Huffman tables are not needed after the scans).
+static int pg_finish(JPGReader* jpg) {
+  CJReaderDevice* d = jpg->dev;
+  const int err = pg_decode_noted(jpg);
+  if (err) return err;
   CJScanParams* hp = (CJScanParams*)d->h_params.p;
   cj_fill_params(jpg, hp);
   CJ_CUDA_TRY(cudaMemcpyAsync(d->params.p, hp, sizeof(CJScanParams), cudaMemcpyHostToDevice, d->stream),
               CUDA_MEM_ERROR);
   CJ_CUDA_TRY(cudaEventRecord(d->ev_scan, d->stream), CUDA_KERNEL_LAUNCH_ERROR);
   return 0;
+}
+
+// (no exception leaves the library: its callers are C)
+int cj_prog_scan(JPGReader* jpg) {
+  try {
+    return pg_note_scan(jpg);
+  } catch (const std::bad_alloc&) {
+    return OOM_ERROR;
+  }
+}
+
+int cj_prog_finish(JPGReader* jpg) {
+  try {
+    return pg_finish(jpg);
+  } catch (const std::bad_alloc&) {
+    return OOM_ERROR;
+  }
 }
