@@ -103,6 +103,7 @@ struct PGShared {
   int bit, blk, eob, err, dc[3];
   int pos, done;  // after the walk: bits and blocks of this chunk
   int ready;      // the scans before it are past this chunk's blocks
+  int range;      // its first block with a value outside int16 (INT_MAX: none)
 };
 
 // Symbol entries.  DC (16 bits): bits 0-4 bits consumed, 5-8 magnitude size, 15
@@ -429,6 +430,7 @@ __global__ void __launch_bounds__(PG_THREADS) k_prog_scans(const CJProgBlock* __
       }
     S.rawpos = wk.begin;
     S.bit = S.blk = S.eob = S.err = 0;
+    S.range = INT_MAX;
     S.dc[0] = S.dc[1] = S.dc[2] = 0;
   }
   const int u0 = s.ri ? wk.iv * s.ri : 0;
@@ -539,7 +541,7 @@ __global__ void __launch_bounds__(PG_THREADS) k_prog_scans(const CJProgBlock* __
         for (int b = tid; b < done; b += PG_THREADS) {
           const int64_t at = pg_block(s, S, u0, bps, blk0 + b);
           const int64_t v = (int64_t)(int)S.ev0[b] * (1 << al);
-          if (v < -32768 || v > 32767) cj_raise(st, at, CJ_DEV_DC_RANGE);
+          if (v < -32768 || v > 32767) atomicMin(&S.range, b);
           else coef[at * 64] = (int16_t)v;
         }
       } else if (!refine) {
@@ -547,14 +549,13 @@ __global__ void __launch_bounds__(PG_THREADS) k_prog_scans(const CJProgBlock* __
         for (int b = tid; b < last; b += PG_THREADS) {
           const uint32_t v0 = S.ev0[b];
           if (!(v0 >> 16)) continue;
-          const int64_t at = pg_block(s, S, u0, bps, blk0 + b);
-          int16_t* blk = coef + at * 64;
+          int16_t* blk = coef + pg_block(s, S, u0, bps, blk0 + b) * 64;
           for (uint32_t i = 0; i < (v0 >> 16); i++) {
             const uint32_t ev = S.evt[(v0 & 0xFFFFu) + i], e = S.sym[(ev & 0xFFFFu) >> 2], size = (e >> 16) & 255;
             if (!size) continue;  // ZRL
             const int v = cj_extend(pg_bits(S, (((ev & 0xFFFFu) + (e & 255)) >> 2) - size, size), size) * (1 << al);
             if (v < -32768 || v > 32767) {
-              cj_raise(st, at, CJ_DEV_DC_RANGE);
+              atomicMin(&S.range, b);
               break;
             }
             blk[S.zz[ev >> 16]] = (int16_t)v;
@@ -590,7 +591,9 @@ __global__ void __launch_bounds__(PG_THREADS) k_prog_scans(const CJProgBlock* __
       __syncthreads();
     }
     if (tid == 0) {
-      if (S.err) cj_raise(st, pg_block(s, S, u0, bps, blk0 + S.done), S.err);
+      // the interval ends at its first error; a value out of range precedes the symbol that ends the walk
+      if (S.range < INT_MAX) S.err = CJ_DEV_DC_RANGE;
+      if (S.err) cj_raise(st, pg_block(s, S, u0, bps, blk0 + min(S.done, S.range)), S.err);
       S.blk = blk0 + S.done;
       if (progress) pg_publish(progress, nscans, wk.scan, S.done);
       S.rawpos = raw0 + min((int)S.raw[min(S.pos >> 3, PG_BYTES)], (int)min((int64_t)65535, wk.end - raw0));
