@@ -686,6 +686,14 @@ static int pg_note_scan(JPGReader* jpg) {
   S.nunits = S.ns > 1 ? hp->mcux * hp->mcuy : S.bw * S.bh;
   S.ri = jpg->restart_interval;
   S.nint = S.ri ? (S.nunits + S.ri - 1) / S.ri : 1;
+  // a frame header behind the first scan does not take later ones outside the coefficient
+  // buffer, which the first scan's geometry sized
+  int64_t top = 0;  // the last block of the scan
+  for (int j = 0; j < S.ns; j++) {
+    const int64_t mcu = S.ns > 1 ? S.nunits - 1 : (int64_t)((S.bh - 1) / S.sy[0]) * S.mcux + (S.bw - 1) / S.sx[0];
+    top = std::max(top, mcu * S.bpm + S.first[j] + S.sx[j] * S.sy[j] - 1);
+  }
+  if (top >= hp->total_blocks) return SYNTAX_ERROR;
   for (int slot = 0; slot < 4; slot++) {
     if (jpg->huff_defined & (1 << slot)) cj_build_huff(d->huff[slot].counts, d->huff[slot].symbols, &blk.huff[slot]);
     else memset(&blk.huff[slot], 0, sizeof(CJHuff));
@@ -859,6 +867,9 @@ static int pg_finish(JPGReader* jpg) {
   if (err) return err;
   CJScanParams* hp = (CJScanParams*)d->h_params.p;
   cj_fill_params(jpg, hp);
+  // (the pixel stage reads as many blocks as the last frame header says)
+  if (hp->total_blocks > d->total_blocks) return SYNTAX_ERROR;
+  d->total_blocks = hp->total_blocks;
   CJ_CUDA_TRY(cudaMemcpyAsync(d->params.p, hp, sizeof(CJScanParams), cudaMemcpyHostToDevice, d->stream),
               CUDA_MEM_ERROR);
   CJ_CUDA_TRY(cudaEventRecord(d->ev_scan, d->stream), CUDA_KERNEL_LAUNCH_ERROR);

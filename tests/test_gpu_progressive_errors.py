@@ -62,3 +62,28 @@ def test_first_error_of_an_interval(cj, oracle_mod, name):
         assert r.open_bytes(data, check=False) == want
         r.open_bytes(good)
         assert np.array_equal(r.pixels(), oracle_mod.decode(good).pixels)
+
+
+def sof(w, h):
+    return seg(0xC2, struct.pack(">BHHB", 8, h, w, 1) + bytes([1, 0x11, 0]))
+
+
+DC = seg(0xDA, bytes([1, 1, 0, 0, 0, 0]))
+
+
+@pytest.mark.parametrize("first,second,scan,ok", [((8, 8), (4096, 4096), True, False), ((8, 8), (4096, 4096), False, False),
+                                                  ((64, 64), (8, 8), True, True), ((64, 64), (64, 64), True, True),
+                                                  ((256, 8), (8, 256), True, False), ((256, 8), (8, 256), False, True)])
+def test_a_second_frame_header_stays_inside_the_coefficients(cj, first, second, scan, ok):
+    """The first scan sizes the coefficient buffer and its rows of blocks; later scans that do not fit it, and
+    a larger last frame, are refused."""
+    head = b"\xff\xd8" + seg(0xDB, b"\0" + b"\x01" * 64) + seg(0xC4, bytes([0x00, 1, 1] + [0] * 14 + [0, 11]))
+    zeros = bytes(-(-(first[0] // 8) * (first[1] // 8) // 8))
+    data = head + sof(*first) + DC + zeros + sof(*second) + ((DC + bytes(32768)) if scan else seg(0xFE, b"comment")) + b"\xff\xd9"
+    with cj.Reader(host_coefficients=True) as r:
+        assert r.open_bytes(data, check=False) == (0 if ok else cj.SYNTAX_ERROR)
+        if ok:
+            assert (r.pixels() == 128).all() and r.pixels().shape[:2] == (second[1], second[0])
+            assert not r.coefficients()[0].any()
+        good = W.small_case(2, 64, 48, "420").data
+        r.open_bytes(good)
