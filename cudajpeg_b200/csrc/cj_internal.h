@@ -42,7 +42,7 @@ struct CJReaderDevice {
   std::vector<int64_t> prog_spans;
   // GPU resources, created on the first scan
   bool gpu_ready = false;
-  int device = -1;
+  int device = -1, sms = 0;  // and its SMs
   cudaStream_t stream = nullptr;
   cudaEvent_t ev_begin = nullptr, ev_scan = nullptr, ev_end = nullptr;
   CJDevBuf raw, data, tile_keep, tile_mark, mpos, mcode, segs, recs, ckpt, snap, wagg, carry, coef,

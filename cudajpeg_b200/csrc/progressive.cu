@@ -9,7 +9,8 @@
 // (interleaved or not), DC refinement (one bit per block), AC first with
 // end-of-band runs, and AC refinement with correction bits.
 //
-// One CTA per restart interval of a scan.  A scan that touches coefficients of
+// One CTA per restart interval of a scan (a thread per interval, and a launch per scan,
+// where the intervals are many and short).  A scan that touches coefficients of
 // scans before it follows them: all scans run in one launch, and a chunk of
 // blocks is decoded once the scans it follows have published that they are past
 // these blocks (the refinements of a component run a chunk behind one another).
@@ -34,11 +35,15 @@
 #define PG_NOTE_INTERVALS (1u << 16)
 #define PG_DEPS 16  // scans that one scan follows (64 bands at the most; more take the launch per level)
 
-// A scan's parameter block: the scan, its four Huffman tables, the scans it
-// follows in the same launch (block by block, or after their last: whole).
-struct CJProgBlock {
+// A scan and its four Huffman tables.
+struct CJProgTables {
   CJProgScan s;
   CJHuff huff[4];
+};
+
+// A scan's parameter block: with them the scans it follows in the same launch (block
+// by block, or after their last: whole).
+struct CJProgBlock : CJProgTables {
   int32_t ndep, dep[PG_DEPS];
   uint32_t whole;  // bit per dependency
   int32_t blocks;  // of the scan in all
@@ -604,7 +609,198 @@ __global__ void __launch_bounds__(PG_THREADS) k_prog_scans(const CJProgBlock* __
   if (progress && tid == 0) pg_publish(progress, nscans, wk.scan, nseq - S.blk);  // an error's blocks: none waits for them
 }
 
+// ---- short intervals: a thread each.  A CTA of k_prog_scans takes 8 us for an
+// interval however short, and one at a time fits an SM; thousands of intervals of a
+// few bytes are done sooner by a thread each, decoding symbol by symbol from global
+// memory (pg_thin).
+
+// MSB-first bits of one interval's stuffed bytes: FF 00 reads as FF; bytes
+// past the end read as 0.
+struct PGBits {
+  const uint8_t* p;
+  const uint8_t* e;
+  uint64_t acc;
+  int n;
+  __device__ __forceinline__ void fill() {
+    while (n <= 56) {
+      uint32_t b = 0;
+      if (p < e) {
+        b = *p++;
+        if (b == 0xFF && p < e && *p == 0x00) p++;
+      }
+      acc |= (uint64_t)b << (56 - n);
+      n += 8;
+    }
+  }
+  __device__ __forceinline__ uint32_t peek16() {
+    fill();
+    return (uint32_t)(acc >> 48);
+  }
+  __device__ __forceinline__ uint32_t bits(int k) {  // k <= 16
+    if (!k) return 0;
+    fill();
+    const uint32_t v = (uint32_t)(acc >> (64 - k));
+    acc <<= k;
+    n -= k;
+    return v;
+  }
+  // Huffman symbol, or -1 when no code matches
+  __device__ __forceinline__ int huff(const CJHuff& t) {
+    const uint32_t e = cj_huff_decode(t, peek16());
+    if (!e) return -1;
+    acc <<= (e >> 8);
+    n -= (int)(e >> 8);
+    return (int)(e & 255);
+  }
+};
+
+// A value into an int16 coefficient; false when it does not fit.
+__device__ __forceinline__ bool pg_store(int16_t* c, int v) {
+  if (v < -32768 || v > 32767) return false;
+  *c = (int16_t)v;
+  return true;
+}
+
+// One block of a scan (T.81 G.1.2): returns 0 or a CJ_DEV_* code.
+__device__ int pg_serial_block(const CJProgTables& P, int j, PGBits& br, int16_t* blk, int* dc_pred, int* eobrun,
+                               const uint8_t* zz) {
+  const CJProgScan& S = P.s;
+  if (S.ss == 0) {
+    if (!S.ah) {
+      const int s = br.huff(P.huff[S.dc_slot[j]]);
+      if (s < 0) return CJ_DEV_BAD_CODE;
+      if (s > 11) return CJ_DEV_BAD_AC;
+      dc_pred[j] += s ? cj_extend(br.bits(s), s) : 0;
+      if (!pg_store(&blk[0], dc_pred[j] * (1 << S.al))) return CJ_DEV_DC_RANGE;
+    } else if (br.bits(1)) {
+      blk[0] = (int16_t)(blk[0] | (1 << S.al));
+    }
+    return 0;
+  }
+  const CJHuff& t = P.huff[S.ac_slot[j]];
+  int k = S.ss;
+  if (!S.ah) {
+    if (*eobrun > 0) {
+      (*eobrun)--;
+      return 0;
+    }
+    while (k <= S.se) {
+      const int rs = br.huff(t);
+      if (rs < 0) return CJ_DEV_BAD_CODE;
+      const int r = rs >> 4, s = rs & 15;
+      if (s) {
+        k += r;
+        if (k > S.se) return CJ_DEV_BAD_AC;
+        if (!pg_store(&blk[zz[k]], cj_extend(br.bits(s), s) * (1 << S.al))) return CJ_DEV_DC_RANGE;
+        k++;
+      } else if (r == 15) {
+        k += 16;
+      } else {
+        *eobrun = (1 << r) - 1;
+        if (r) *eobrun += (int)br.bits(r);
+        break;
+      }
+    }
+    return 0;
+  }
+  const int p1 = 1 << S.al, m1 = -(1 << S.al);
+  if (*eobrun == 0) {
+    for (; k <= S.se; k++) {
+      const int rs = br.huff(t);
+      if (rs < 0) return CJ_DEV_BAD_CODE;
+      int r = rs >> 4, val = 0;
+      const int s = rs & 15;
+      if (s) {
+        if (s != 1) return CJ_DEV_BAD_AC;
+        val = br.bits(1) ? p1 : m1;
+      } else if (r != 15) {
+        *eobrun = 1 << r;
+        if (r) *eobrun += (int)br.bits(r);
+        break;
+      }
+      // pass r zero-history coefficients, refining the nonzero ones met
+      while (k <= S.se) {
+        int16_t* c = &blk[zz[k]];
+        if (*c) {
+          if (br.bits(1) && !(*c & p1)) *c = (int16_t)(*c + (*c >= 0 ? p1 : m1));
+        } else if (--r < 0) {
+          break;
+        }
+        k++;
+      }
+      if (val) {
+        if (k > S.se) return CJ_DEV_BAD_AC;
+        blk[zz[k]] = (int16_t)val;
+      }
+    }
+  }
+  if (*eobrun > 0) {
+    // inside an end-of-band run: the correction bits of the nonzero coefficients
+    for (; k <= S.se; k++) {
+      int16_t* c = &blk[zz[k]];
+      if (*c && br.bits(1) && !(*c & p1)) *c = (int16_t)(*c + (*c >= 0 ? p1 : m1));
+    }
+    (*eobrun)--;
+  }
+  return 0;
+}
+
+#define PG_THIN_THREADS 128
+__global__ void __launch_bounds__(PG_THIN_THREADS) k_prog_thin(const CJProgTables* __restrict__ scan,
+                                                              const int64_t* __restrict__ spans,
+                                                              const uint8_t* __restrict__ file,
+                                                              int16_t* __restrict__ coef, CJStatus* st) {
+  __shared__ CJProgTables P;
+  __shared__ uint8_t zz[64];
+  const int iv = blockIdx.x * PG_THIN_THREADS + threadIdx.x;
+#pragma unroll 10
+  for (int k = threadIdx.x; k < (int)(sizeof(P) / 4); k += PG_THIN_THREADS)
+    reinterpret_cast<uint32_t*>(&P)[k] = reinterpret_cast<const uint32_t*>(scan)[k];
+  if (threadIdx.x < 64) zz[threadIdx.x] = c_prog_zz[threadIdx.x];
+  __syncthreads();
+  const CJProgScan& s = P.s;
+  if (iv >= s.nint) return;
+  PGBits br = {file + spans[2 * iv], file + spans[2 * iv + 1], 0, 0};
+  int dc_pred[3] = {0, 0, 0}, eobrun = 0;
+  const int u0 = s.ri ? iv * s.ri : 0;
+  const int u1 = s.ri ? min(s.nunits, u0 + s.ri) : s.nunits;
+  for (int u = u0; u < u1; u++) {
+    int64_t at = (int64_t)u * s.bpm;
+    if (s.ns == 1) {  // one component: its blocks in raster order
+      const int bx = u % s.bw, by = u / s.bw;
+      at = ((int64_t)(by / s.sy[0]) * s.mcux + bx / s.sx[0]) * s.bpm + (by % s.sy[0]) * s.sx[0] + bx % s.sx[0];
+    }
+    for (int j = 0; j < s.ns; j++)
+      for (int w = 0; w < (s.ns > 1 ? s.sx[j] * s.sy[j] : 1); w++) {
+        const int64_t blk = at + s.first[j] + w;
+        const int e = pg_serial_block(P, j, br, coef + blk * 64, dc_pred, &eobrun, zz);
+        if (e) {
+          cj_raise(st, blk, e);
+          return;
+        }
+      }
+  }
+}
+
 // ---------------------------------------------------------------- host side
+
+// Whether a scan's intervals are decoded by a thread each: the estimated times of both
+// ways, in us.  A thread's chain is its interval's bytes and, in an AC refinement,
+// the loads of every coefficient of the band in its blocks (21 us a block of the whole
+// band); the CTAs run in waves of one per SM, 8.3 us each.  Fitted to 4:2:0 files of
+// 128x96 to 2048x1536 samples and qualities 60 to 95; device time of all ten scans by
+// CTAs / by threads at 1024x768, q 80: an interval per MCU 4.0 / 0.6 ms, per 4 MCUs
+// 1.1 / 0.75, per 8 0.65 / 1.3, per 32 0.29 / 4.9; 2048x1536: per MCU 13.0 / 1.9, per
+// 16 1.4 / 2.6.  `change`: what a change of way costs, where the scan before went the
+// other (a launch of its own for what is noted, which then overlaps with less).
+#define PG_CHANGE_US 20.0
+static bool pg_thin(const CJProgScan& s, int64_t longest, int64_t bytes, int sms, double change) {
+  double thread = 15.0 + 0.0066 * s.nint;
+  if (!s.ah) thread += 1.5 * longest;
+  else if (s.ss) thread += 4.0 * longest + 21.0 / 63 * (s.se - s.ss + 1) * (s.ri ? s.ri : s.nunits);
+  else thread += 4.0 * longest;  // (eight blocks a byte)
+  return thread + change < 8.0 + (8.3 * s.nint + 0.15 * bytes) / sms;
+}
 
 // Validate the SOS header of a progressive frame (T.81 B.2.3, G.1.1.1.1) at
 // jpg->pos and fill `s` with the scan's components and band; on success
@@ -659,6 +855,26 @@ int cj_parse_prog_sos(JPGReader* jpg, CJProgScan* s) {
 
 static int pg_decode_noted(JPGReader* jpg);
 
+// Queue the decode of one scan by a thread per interval.
+static int pg_decode_thin(CJReaderDevice* d, const CJProgBlock& blk, const std::vector<int64_t>& spans) {
+  // the block and the spans, in one stream-ordered copy: the next scan's copy into the
+  // same buffer waits for this scan's kernel
+  const size_t pbytes = (sizeof(CJProgTables) + 15) & ~(size_t)15, sbytes = spans.size() * sizeof(int64_t);
+  std::vector<uint8_t> host(pbytes + sbytes);
+  memcpy(host.data(), static_cast<const CJProgTables*>(&blk), sizeof(CJProgTables));
+  memcpy(host.data() + pbytes, spans.data(), sbytes);
+  if (cj_dev_ensure(d->pscan, host.size())) return CUDA_MEM_ERROR;
+  CJ_CUDA_TRY(cudaMemcpyAsync(d->pscan.p, host.data(), host.size(), cudaMemcpyHostToDevice, d->stream), CUDA_MEM_ERROR);
+  d->param_bytes += host.size();
+  if (!d->nkev) cj_profile_begin(d);
+  k_prog_thin<<<(blk.s.nint + PG_THIN_THREADS - 1) / PG_THIN_THREADS, PG_THIN_THREADS, 0, d->stream>>>(
+      (const CJProgTables*)d->pscan.p, (const int64_t*)((const uint8_t*)d->pscan.p + pbytes), (const uint8_t*)d->raw.p,
+      (int16_t*)d->coef.p, (CJStatus*)d->status.p);
+  cj_after_launch(d, CJ_K_PROG_SCAN);
+  CJ_CUDA_TRY(cudaGetLastError(), CUDA_KERNEL_LAUNCH_ERROR);
+  return 0;
+}
+
 // decodeScanGPU for a scan of a progressive frame: check the header, find the
 // scan's restart intervals and its end (the next marker that is not RSTn),
 // and note it for the frame's pixel stage (cj_prog_finish), or for an earlier
@@ -673,7 +889,6 @@ static int pg_note_scan(JPGReader* jpg) {
     k += jpg->channels[c].samples_x * jpg->channels[c].samples_y;
   }
   CJProgBlock blk;
-  memset(&blk, 0, sizeof(blk));
   int err = cj_parse_prog_sos(jpg, &blk.s);
   if (err) return err;
   err = cj_gpu_init(jpg);
@@ -707,6 +922,7 @@ static int pg_note_scan(JPGReader* jpg) {
   unsigned char* q = jpg->pos;
   const unsigned char* lim = jpg->end;  // the EOI marker lies past it
   int expect = 0;
+  int64_t longest = 0;
   for (;;) {
     q = (unsigned char*)memchr(q, 0xFF, (size_t)(lim - q));
     if (!q || q + 1 >= lim + 2) {
@@ -721,6 +937,7 @@ static int pg_note_scan(JPGReader* jpg) {
     if ((m & 0xF8) == 0xD0) {  // RSTn: ends one interval, starts the next
       if ((m & 7) != expect || (int)(spans.size() / 2) + 1 >= S.nint) return SYNTAX_ERROR;
       expect = (expect + 1) & 7;
+      longest = std::max(longest, (int64_t)(q - base) - spans.back());
       spans.push_back((int64_t)(q - base));
       spans.push_back((int64_t)(q + 2 - base));
       q += 2;
@@ -728,6 +945,7 @@ static int pg_note_scan(JPGReader* jpg) {
     }
     break;  // the next marker segment (or EOI)
   }
+  longest = std::max(longest, (int64_t)(q - base) - spans.back());
   spans.push_back((int64_t)(q - base));
   if ((int)(spans.size() / 2) != S.nint) return SYNTAX_ERROR;
   const size_t file_bytes = (size_t)(jpg->end + 2 - base);
@@ -749,6 +967,15 @@ static int pg_note_scan(JPGReader* jpg) {
     d->prog_blocks.clear();
     d->prog_spans.clear();
     d->prog_noted = 0;
+  }
+  const double change = d->prog_noted ? PG_CHANGE_US : (d->prog_scans ? -PG_CHANGE_US : 0.0);
+  if (pg_thin(S, longest, spans.back() - spans.front(), d->sms, change)) {  // decoded at once, behind what is noted
+    err = pg_decode_noted(jpg);
+    if (!err) err = pg_decode_thin(d, blk, spans);
+    if (err) return err;
+    d->prog_scans++;
+    jpg->pos = q;
+    return 0;
   }
   const uint8_t* pb = reinterpret_cast<const uint8_t*>(&blk);
   d->prog_blocks.insert(d->prog_blocks.end(), pb, pb + sizeof(blk));
@@ -817,11 +1044,10 @@ static int pg_decode_noted(JPGReader* jpg) {
   }
   CJ_CUDA_TRY(cudaFuncSetAttribute(k_prog_scans, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PGShared)),
               CUDA_KERNEL_LAUNCH_ERROR);
-  int sms = 0, per = 0;
-  CJ_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d->device), CUDA_MEM_ERROR);
+  int per = 0;
   CJ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_prog_scans, PG_THREADS, sizeof(PGShared)),
               CUDA_KERNEL_LAUNCH_ERROR);
-  one_launch = one_launch && levels > 1 && work.size() <= (size_t)sms * per;
+  one_launch = one_launch && levels > 1 && work.size() <= (size_t)d->sms * per;
   // copied together: the scans' blocks, the work items, the progress counters' zeros
   const size_t pbytes = ((size_t)n * sizeof(CJProgBlock) + 15) & ~(size_t)15;
   const size_t wbytes = work.size() * sizeof(CJProgWork), bytes = pbytes + wbytes + (n + 1) * sizeof(int);

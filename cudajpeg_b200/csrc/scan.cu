@@ -69,6 +69,7 @@ int cj_gpu_init(JPGReader* jpg) {
     return CUDA_MEM_ERROR;
   }
   CJ_CUDA_TRY(cudaGetDevice(&d->device), CUDA_MEM_ERROR);
+  CJ_CUDA_TRY(cudaDeviceGetAttribute(&d->sms, cudaDevAttrMultiProcessorCount, d->device), CUDA_MEM_ERROR);
   CJ_CUDA_TRY(cudaStreamCreateWithFlags(&d->stream, cudaStreamNonBlocking), CUDA_MEM_ERROR);
   CJ_CUDA_TRY(cudaEventCreate(&d->ev_begin), CUDA_MEM_ERROR);
   CJ_CUDA_TRY(cudaEventCreate(&d->ev_scan), CUDA_MEM_ERROR);
