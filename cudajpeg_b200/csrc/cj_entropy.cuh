@@ -713,7 +713,9 @@ static __device__ __noinline__ void cj_write_warp(CJWriteJob* job, bool active) 
     if (p >= x.stop || (!x.last && p >= x.end)) return;
     if (b >= bend) {
       if (!x.last) cj_raise_dec(x.st, x.base + b, CJ_DEV_EXTRA);
-      else if (x.marker ? ((p + 7) >> 3) != x.end_byte : x.end_byte > ((p + 7) >> 3) + 2)
+      // (where the last block ends; a unit that starts behind it starts where the speculative decode took
+      // the padding bits for a block, and that may reach past the segment)
+      else if (b == bend && (x.marker ? ((p + 7) >> 3) != x.end_byte : x.end_byte > ((p + 7) >> 3) + 2))
         cj_raise_dec(x.st, x.base + b, CJ_DEV_TRAILING);
     } else {
       cj_raise_dec(x.st, x.base + b, CJ_DEV_OVERRUN);
