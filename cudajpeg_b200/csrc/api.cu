@@ -113,17 +113,20 @@ int cjDebugHuffDecode(const unsigned char counts[16], const unsigned char* symbo
 
 int cjDebugStepTable(const unsigned char counts[16], const unsigned char* symbols, int ac,
                      unsigned short* out) {
-  CJScanParams* sp = new (std::nothrow) CJScanParams;
-  if (!sp || !out) {
-    delete sp;
+  CJSteps* T = new (std::nothrow) CJSteps;
+  if (!T || !out) {
+    delete T;
     return PROGRAMMER_ERROR;
   }
-  memset(sp, 0, sizeof(*sp));
   const int slot = ac ? 2 : 0;
-  cj_build_huff(counts, symbols, &sp->huff[slot]);
-  cj_build_steps(sp->huff[slot], counts, true, slot, &sp->steps);
-  for (uint32_t w = 0; w < 65536; w++) out[w] = (unsigned short)cj_step(*sp, slot, w << 16);
-  delete sp;
+  CJHuff t;
+  cj_build_huff(counts, symbols, &t);
+  cj_build_steps(t, counts, true, slot, T);
+  for (uint32_t w = 0; w < 65536; w++) {
+    out[w] = (unsigned short)cj_step(*T, t, slot, w << 16);
+    if (out[w] != cj_step_canonical(t, slot, w << 16)) out[w] = 0xFFFF;  // (the two forms agree)
+  }
+  delete T;
   return 0;
 }
 

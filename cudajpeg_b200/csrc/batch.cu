@@ -320,7 +320,7 @@ __device__ __forceinline__ bool bt_settle_map(const CJBatchArgs& a, CJSpecJob& x
     if (__any_sync(CJ_FULL, redo)) {
       if (!filled && ln.active && !ln.head) cj_hyp_fill(hpp, hck, nhi + 1);
       filled = true;
-      cj_spec_warp<true>(&x, redo, want);
+      cj_spec_run<true, false>(x, redo, want);
       dirty = dirty || redo;
     }
   }
@@ -357,15 +357,23 @@ __device__ __forceinline__ void bt_rank_end(CJBatchCtl* ctl, BTRank& k) {
 // first, then thread 0 takes one and the CTA shares it.  The leading barrier
 // also ends the previous group: every warp is done with it and with the tables
 // staged for it.
-__device__ __forceinline__ int bt_next_group(int* counter, int* s_slot, int rank, bool& first) {
+__device__ __forceinline__ int bt_next_group(int* counter, int* s_slot, int rank, bool& first, int per = BT_WARPS) {
   __syncthreads();
   if (first) {
     first = false;
-    return rank * BT_WARPS;
+    return rank * per;
   }
-  if (threadIdx.x == 0) *s_slot = atomicAdd(counter, BT_WARPS) + (int)gridDim.x * BT_WARPS;
+  if (threadIdx.x == 0) *s_slot = atomicAdd(counter, per) + (int)gridDim.x * per;
   __syncthreads();
   return *s_slot;
+}
+
+// Items per group: fewer than the CTA's warps where the items would not give every
+// CTA a full group.
+__device__ __forceinline__ int bt_group(int items) {
+  int g = BT_WARPS;
+  while (g > 1 && items <= (int)gridDim.x * (g / 2)) g /= 2;
+  return g;
 }
 
 // Largest i with key(i) <= v over a sorted int32 field of the descriptors.
@@ -434,7 +442,7 @@ __device__ __forceinline__ BTItem bt_item(const CJBatchArgs& a, int w, int h) {
 struct BTTabs {
   int want[BT_WARPS], id[2];
 };
-template <int SLOTS, int OFF, class F>
+template <int SLOTS, int OFF, bool GLOBAL, class F>
 __device__ __forceinline__ void bt_with_tables(const CJBatchArgs& a, BTTabs& s, uint8_t* slots, int tab, F f) {
   constexpr int BYTES = (int)sizeof(CJSpecTab) - OFF;
   if ((threadIdx.x & 31) == 0) s.want[threadIdx.x >> 5] = tab;
@@ -468,7 +476,11 @@ __device__ __forceinline__ void bt_with_tables(const CJBatchArgs& a, BTTabs& s, 
       }
       __syncthreads();
     }
-    if (tab >= 0 && (tab == ta || tab == tb)) f(bt_smem_addr(slots + (tab == ta ? sa : sb) * BYTES) - (uint32_t)OFF);
+    const bool staged = tab == ta || tab == tb;
+    if (tab >= 0 && (staged || GLOBAL))
+      f(staged ? bt_smem_addr(slots + (tab == ta ? sa : sb) * BYTES) - (uint32_t)OFF : 0u,
+        staged ? nullptr : reinterpret_cast<const uint8_t*>(a.spec + tab));
+    if (GLOBAL) break;
     todo &= ~mask;
     if (todo) __syncthreads();  // before a slot is overwritten
   }
@@ -491,72 +503,79 @@ __device__ __forceinline__ bool bt_same_tables(const CJImageHeader& x, const CJI
 static_assert(BT_THREADS == 256, "one thread per symbol word");
 static_assert(offsetof(CJImageHeader, symbols) % 4 == 0, "symbol words");
 
-// Phase 0: one CTA builds one Huffman table slot of one image on the device --
-// the canonical table, its decode steps and its CJSpecTab entries -- in
-// shared memory, where every entry's searches are short, and copies them out.
+// Phase 0: one CTA builds `ns` Huffman table slots of one image from s0 on -- the
+// canonical tables and their CJSpecTab entries -- in shared memory, where every
+// entry's searches are short, and copies them out.  Slots no component uses stay as
+// they are.
 struct BTBuild {
   CJHuff t;
   uint16_t pri[1 << CJ_FAST_BITS];
   uint8_t counts[16];
   int pmin, pmax;
 };
-static_assert(sizeof(BTBuild) <= BT_DECODE_SMEM && sizeof(CJHuff) % 4 == 0, "table build space");
-__device__ void bt_build_slot(const CJImageHeader& h, CJScanParams& p, CJSpecTab& tb, int slot, BTBuild& s) {
-  const bool defined = (h.huff_mask >> slot) & 1, ac = slot >= 2;
-  if (threadIdx.x < 16) s.counts[threadIdx.x] = h.counts[slot][threadIdx.x];
-  s.t.vals[threadIdx.x] = h.symbols[slot][threadIdx.x];
+static_assert(4 * sizeof(BTBuild) <= BT_DECODE_SMEM && sizeof(CJHuff) % 4 == 0, "table build space");
+__device__ void bt_build_slots(const CJImageHeader& h, CJScanParams& p, CJSpecTab& tb, int s0, int ns, BTBuild* s) {
+  const int tid = threadIdx.x;
+  const uint32_t mask = h.huff_mask;
+  for (int q = 0; q < ns; q++) s[q].t.vals[tid] = h.symbols[s0 + q][tid];
+  if (tid < 16 * ns) s[tid >> 4].counts[tid & 15] = h.counts[s0 + (tid >> 4)][tid & 15];
   __syncthreads();
-  if (threadIdx.x == 0) {  // cj_build_huff's canonical arrays
+  if (tid < ns) {  // cj_build_huff's canonical arrays
+    CJHuff& t = s[tid].t;
     int code = 0, k = 0;
-    s.t.maxcode[0] = -1;
-    s.t.valoff[0] = 0;
+    t.maxcode[0] = -1;
+    t.valoff[0] = 0;
     for (int l = 1; l <= 16; l++) {
-      const int n = s.counts[l - 1];
-      s.t.valoff[l] = k - code;
+      const int n = s[tid].counts[l - 1];
+      t.valoff[l] = k - code;
       code += n;
       k += n;
-      s.t.maxcode[l] = n ? code - 1 : -1;
+      t.maxcode[l] = n ? code - 1 : -1;
       code <<= 1;
     }
-    s.t.maxcode[17] = -1;
-    s.t.valoff[17] = 0;
-  }
-  if (threadIdx.x == 32) {
-    s.pmin = 1 << CJ_FAST_BITS;
-    s.pmax = -1;
-    if (defined) cj_long_prefixes(s.counts, &s.pmin, &s.pmax);
+    t.maxcode[17] = -1;
+    t.valoff[17] = 0;
+  } else if (tid >= 32 && tid < 32 + ns) {
+    cj_long_prefixes(s[tid - 32].counts, &s[tid - 32].pmin, &s[tid - 32].pmax);
   }
   __syncthreads();
-  for (int f = threadIdx.x; f < (1 << CJ_FAST_BITS); f += blockDim.x) {
-    uint32_t e = 0;
-    for (int l = 1; defined && l <= CJ_FAST_BITS; l++) {
-      const int c = f >> (CJ_FAST_BITS - l);
-      if (c <= s.t.maxcode[l]) {
-        e = ((uint32_t)l << 8) | s.t.vals[(s.t.valoff[l] + c) & 255];
-        break;
+  for (int q = 0; q < ns; q++) {
+    const int slot = s0 + q;
+    BTBuild& b = s[q];
+    if (!((mask >> slot) & 1)) continue;
+    for (int f = tid; f < (1 << CJ_FAST_BITS); f += BT_THREADS) {
+      uint32_t e = 0;
+      for (int l = 1; l <= CJ_FAST_BITS; l++) {
+        const int c = f >> (CJ_FAST_BITS - l);
+        if (c <= b.t.maxcode[l]) {
+          e = ((uint32_t)l << 8) | b.t.vals[(b.t.valoff[l] + c) & 255];
+          break;
+        }
       }
+      b.t.fast[f] = (uint16_t)e;
+      b.pri[f] = cj_step_primary(b.t, b.pmin, b.pmax, f, slot >= 2);
     }
-    s.t.fast[f] = (uint16_t)e;
-    const uint16_t st = defined ? cj_step_primary(s.t, s.pmin, s.pmax, f, ac) : (uint16_t)CJ_STEP_BAD;
-    s.pri[f] = st;
-    p.steps.pri[slot][f] = st;
-  }
-  for (int e = threadIdx.x; e < CJ_STEP_SUBS * 64; e += blockDim.x) {
-    const int i = e >> 6, j = e & 63;
-    const uint16_t st = defined && s.pmin + i <= s.pmax ? cj_step_sub(s.t, s.pmin, i, j, ac) : (uint16_t)CJ_STEP_BAD;
-    p.steps.sub[slot][i][j] = st;
-    if (ac) tb.sub[slot - 2][i][j] = cj_spec_sub(st);
+    for (int e = tid; slot >= 2 && e < CJ_STEP_SUBS * 64; e += BT_THREADS) {
+      const int i = e >> 6, j = e & 63;
+      const uint16_t st = b.pmin + i <= b.pmax ? cj_step_sub(b.t, b.pmin, i, j, true) : (uint16_t)CJ_STEP_BAD;
+      tb.sub[slot - 2][i][j] = cj_spec_sub(st);
+    }
   }
   __syncthreads();
-  for (int k = threadIdx.x; k < (int)(sizeof(CJHuff) / 4); k += blockDim.x)
-    reinterpret_cast<uint32_t*>(&p.huff[slot])[k] = reinterpret_cast<const uint32_t*>(&s.t)[k];
-  if (ac) {
-    for (int e = threadIdx.x; e < (1 << CJ_MULTI_BITS); e += blockDim.x) tb.acm[slot - 2][e] = cj_spec_acm(s.pri, e);
-    for (int e = threadIdx.x; e < (1 << CJ_FAST_BITS); e += blockDim.x) tb.ac1[slot - 2][e] = cj_spec_ac1(s.pri[e]);
-  } else {
-    for (int e = threadIdx.x; e < (1 << CJ_MULTI_DC_BITS); e += blockDim.x) tb.dc[slot][e] = cj_spec_dc(s.pri, e);
+  for (int q = 0; q < ns; q++) {
+    const int slot = s0 + q;
+    const BTBuild& b = s[q];
+    if (!((mask >> slot) & 1)) continue;
+    for (int k = tid; k < (int)(sizeof(CJHuff) / 4); k += BT_THREADS)
+      reinterpret_cast<uint32_t*>(&p.huff[slot])[k] = reinterpret_cast<const uint32_t*>(&b.t)[k];
+    if (slot >= 2) {
+      for (int e = tid; e < (1 << CJ_MULTI_BITS); e += BT_THREADS) tb.acm[slot - 2][e] = cj_spec_acm(b.pri, e);
+      for (int e = tid; e < (1 << CJ_FAST_BITS); e += BT_THREADS) tb.ac1[slot - 2][e] = cj_spec_ac1(b.pri[e]);
+    } else {
+      for (int e = tid; e < (1 << CJ_MULTI_DC_BITS); e += BT_THREADS) tb.dc[slot][e] = cj_spec_dc(b.pri, e);
+    }
   }
-  __syncthreads();  // s is reused by the CTA's next slot
+  __syncthreads();  // s is reused for the CTA's next item
 }
 
 // Phase 0: one CTA writes one image's geometry and quantisation tables (the
@@ -621,14 +640,18 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) k_decode_batch(CJBatchArgs a
   const int lane = threadIdx.x & 31;
 
   bt_stamp(a.ctl, 0);
-  // ---- phase 0: tables + status, one item per image and table slot (a single
-  // image's four slots go to four CTAs).  An image whose DHT contents equal
-  // the reference image's is served by that image's tables.
-  for (int e = blockIdx.x; e < 4 * a.n; e += gridDim.x) {
-    const int i = e >> 2, slot = e & 3;
+  // ---- phase 0: tables + status, an item per image, or per image and table slot
+  // while that gives no CTA a second one (a single image's four slots go to four
+  // CTAs; of 8192 images, slot by slot, the comparison below alone took 0.2 ms).  An
+  // image whose DHT contents equal the reference image's is served by that
+  // image's tables.
+  const int spread = 4 * (int64_t)a.n <= gridDim.x ? 4 : 1;
+  for (int e = blockIdx.x; e < spread * a.n; e += gridDim.x) {
+    const int i = e / spread, part = e % spread;
     const int tab = i != a.tab_ref && bt_same_tables(a.hdr[i], a.hdr[a.tab_ref]) ? a.tab_ref : i;
-    if (tab == i) bt_build_slot(a.hdr[i], a.prm[i], a.spec[i], slot, *reinterpret_cast<BTBuild*>(smem));
-    if (slot) continue;
+    if (tab == i)
+      bt_build_slots(a.hdr[i], a.prm[i], a.spec[i], part, 4 / spread, reinterpret_cast<BTBuild*>(smem));
+    if (part) continue;
     bt_build_params(a.hdr[i], a.prm[i], tab);
     if (threadIdx.x == 0) {
       CJStatus z;
@@ -841,7 +864,7 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) k_decode_batch(CJBatchArgs a
       if (wg >= a.nwarps) continue;  // CTA-uniform
       const int w = wg + (int)(threadIdx.x >> 5);
       const BTItem it = bt_item(a, w, h);
-      bt_with_tables<2, 0>(a, s_tabs, smem, it.tab, [&](uint32_t tb) {
+      bt_with_tables<2, 0, false>(a, s_tabs, smem, it.tab, [&](uint32_t tb, const uint8_t* gt) {
         const CJImageDesc& d = a.desc[it.i];
         const CJScanParams &sp = a.prm[it.i], &tp = a.prm[it.tab];
         CJLane ln = cj_lane(a.segs + d.seg0, it.nseg, it.nsub, it.j0 + lane, d.sub_bits);
@@ -851,8 +874,8 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) k_decode_batch(CJBatchArgs a
         const int64_t gs = d.sub0 + it.j0 + lane, hs = gs * 2 * (nh + 1) + h;
         CJCkpt* hc = cj_lane_ckpts(a.hckpt, hs);
         CJSpecJob x;
-        cj_spec_job(x, sp, tp, tb, a.data + d.data_off, ln, hc, cj_ckpt_step(d.sub_bits), spw);
-        cj_spec_warp<true>(&x, run, cj_state(ln.begin, (uint32_t)h));
+        cj_spec_job(x, sp, tp, tb, gt, a.data + d.data_off, ln, hc, cj_ckpt_step(d.sub_bits), spw);
+        cj_spec_run<true, false>(x, run, cj_state(ln.begin, (uint32_t)h));
         if (run) {
           a.hrecs[hs] = x.r;
           if (h == 0) {
@@ -878,7 +901,7 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) k_decode_batch(CJBatchArgs a
       if (wg >= a.nwarps) continue;  // CTA-uniform
       const int w = wg + (int)(threadIdx.x >> 5);
       const BTItem it = bt_item(a, w, 0);
-      bt_with_tables<2, 0>(a, s_tabs, smem, it.tab, [&](uint32_t tb) {
+      bt_with_tables<2, 0, false>(a, s_tabs, smem, it.tab, [&](uint32_t tb, const uint8_t* gt) {
         const CJImageDesc& d = a.desc[it.i];
         const CJScanParams &sp = a.prm[it.i], &tp = a.prm[it.tab];
         const int nhi = min(nh, sp.bpm - 1);
@@ -889,7 +912,7 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) k_decode_batch(CJBatchArgs a
         const bool run = ln.active && !ln.head && p <= (pred_head ? 0 : nhi);
         CJCkpt* pc = cj_lane_ckpts(a.hckpt, hb + (nh + 1) + p);
         CJSpecJob x;
-        cj_spec_job(x, sp, tp, tb, a.data + d.data_off, ln, pc, cj_ckpt_step(d.sub_bits), spw);
+        cj_spec_job(x, sp, tp, tb, gt, a.data + d.data_off, ln, pc, cj_ckpt_step(d.sub_bits), spw);
         x.hck = cj_lane_ckpts(a.hckpt, hb);
         x.hrec = a.hrecs + hb;
         x.hpp = (uint32_t)__cvta_generic_to_shared(hpp);
@@ -899,7 +922,7 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) k_decode_batch(CJBatchArgs a
           from = __ldcg(&a.hrecs[(gs - 1) * 2 * (nh + 1) + p].exit);
           cj_hyp_fill(hpp, x.hck, nhi + 1);
         }
-        cj_spec_warp<true>(&x, run, from);
+        cj_spec_run<true, false>(x, run, from);
         if (run) {
           a.hrecs[hb + (nh + 1) + p] = x.r;
           mk = (uint8_t)bt_exit_index(a.hrecs + hb, nhi, x.r.exit);
@@ -911,20 +934,21 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) k_decode_batch(CJBatchArgs a
   }
   // ---- phase 5: speculative decode + warp settle, in groups of BT_WARPS
   // consecutive warps per CTA (handed out dynamically) with staged tables
+  const int per = bt_group(a.nwarps);
   bool first = true;
   for (;;) {
-    const int g0 = bt_next_group(&a.ctl->next_sync, &s_grp, s_rank.rank, first);
+    const int g0 = bt_next_group(&a.ctl->next_sync, &s_grp, s_rank.rank, first, per);
     if (g0 >= a.nwarps) break;
-    const int w = g0 + (int)(threadIdx.x >> 5);
+    const int w = (int)(threadIdx.x >> 5) < per ? g0 + (int)(threadIdx.x >> 5) : a.nwarps;
     const BTItem it = bt_item(a, w, 0);
-    bt_with_tables<2, 0>(a, s_tabs, smem, it.tab, [&](uint32_t tb) {
+    bt_with_tables<2, 0, !HYP>(a, s_tabs, smem, it.tab, [&](uint32_t tb, const uint8_t* gt) {
       const CJImageDesc& d = a.desc[it.i];
       const CJScanParams &sp = a.prm[it.i], &tp = a.prm[it.tab];
       CJLane ln = cj_lane(a.segs + d.seg0, it.nseg, it.nsub, it.j0 + lane, d.sub_bits);
       const int64_t gs = d.sub0 + it.j0 + lane;
       const uint64_t guess = cj_state(ln.begin, 0);
       CJSpecJob x;
-      cj_spec_job(x, sp, tp, tb, a.data + d.data_off, ln, cj_lane_ckpts(a.ckpt, gs), cj_ckpt_step(d.sub_bits), spw);
+      cj_spec_job(x, sp, tp, tb, gt, a.data + d.data_off, ln, cj_lane_ckpts(a.ckpt, gs), cj_ckpt_step(d.sub_bits), spw);
       x.r.start = x.r.exit = guess;
       x.r.nblocks = x.r.dc[0] = x.r.dc[1] = x.r.dc[2] = 0;
       if constexpr (HYP) {
@@ -934,8 +958,8 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) k_decode_batch(CJBatchArgs a
         if (ln.active) x.r = bt_load_rec(&a.recs[gs]);
         bt_settle_map(a, x, ln, pred_head, x.r.start, gs, min(nh, sp.bpm - 1), hpp);
       } else {
-        cj_spec_warp<false>(&x, ln.active, guess);
-        cj_warp_settle(x, ln, guess);
+        cj_spec_run<false, true>(x, ln.active, guess);
+        cj_warp_settle<true>(x, ln, guess);
       }
       if (ln.active) a.recs[gs] = x.r;
       unsigned act = __ballot_sync(CJ_FULL, ln.active);
@@ -962,9 +986,9 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) k_decode_batch(CJBatchArgs a
     }
     first = true;
     for (;;) {
-      const int g0 = bt_next_group(next, &s_grp, s_rank.rank, first);
+      const int g0 = bt_next_group(next, &s_grp, s_rank.rank, first, per);
       if (g0 >= a.nwarps) break;
-      const int w = g0 + (int)(threadIdx.x >> 5);
+      const int w = (int)(threadIdx.x >> 5) < per ? g0 + (int)(threadIdx.x >> 5) : a.nwarps;
       const BTItem it = bt_item(a, w, 0);
       const bool work = it.tab >= 0;  // warp-uniform, like everything below
       if (!work && w < a.nwarps && lane == 0) {
@@ -987,17 +1011,17 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) k_decode_batch(CJBatchArgs a
       const uint64_t want = ln.head ? r.start : (lane == 0 ? in0 : pred);
       bool moved = false;
       const bool redo = __any_sync(CJ_FULL, ln.active && want != r.start);
-      bt_with_tables<2, 0>(a, s_tabs, smem, redo ? it.tab : -1, [&](uint32_t tb) {
+      bt_with_tables<2, 0, !HYP>(a, s_tabs, smem, redo ? it.tab : -1, [&](uint32_t tb, const uint8_t* gt) {
         const CJScanParams &sp = a.prm[it.i], &tp = a.prm[it.tab];
         const int64_t gs = d.sub0 + j0 + lane;
         CJSpecJob x;
-        cj_spec_job(x, sp, tp, tb, a.data + d.data_off, ln, cj_lane_ckpts(a.ckpt, gs), cj_ckpt_step(d.sub_bits), spw);
+        cj_spec_job(x, sp, tp, tb, gt, a.data + d.data_off, ln, cj_lane_ckpts(a.ckpt, gs), cj_ckpt_step(d.sub_bits), spw);
         x.r = r;
         if constexpr (HYP) {
           const bool pred_head = ln.active && !ln.head && j0 + lane - 1 == a.segs[d.seg0 + ln.seg].first_sub;
           moved = bt_settle_map(a, x, ln, pred_head, in0, gs, min(nh, sp.bpm - 1), hpp);
         } else {
-          moved = cj_warp_settle(x, ln, in0);
+          moved = cj_warp_settle<true>(x, ln, in0);
         }
         r = x.r;
       });
@@ -1091,6 +1115,7 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) k_decode_batch(CJBatchArgs a
   {
     constexpr int UNITS = CJ_CKPTS + 1, LANES = 32 / UNITS;
     const int nitems = a.nwarps * UNITS;
+    const int per_write = bt_group(nitems);
     const int wp = threadIdx.x >> 5;
     // the warps' block buffers, zero between blocks
     for (int k = threadIdx.x; k < BT_WTAB_OFF / 16; k += BT_THREADS)
@@ -1099,11 +1124,12 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) k_decode_batch(CJBatchArgs a
     CJWriteWarp& ww = reinterpret_cast<CJWriteWarp*>(smem + BT_WRITE_OFF)[wp];
     first = true;
     for (;;) {
-      const int g0 = bt_next_group(&a.ctl->next_write, &s_grp, s_rank.rank, first);
+      const int g0 = bt_next_group(&a.ctl->next_write, &s_grp, s_rank.rank, first, per_write);
       if (g0 >= nitems) break;
-      const int t = g0 + wp, w = t / UNITS, part = t % UNITS;
-      const BTItem it = bt_item(a, t < nitems ? w : a.nwarps, 0);
-      bt_with_tables<1, BT_WTAB_FROM>(a, s_tabs, smem + BT_WTAB_OFF, it.tab, [&](uint32_t tb) {
+      const int t = wp < per_write ? g0 + wp : nitems, part = t / a.nwarps, w = t - part * a.nwarps;
+      BTItem it = bt_item(a, t < nitems ? w : a.nwarps, 0);
+      if (it.j0 + part * LANES >= it.nsub) it.tab = -1;
+      bt_with_tables<1, BT_WTAB_FROM, true>(a, s_tabs, smem + BT_WTAB_OFF, it.tab, [&](uint32_t tb, const uint8_t* gt) {
         const CJImageDesc& d = a.desc[it.i];
         const int j0 = it.j0, nsub = it.nsub, nseg = it.nseg;
         // block / DC prefix of the 32 lanes of warp w (thread = lane `lane`)
@@ -1160,6 +1186,7 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) k_decode_batch(CJBatchArgs a
         x.base = __shfl_sync(CJ_FULL, blk, 0);
         x.coef = a.coef + (d.coef0 + x.base) * 64;
         x.tab = tb;
+        x.gtab = gt;
         x.ring = bt_smem_addr(ww.ring) + 4 * lane;
         x.phase = bt_smem_addr(ww.phase);
         x.order = bt_smem_addr(ww.order);
@@ -1174,7 +1201,8 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) k_decode_batch(CJBatchArgs a
         x.bend = (int)(seg.first_block + seg.nblocks - x.base);
         x.last = ln.last;
         x.marker = seg.marker_follows != 0;
-        cj_write_warp(&x, ln.active);
+        if (gt) cj_write_warp<true>(&x, ln.active);
+        else cj_write_warp<false>(&x, ln.active);
         // blocks of the range an early stop left undecoded read as zeros
         for (int64_t y = x.base + x.blk + (x.cut ? 1 : 0); ln.active && y < end; y++) {
           uint4* z = reinterpret_cast<uint4*>(a.coef + (d.coef0 + y) * 64);

@@ -97,7 +97,6 @@ struct CJSpecTab {
 // Per-scan parameters, built on the host after SOS and copied once.
 struct alignas(16) CJScanParams {
   CJHuff huff[4];                 // DC0, DC1, AC0, AC1
-  CJSteps steps;                  // the same four tables as decode steps
   int16_t qnat[4][64];            // quantisation tables, natural order
   uint8_t phase_comp[CJ_MAX_BPM]; // component of the k-th block of an MCU
   uint8_t phase_blk[CJ_MAX_BPM];  // index of that block inside its component's MCU part
@@ -282,19 +281,20 @@ CJ_HD uint16_t cj_step_sub(const CJHuff& t, int pmin, int s, int j, bool ac) {
   return (uint16_t)cj_step_of(cj_huff_slow(t, win), ac);
 }
 
-// The decode step for the 32-bit window v (MSB = next bit) of table `slot`,
-// from step tables `T` (sp.steps or a copy of them, e.g. in shared memory).
-CJ_HD uint32_t cj_step(const CJSteps& T, const CJScanParams& sp, uint32_t slot, uint32_t v) {
+// The decode step for the 32-bit window v (MSB = next bit) from the step tables
+// of `slot`; `t` is its canonical table.
+CJ_HD uint32_t cj_step(const CJSteps& T, const CJHuff& t, uint32_t slot, uint32_t v) {
   uint32_t st = T.pri[slot][v >> (32 - CJ_FAST_BITS)];
   if (!(st & 31)) {
     const uint32_t i = st >> 5;
-    st = i != CJ_STEP_SEARCH ? T.sub[slot][i][(v >> 16) & 63]
-                             : cj_step_of(cj_huff_slow(sp.huff[slot], v >> 16), slot >= 2);
+    st = i != CJ_STEP_SEARCH ? T.sub[slot][i][(v >> 16) & 63] : cj_step_of(cj_huff_slow(t, v >> 16), slot >= 2);
   }
   return st;
 }
-CJ_HD uint32_t cj_step(const CJScanParams& sp, uint32_t slot, uint32_t v) { return cj_step(sp.steps, sp, slot, v); }
-
+// The same step from the canonical table alone.
+CJ_HD uint32_t cj_step_canonical(const CJHuff& t, uint32_t slot, uint32_t v) {
+  return cj_step_of(cj_huff_decode(t, v >> 16), slot >= 2);
+}
 
 // Entries of the CJSpecTab from the decode steps: a step, a primary entry of an
 // AC table, entry of a subtable.

@@ -153,6 +153,15 @@ __device__ __forceinline__ uint32_t cj_tab16(uint32_t a) {
   asm("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
   return v;
 }
+// An entry of a CJSpecTab: in shared memory at address a, or (GLOBAL) a bytes into
+// the set at `set` in global memory.
+template <bool GLOBAL>
+__device__ __forceinline__ uint32_t cj_entry(const uint8_t* set, uint32_t a) {
+  if (!GLOBAL) return cj_tab16(a);
+  uint16_t v;
+  asm("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(set + a));
+  return v;
+}
 __device__ __forceinline__ uint32_t cj_tab8(uint32_t a) {
   uint32_t v;
   asm("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(a));
@@ -348,6 +357,7 @@ struct CJSpecWarp {
 struct CJSpecJob {
   const CJScanParams *sp, *tp;
   const uint4* data;
+  const uint8_t* gtab;             // the CJSpecTab where it is not in shared memory (tab: 0)
   uint32_t tab, ring, phase, hpp;  // shared addresses: CJSpecTab, ring column, phase entries, hypothesis column
   uint32_t begin, end, end_byte, cstep;
   int nh;
@@ -358,11 +368,12 @@ struct CJSpecJob {
   CJSubRec r;
 };
 __device__ __forceinline__ void cj_spec_job(CJSpecJob& x, const CJScanParams& sp, const CJScanParams& tp,
-                                            uint32_t tab, const void* data, const CJLane& ln, CJCkpt* ck,
+                                            uint32_t tab, const uint8_t* gtab, const void* data, const CJLane& ln, CJCkpt* ck,
                                             uint32_t cstep, const CJSpecWarp& sw) {
   x.sp = &sp;
   x.tp = &tp;
   x.tab = tab;
+  x.gtab = gtab;
   x.data = reinterpret_cast<const uint4*>(data);
   x.begin = (uint32_t)ln.begin;
   x.end = (uint32_t)ln.end;
@@ -379,9 +390,10 @@ __device__ __forceinline__ void cj_spec_job(CJSpecJob& x, const CJScanParams& sp
 // register budget, and the phases around it keep their state across the call
 // in local memory instead of squeezing the loop (550 bytes of spills, some in
 // the loop, when inlined at 64 registers).
-template <bool HYP>
+template <bool HYP, bool GLOBAL>
 __device__ __noinline__ void cj_spec_warp(CJSpecJob* job, bool run, uint64_t start) {
   CJSpecJob& x = *job;
+  const uint8_t* const set = x.gtab;
   CJWin<CJ_RING_WORDS> br;
   const uint32_t begin = x.begin, end = x.end, cstep = x.cstep, phases = x.phase;
   CJCkpt* const ck = x.ck;
@@ -463,7 +475,7 @@ __device__ __noinline__ void cj_spec_warp(CJSpecJob* job, bool run, uint64_t sta
 #pragma unroll
       for (int q = 0; q < CJ_STEPS_PER_ROUND; q++) {
         const uint32_t v = br.peek();
-        uint32_t st = cj_tab16(tab + 2 * (v >> sh));
+        uint32_t st = cj_entry<GLOBAL>(set, tab + 2 * (v >> sh));
         if (q == 0) {  // a DC symbol can only come first in a round
           dcv = k < 0 ? v : dcv;
           dce = k < 0 ? st : dce;
@@ -477,7 +489,8 @@ __device__ __noinline__ void cj_spec_warp(CJSpecJob* job, bool run, uint64_t sta
         if (k >= CJ_SPEC_FARK) {  // rare
           k -= (int)(CJ_SPEC_FAR >> 9);
           const uint32_t v = br.peek();
-          const uint32_t st = cj_spec_entry(cj_step(*x.tp, k < 0 ? x.sp->comp_dc[c] : x.sp->comp_ac[c], v), 0, k < 0);
+          const uint32_t slot = k < 0 ? x.sp->comp_dc[c] : x.sp->comp_ac[c];
+          const uint32_t st = cj_spec_entry(cj_step_canonical(x.tp->huff[slot], slot, v), 0, k < 0);
           if (k < 0) {
             dcv = v;
             dce = st;
@@ -540,6 +553,13 @@ __device__ __noinline__ void cj_spec_warp(CJSpecJob* job, bool run, uint64_t sta
   }
 }
 
+// GLOBAL: the job's tables may be in global memory (warp-uniform).
+template <bool HYP, bool GLOBAL>
+__device__ __forceinline__ void cj_spec_run(CJSpecJob& x, bool run, uint64_t start) {
+  if (GLOBAL && x.gtab) cj_spec_warp<HYP, GLOBAL>(&x, run, start);
+  else cj_spec_warp<HYP, false>(&x, run, start);
+}
+
 // The checkpoint positions of a lane's `nh` hypothesis decodes into its
 // column of shared memory (entry 32 * (h * CJ_CKPTS + j)).
 __device__ __forceinline__ void cj_hyp_fill(uint32_t* hpp, const CJCkpt* hck, int nh) {
@@ -554,6 +574,7 @@ __device__ __forceinline__ uint32_t cj_ckpt_step(int sub_bits) { return (uint32_
 // Re-decode lanes whose input state (lane 0: `lane0_in`; others: the exit of
 // the previous lane) differs from the state they last decoded from, until no
 // lane changes.  Lane l settles after at most l+1 re-decodes.
+template <bool GLOBAL>
 __device__ __forceinline__ bool cj_warp_settle(CJSpecJob& x, const CJLane& ln, uint64_t lane0_in) {
   int lane = threadIdx.x & 31;
   bool dirty = false;
@@ -563,7 +584,7 @@ __device__ __forceinline__ bool cj_warp_settle(CJSpecJob& x, const CJLane& ln, u
     uint64_t want = ln.head ? x.r.start : (lane == 0 ? lane0_in : pred);
     bool change = ln.active && want != x.r.start;
     if (!__any_sync(CJ_FULL, change)) break;
-    cj_spec_warp<false>(&x, change, want);
+    cj_spec_run<false, GLOBAL>(x, change, want);
     dirty = dirty || change;
   }
   return dirty;
@@ -654,6 +675,7 @@ struct CJWriteJob {
   const uint4* data;
   int16_t* coef;  // of block `base`
   int64_t base;   // blk and bend count from here
+  const uint8_t* gtab;  // as in CJSpecJob
   uint32_t tab, ring, phase, order, wbuf, zz;  // shared addresses (wbuf: the warp's 32 blocks; zz: 2 x zig-zag index)
   uint32_t end_byte, end, stop, seg_end;       // bits: of the subsequence, of the unit, of the segment
   uint32_t pos, m;                             // the unit's first block
@@ -677,8 +699,10 @@ struct CJWriteJob {
 // Measured on the 1024-image mix: 1.05 ms with a branch per event, tables in
 // global memory and a store loop per symbol; 0.72 ms as here (48 1080p frames
 // 0.35 -> 0.23, 512 thumbnails 0.25 -> 0.12).
+template <bool GLOBAL>
 static __device__ __noinline__ void cj_write_warp(CJWriteJob* job, bool active) {
   CJWriteJob& x = *job;
+  const uint8_t* const set = x.gtab;
   const int lane = threadIdx.x & 31;
   cj_phase_entries(*x.sp, x.tab, x.phase);
   CJWin<CJ_WRITE_WORDS> br;
@@ -755,17 +779,18 @@ static __device__ __noinline__ void cj_write_warp(CJWriteJob* job, bool active) 
 #pragma unroll
     for (int q = 0; q < CJ_STEPS_PER_ROUND; q++) {
       const uint32_t v = br.peek();
-      uint32_t st = cj_tab16(tab + 2 * (v >> sh));
+      uint32_t st = cj_entry<GLOBAL>(set, tab + 2 * (v >> sh));
       lst = k < 63 ? st : lst;
       st = k < 63 ? st : 0;
       symbol(st, v, q == 0);
     }
     bool done = false;
     if (live && k >= 63) {
-      if (k >= CJ_SPEC_FARK) {  // rare: through the steps in memory
+      if (k >= CJ_SPEC_FARK) {  // rare: from the canonical table in memory
         k -= (int)(CJ_SPEC_FAR >> 9);
         const uint32_t v = br.peek();
-        lst = cj_spec_entry(cj_step(*x.tp, k < 0 ? x.sp->comp_dc[c] : x.sp->comp_ac[c], v), 0, k < 0);
+        const uint32_t slot = k < 0 ? x.sp->comp_dc[c] : x.sp->comp_ac[c];
+        lst = cj_spec_entry(cj_step_canonical(x.tp->huff[slot], slot, v), 0, k < 0);
         symbol(lst, v, true);
       }
       if (k >= 63) {
