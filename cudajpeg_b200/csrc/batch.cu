@@ -1977,11 +1977,15 @@ static int bt_sub_cap(int64_t scan_len, int nseg, int sub_bits) {
 //
 // Hypotheses (one image, or a batch small enough): only for MCUs of
 // 5 blocks and more, where a decode out of step with the MCU phase stays so for
-// thousands of bits, and up to 16 warps per SM of them.  One 4:2:0 file
+// thousands of bits, and up to 16 warps per SM of them, or 32 at a size that was
+// set (no larger one can be taken instead).  One 4:2:0 file
 // with / without: 1024x768 0.22 / 0.30 ms, 4096x4096 0.44 / 0.70; 4:2:2
-// 1024x768 0.19 / 0.15, 4:4:4 0.17 / 0.13.
+// 1024x768 0.19 / 0.15, 4:4:4 0.17 / 0.13.  Sizes set, with / without, whole call:
+// 3000x2000 at 512 bits (16.3 warps per SM) 0.66 / 0.94, 2048x1536 at 256 (23.4) 0.52 /
+// 0.68, 1600x1200 at 128 (28.5) 0.56 / 0.68, 8 of 1024x768 at 512 (18.5) 0.41 / 0.65.
 #define BT_FILL_WARPS 8
 #define BT_FILL_HYP 16
+#define BT_FILL_HYP_SET 32
 #define BT_HYP_MIN_BPM 5
 template <class F>
 static int bt_fill_bits(int from, int to, int sms, F warps) {
@@ -2381,7 +2385,8 @@ int cjBatchStage(CJBatch* b, int n, const unsigned char* blob, const int64_t* of
     CJ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
                     &per_sm_hyp, (const void*)bt_decode_kernel(b->decode_ctas, true), BT_THREADS, bt_decode_smem(nh)),
                 CUDA_KERNEL_LAUNCH_ERROR);
-    if (nh >= BT_HYP_MIN_BPM && per_sm_hyp > 0 && (int64_t)nsubw * nh <= (int64_t)BT_FILL_HYP * b->sm_count) {
+    const int64_t room = (int64_t)(b->sub_bits_auto ? BT_FILL_HYP : BT_FILL_HYP_SET) * b->sm_count;
+    if (nh >= BT_HYP_MIN_BPM && per_sm_hyp > 0 && (int64_t)nsubw * nh <= room) {
       const size_t nsub = (size_t)nsubw * 32, nrec = nsub * 2 * nh;  // hypotheses and probes
       if (bt_ensure(b, b->hrecs, nrec * sizeof(CJSubRec)) || bt_ensure(b, b->hckpt, nrec * CJ_CKPTS * sizeof(CJCkpt)) ||
           bt_ensure(b, b->hmap, nsub * 16))
@@ -2869,7 +2874,8 @@ int cj_reader_decode(JPGReader* jpg, bool stage) {
     d->b_nhyp = 1;
     int cap_run = cap;  // co-resident CTAs of the variant that runs
     const int groups = (nwarps + BT_WARPS - 1) / BT_WARPS;
-    if (nh >= BT_HYP_MIN_BPM && (int64_t)nwarps * nh <= (int64_t)BT_FILL_HYP * sms) {
+    const int64_t room = (int64_t)(d->sub_bits_auto ? BT_FILL_HYP : BT_FILL_HYP_SET) * sms;
+    if (nh >= BT_HYP_MIN_BPM && (int64_t)nwarps * nh <= room) {
       int per_hyp = 0;
       CJ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_hyp, (const void*)bt_decode_kernel(BT_HYP_CTAS, true),
                                                                 BT_THREADS, bt_decode_smem(nh)),
