@@ -2897,7 +2897,7 @@ int cj_reader_decode(JPGReader* jpg, bool stage) {
     d->b_nptiles = desc.nptiles;
     d->raw_len = (size_t)n;
     d->total_blocks = h.total_blocks;
-    d->param_bytes = sizeof(CJImageHeader) + sizeof(CJImageDesc);
+    d->param_bytes = sizeof(BTReaderBlock);
     CJ_CUDA_TRY(cudaEventRecord(d->ev_begin, s), CUDA_KERNEL_LAUNCH_ERROR);
     BTReaderBlock blk;
     memset(&blk, 0, sizeof(blk));

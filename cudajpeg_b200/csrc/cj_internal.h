@@ -59,7 +59,7 @@ struct CJReaderDevice {
   int comp_first[3];      // first block of each component inside an MCU
   // the scan as one image of the batch decode kernel (cj_reader_decode)
   int b_grid = 0, b_ntiles = 0, b_nwarps = 0, b_nptiles = 0, b_nhyp = 1;
-  size_t param_bytes = 0;  // header + plan bytes copied to the device per scan
+  size_t param_bytes = 0;  // bytes copied to the device per scan beside the file's (header, plan, control block)
   // kernel accounting: launches since reader creation, and (when profiling)
   // one event after each kernel of the last decode
   long long launches = 0;
