@@ -56,8 +56,6 @@
 #define BT_MAX_HYP 10
 #define BT_TILE_BYTES 4096  // destuff tile: 256 threads x 16 bytes
 #define BT_TILE_BAD (1 << 30)  // flag in a tile's marker count: malformed FF sequence
-// fixed shared-memory offsets of the tensor-core form's A tile and basis
-// (cj_pix_layout with two coefficient buffers)
 
 // ---------------------------------------------------------------- layouts
 
@@ -153,9 +151,6 @@ struct CJBatchArgs {
 
 __device__ __forceinline__ void bt_raise(CJStatus* st, int64_t block, int code) {
   atomicMax(&st->err_key, ~(((unsigned long long)block << 8) | (unsigned)code));
-}
-__device__ __forceinline__ void bt_raise_dec(CJStatus* st, int64_t block, int code) {
-  atomicMax(&st->dec_err_key, ~(((unsigned long long)block << 8) | (unsigned)code));
 }
 
 // Grid barrier for a cooperative launch (all CTAs co-resident).  The wait is
@@ -612,7 +607,6 @@ __device__ void bt_build_params(const CJImageHeader& h, CJScanParams& p, int tab
     p.restart_interval = h.restart_interval;
     p.nseg_expected = h.nseg_expected;
     p.total_blocks = h.total_blocks;
-    p.phase_pack = cj_phase_pack(p);
     p.tab = tab;
   }
 }
@@ -1223,7 +1217,6 @@ static bt_decode_fn bt_decode_kernel(int ctas_per_sm, bool hyp = false) {
   if (hyp) return k_decode_batch<BT_HYP_CTAS, true>;
   switch (ctas_per_sm) {
     case 3: return k_decode_batch<3>;
-    case 5: return k_decode_batch<5>;
     default: return k_decode_batch<4>;
   }
 }
@@ -1233,7 +1226,7 @@ static bt_decode_fn bt_decode_kernel(int ctas_per_sm, bool hyp = false) {
 static cudaError_t bt_decode_attrs() {
   cudaError_t e = cudaFuncSetAttribute((const void*)bt_decode_kernel(BT_HYP_CTAS, true),
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bt_decode_smem(BT_MAX_HYP));
-  for (int c = 3; c <= 5 && e == cudaSuccess; c++)
+  for (int c = 3; c <= 4 && e == cudaSuccess; c++)
     e = cudaFuncSetAttribute((const void*)bt_decode_kernel(c), cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)bt_decode_smem(1));
   return e;
@@ -2731,7 +2724,7 @@ int cjBatchAutotune(CJBatch* b, int n, const unsigned char* blob, const int64_t*
   if (!b || n <= 0 || !blob) return PROGRAMMER_ERROR;
   if (reps < 1) reps = 3;
   static const int subs[] = {512, 1024, 2048, 4096};
-  static const int ctas[] = {3, 4, 5};
+  static const int ctas[] = {3, 4};
   int best_s = b->sub_bits, best_c = b->decode_ctas, best_t = 0;
   float best = 1e30f;
   int trial = 0;
@@ -2982,8 +2975,8 @@ int cj_reader_decode_status(const JPGReader* jpg) {
 // memory.  The array is held by every GPU that loads the library until the
 // process exits.
 
-// 24 MiB per device, and room for the speculative-decode tables
-#define CJ_NOALLOC_SCRATCH_BYTES ((24u << 20) + (32u << 10))
+// 24 MiB per device, and room for the entropy loops' tables
+#define CJ_NOALLOC_SCRATCH_BYTES ((24u << 20) + (4u << 10))
 #define CJ_NOALLOC_MAX_DEVICES 64
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[CJ_NOALLOC_SCRATCH_BYTES];

@@ -71,7 +71,7 @@ struct CJSteps {
 //              invalid code adds 63, in a DC table 64); 0: the first 10 bits of
 //              a longer code, decoded on from its row by the next 6 bits
 // CJ_SPEC_FAR (nothing consumed, the position past every other): decode the
-// symbol through the CJSteps in memory -- DC codes of more than 9 bits and AC
+// symbol through the canonical table in memory -- DC codes of more than 9 bits and AC
 // tables with more long-code prefixes than rows.
 //   acm  (the speculative decode, which needs positions and DC sums but no AC
 //        values) every whole symbol the next CJ_MULTI_BITS bits determine, as one entry,
@@ -112,21 +112,8 @@ struct alignas(16) CJScanParams {
   int64_t total_blocks;              // mcux*mcuy*bpm
   int32_t comp_stride[3];            // plane strides (bytes) for plane outputs
   int32_t comp_rows[3];
-  // phases 0..bpm-1 of an MCU, 6 bits each: component | DC slot << 2 |
-  // AC slot << 4 (valid when bpm <= 10, the standard's limit)
-  uint64_t phase_pack;
   int32_t tab;  // batch: the image whose decode tables serve this one (the same DHT contents)
 };
-
-// Component and DC / AC table slots of MCU phase m.
-CJ_HD uint64_t cj_phase_pack(const CJScanParams& p) {
-  uint64_t pack = 0;
-  for (int m = 0; m < p.bpm && m < 10; m++) {
-    const int c = p.phase_comp[m];
-    pack |= (uint64_t)(c | (p.comp_dc[c] << 2) | (p.comp_ac[c] << 4)) << (6 * m);
-  }
-  return pack;
-}
 
 // A restart interval (or the whole scan) in the destuffed buffer.
 struct CJSegment {
@@ -210,17 +197,6 @@ CJ_HD uint32_t cj_bswap(uint32_t v) {
 #else
   return __builtin_bswap32(v);
 #endif
-}
-
-// 32-bit big-endian word `w` of the destuffed buffer; bytes at or past
-// `end_byte` read as 0xFF (the padding the reference's bit reader supplies).
-CJ_HD uint32_t cj_word(const uint32_t* words, uint64_t w, uint64_t end_byte) {
-  uint64_t first = w * 4;
-  if (first >= end_byte) return 0xFFFFFFFFu;
-  uint32_t v = cj_bswap(words[w]);
-  uint64_t last = first + 4;
-  if (last > end_byte) v |= (1u << (8 * (uint32_t)(last - end_byte))) - 1u;
-  return v;
 }
 
 // Decode one Huffman code from a left-aligned 16-bit window.  Returns

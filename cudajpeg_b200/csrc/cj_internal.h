@@ -51,7 +51,7 @@ struct CJReaderDevice {
   unsigned wait_limit = 0;  // polls of a wait between CTAs before it is given up (0 = default)
   // per-scan bookkeeping
   int sub_bits = CJ_SUB_BITS_DEFAULT;
-  bool sub_bits_auto = true;  // no size set: the decode picks 512 or 1024 bits per image
+  bool sub_bits_auto = true;  // no size set: the decode picks one per image (bt_fill_bits)
   size_t raw_len = 0;
   int64_t total_blocks = 0;
   int nsub_cap = 0, nwarp_cap = 0, nseg_exp = 0, mark_cap = 0;

@@ -92,7 +92,7 @@ long long cjReaderLaunchCount(const JPGReader *r);
 int cjDebugHuffDecode(const unsigned char counts[16], const unsigned char *symbols,
                       unsigned int win16);
 
-/* Host check of the decode-step tables the entropy kernels use: for every
+/* Host check of the decode steps the entropy kernels' tables are made of: for every
  * 16-bit window w, out[w] = the step entry for a DC (ac = 0) or AC table built
  * from the DHT counts and symbols -- bits consumed (code + magnitude) in bits
  * 0-4, zig-zag advance in bits 5-11 (DC 1, AC run + 1, ZRL 16, EOB 64,
@@ -134,10 +134,11 @@ int cjBatchSetSubsequenceBits(CJBatch *b, int bits);
 
 /* Tuning of later stages/runs: bits per speculative subsequence (0 =
  * default: 4096 for a full batch, less for one that leaves the GPU unfilled;
- * multiple of 32, 128..65536), decode-kernel CTAs per SM (3, 4 or 5,
- * 0 = 4: the register budget per thread of the entropy kernel, 80/64/48), and
- * the largest pixel tile in MCUs (power of two, 0 = the layout maximum:
- * 128 pixels across). */
+ * multiple of 32, 128..65536), decode-kernel CTAs per SM (3 or 4, 0 = 4: the
+ * register budget per thread of the entropy kernel, 80 or 64; 5 is taken as 4,
+ * the most that the kernel's shared memory allows; batches decoded with MCU-phase
+ * hypotheses have one build, at most 3), and the largest pixel tile in MCUs
+ * (power of two, 0 = the layout maximum: 128 pixels across). */
 int cjBatchSetTuning(CJBatch *b, int sub_bits, int decode_ctas_per_sm, int pixel_tile_cap);
 void cjBatchGetTuning(const CJBatch *b, int *sub_bits, int *decode_ctas_per_sm, int *pixel_tile_cap);
 /* Chroma sampling classes of a batch's images (by the sampling factors of
@@ -189,10 +190,10 @@ int cjBatchSetOutput(CJBatch *b, int format, int idct);
 int cjBatchSetParse(CJBatch *b, int on_device);
 /* MCU-phase hypotheses of the entropy decode (on != 0, the default): when a
  * staged batch's speculative decodes leave most of the GPU idle (a few
- * images) and its MCUs have 5 blocks or more (4:2:0), each subsequence is also
- * decoded from
- * its first bit under every other MCU phase and then from each of its
- * predecessor's hypothesis exits; the settle takes those decodes instead of
+ * images: at most 16 warps per SM of these decodes, 32 at a subsequence size that
+ * was set) and its MCUs have 5 blocks or more (4:2:0), each subsequence is also
+ * decoded from its first bit under every other MCU phase and then from each of
+ * its predecessor's hypothesis exits; the settle takes those decodes instead of
  * re-decoding lane after lane.  Results are identical either way; only the
  * time to settle changes (device memory: two records and checkpoint sets
  * per subsequence and hypothesis). */
@@ -208,7 +209,7 @@ void cjBatchGetOutput(const CJBatch *b, int *format, int *idct);
 int cjBatchSetWaitLimit(CJBatch *b, unsigned polls);
 /* Autotuner: times the given batch (device time, median of `reps` runs)
  * under every subsequence size in {512, 1024, 2048, 4096} x decode CTAs per
- * SM in {3, 4, 5}; then, one sampling class of the batch at a time (classes
+ * SM in {3, 4}; then, one sampling class of the batch at a time (classes
  * holding at least 1/16 of its scan bytes), the sizes {1024 .. 16384} other
  * than the batch-wide best for that class alone; then pixel tile caps
  * {8, 4, 2}; and keeps the fastest tuning in `b` (per-class sizes equal to
