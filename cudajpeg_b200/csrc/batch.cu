@@ -348,7 +348,7 @@ __device__ __forceinline__ void bt_rank_end(CJBatchCtl* ctl, BTRank& k) {
   for (int s = 0; s < k.slot; s++) k.rank += __ldcg(&ctl->slot_ctas[s]);
 }
 
-// Next group of BT_WARPS consecutive items for the whole CTA: group `rank`
+// Next group of `per` consecutive items for the whole CTA: group `rank`
 // first, then thread 0 takes one and the CTA shares it.  The leading barrier
 // also ends the previous group: every warp is done with it and with the tables
 // staged for it.
@@ -364,7 +364,9 @@ __device__ __forceinline__ int bt_next_group(int* counter, int* s_slot, int rank
 }
 
 // Items per group: fewer than the CTA's warps where the items would not give every
-// CTA a full group.
+// CTA a full group, so that fewer table sets meet in a CTA.  512 thumbnails with
+// tables of their own, sync phase: groups of 8 0.40 ms, of 2 0.19; with shared
+// tables 0.15 either way.
 __device__ __forceinline__ int bt_group(int items) {
   int g = BT_WARPS;
   while (g > 1 && items <= (int)gridDim.x * (g / 2)) g /= 2;
@@ -429,10 +431,14 @@ __device__ __forceinline__ BTItem bt_item(const CJBatchArgs& a, int w, int h) {
 // few images, and of one if the images share their DHT contents, as files of
 // one encoder do.  The CTA keeps the tables of SLOTS images in shared memory
 // (`id`: which, -1: none) -- each image's bytes from `off` of its CJSpecTab on --
-// and serves its warps in rounds: stage what the first
-// waiting warp and, with two slots, the next one with other tables need (nothing
-// when they are there from an earlier group), and run f(shared address of the
-// CJSpecTab) in the warps with either.
+// and stages what the first warp with work and, with two slots, the next one with
+// other tables need (nothing when they are there from an earlier group).  Warps with
+// either run f(shared address of the CJSpecTab, null).  The others, in a batch of
+// files with tables of their own, run f(0, the CJSpecTab in global memory) beside them
+// (GLOBAL); the hypothesis variant, which batches of a few images run, takes them in
+// further rounds instead.  8192 files of 16-64 pixels with tables of their own: sync 0.52 ms in
+// rounds, 0.45 with tables in global memory beside them; write-out 0.69 and, with the
+// quarters of all warps dealt one after another (phase 8), 0.27.
 // `tab`: the warp's table image, -1: no work.  Every thread calls it.
 struct BTTabs {
   int want[BT_WARPS], id[2];
@@ -926,8 +932,8 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) k_decode_batch(CJBatchArgs a
     }
     if (!bt_grid_sync(a.ctl, gen, a.wait_limit, &s_ok)) return;
   }
-  // ---- phase 5: speculative decode + warp settle, in groups of BT_WARPS
-  // consecutive warps per CTA (handed out dynamically) with staged tables
+  // ---- phase 5: speculative decode + warp settle, in groups of up to BT_WARPS
+  // consecutive warps per CTA (bt_group), handed out dynamically
   const int per = bt_group(a.nwarps);
   bool first = true;
   for (;;) {
@@ -1103,7 +1109,10 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) k_decode_batch(CJBatchArgs a
   // so write items are a quarter as long as sync items whatever the
   // subsequence size.  An item is 8 lanes x 4 units of one 32-lane warp w,
   // whose block / DC prefix it recomputes; the warp writes its 32 units'
-  // blocks cooperatively (cj_write_warp).  (In a corrupt stream a unit may
+  // blocks cooperatively (cj_write_warp).  The items are those of the first 8 lanes of
+  // every warp, then of the next 8, and so on: an image of a few subsequences has work
+  // for its first item only, and four items of one warp in a group left most warps of
+  // a batch of such images idle.  (In a corrupt stream a unit may
   // write past an error an earlier unit stopped at; only blocks after that
   // error, so the first error of the image is the same.)
   {
@@ -1970,15 +1979,18 @@ static int bt_sub_cap(int64_t scan_len, int nseg, int sub_bits) {
 //
 // Hypotheses (one image, or a batch small enough): only for MCUs of
 // 5 blocks and more, where a decode out of step with the MCU phase stays so for
-// thousands of bits, and up to 16 warps per SM of them, or 32 at a size that was
-// set (no larger one can be taken instead).  One 4:2:0 file
+// thousands of bits, and up to 16 warps per SM of them, or 32 where a size of 512
+// bits or less was set (a larger one cannot be taken instead).  One 4:2:0 file
 // with / without: 1024x768 0.22 / 0.30 ms, 4096x4096 0.44 / 0.70; 4:2:2
 // 1024x768 0.19 / 0.15, 4:4:4 0.17 / 0.13.  Sizes set, with / without, whole call:
 // 3000x2000 at 512 bits (16.3 warps per SM) 0.66 / 0.94, 2048x1536 at 256 (23.4) 0.52 /
-// 0.68, 1600x1200 at 128 (28.5) 0.56 / 0.68, 8 of 1024x768 at 512 (18.5) 0.41 / 0.65.
+// 0.68, 1600x1200 at 128 (28.5) 0.56 / 0.68, 8 of 1024x768 at 512 (18.5) 0.41 / 0.65;
+// longer ones do not pay there: 128 mixed files at 4096 (18.7) 1.01 / 0.93, 48 photos at
+// 4096 (30.2) 1.20 / 1.11, 64 mixed at 2048 (21.0) 0.72 / 0.68.
 #define BT_FILL_WARPS 8
 #define BT_FILL_HYP 16
 #define BT_FILL_HYP_SET 32
+#define BT_FILL_HYP_SET_BITS 512
 #define BT_HYP_MIN_BPM 5
 template <class F>
 static int bt_fill_bits(int from, int to, int sms, F warps) {
@@ -2367,18 +2379,20 @@ int cjBatchStage(CJBatch* b, int n, const unsigned char* blob, const int64_t* of
   // batch's own warps (bt_fill_bits)
   b->nhyp = 1;
   if (b->hyp_enabled) {
-    int maxbpm = 1;
+    int maxbpm = 1, max_sub = 0;
     for (int k = 0; k < nd; k++) {
       int bpm = 0;
       for (int c = 0; c < hh[k].nch; c++) bpm += hh[k].comp_sx[c] * hh[k].comp_sy[c];
       maxbpm = std::max(maxbpm, bpm);
+      max_sub = std::max(max_sub, dd[k].sub_bits);
     }
     const int nh = std::min(maxbpm, BT_MAX_HYP);
     int per_sm_hyp = 0;
     CJ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
                     &per_sm_hyp, (const void*)bt_decode_kernel(b->decode_ctas, true), BT_THREADS, bt_decode_smem(nh)),
                 CUDA_KERNEL_LAUNCH_ERROR);
-    const int64_t room = (int64_t)(b->sub_bits_auto ? BT_FILL_HYP : BT_FILL_HYP_SET) * b->sm_count;
+    const int64_t room =
+        (int64_t)(b->sub_bits_auto || max_sub > BT_FILL_HYP_SET_BITS ? BT_FILL_HYP : BT_FILL_HYP_SET) * b->sm_count;
     if (nh >= BT_HYP_MIN_BPM && per_sm_hyp > 0 && (int64_t)nsubw * nh <= room) {
       const size_t nsub = (size_t)nsubw * 32, nrec = nsub * 2 * nh;  // hypotheses and probes
       if (bt_ensure(b, b->hrecs, nrec * sizeof(CJSubRec)) || bt_ensure(b, b->hckpt, nrec * CJ_CKPTS * sizeof(CJCkpt)) ||
@@ -2867,7 +2881,7 @@ int cj_reader_decode(JPGReader* jpg, bool stage) {
     d->b_nhyp = 1;
     int cap_run = cap;  // co-resident CTAs of the variant that runs
     const int groups = (nwarps + BT_WARPS - 1) / BT_WARPS;
-    const int64_t room = (int64_t)(d->sub_bits_auto ? BT_FILL_HYP : BT_FILL_HYP_SET) * sms;
+    const int64_t room = (int64_t)(d->sub_bits_auto || sub > BT_FILL_HYP_SET_BITS ? BT_FILL_HYP : BT_FILL_HYP_SET) * sms;
     if (nh >= BT_HYP_MIN_BPM && (int64_t)nwarps * nh <= room) {
       int per_hyp = 0;
       CJ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_hyp, (const void*)bt_decode_kernel(BT_HYP_CTAS, true),

@@ -328,7 +328,8 @@ struct CJJoin {
 // stall the warp once per lane and checkpoint.
 // Phase entries: per MCU phase the shared addresses of the phase's tables
 // (x: dc | acm << 16), then ac1, the component << 16 and the next phase << 24
-// (y).  Written by the whole warp for an image and its tables at `tab`.
+// (y).  Written by the whole warp for an image and its tables at `tab` (0: offsets
+// into the set, for tables in global memory).
 __device__ __forceinline__ void cj_phase_entries(const CJScanParams& sp, uint32_t tab, uint32_t phases) {
   const int i = threadIdx.x & 31, bpm = sp.bpm;
   __syncwarp();
@@ -368,8 +369,8 @@ struct CJSpecJob {
   CJSubRec r;
 };
 __device__ __forceinline__ void cj_spec_job(CJSpecJob& x, const CJScanParams& sp, const CJScanParams& tp,
-                                            uint32_t tab, const uint8_t* gtab, const void* data, const CJLane& ln, CJCkpt* ck,
-                                            uint32_t cstep, const CJSpecWarp& sw) {
+                                            uint32_t tab, const uint8_t* gtab, const void* data, const CJLane& ln,
+                                            CJCkpt* ck, uint32_t cstep, const CJSpecWarp& sw) {
   x.sp = &sp;
   x.tp = &tp;
   x.tab = tab;

@@ -190,8 +190,8 @@ int cjBatchSetOutput(CJBatch *b, int format, int idct);
 int cjBatchSetParse(CJBatch *b, int on_device);
 /* MCU-phase hypotheses of the entropy decode (on != 0, the default): when a
  * staged batch's speculative decodes leave most of the GPU idle (a few
- * images: at most 16 warps per SM of these decodes, 32 at a subsequence size that
- * was set) and its MCUs have 5 blocks or more (4:2:0), each subsequence is also
+ * images: at most 16 warps per SM of these decodes, 32 where a subsequence size of
+ * at most 512 bits was set) and its MCUs have 5 blocks or more (4:2:0), each subsequence is also
  * decoded from its first bit under every other MCU phase and then from each of
  * its predecessor's hypothesis exits; the settle takes those decodes instead of
  * re-decoding lane after lane.  Results are identical either way; only the
