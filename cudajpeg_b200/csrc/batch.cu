@@ -1888,6 +1888,7 @@ static int bt_parse(CJBatch* b, const unsigned char* data, size_t size, CJImageH
                     int64_t* scan_off, int64_t* scan_len) {
   JPGReader* r = b->parser;
   r->huff_defined = 0;  // images of a batch are independent
+  memset(r->dev->dq16, 0, sizeof(r->dev->dq16));
   int e = cj_parse_to_scan(r, data, size);
   if (e) return e;
   e = bt_fill_header(r, h);
@@ -3040,7 +3041,7 @@ extern "C" int cjDecodeNoAlloc(const unsigned char* jpeg, size_t size, unsigned 
   // host parse on the stack
   JPGReader r;
   memset(&r, 0, sizeof(r));
-  CJReaderDevice rd;
+  CJReaderDevice rd{};  // (zeroed: a table the file does not define reads as zeros, as in a new reader)
   r.dev = &rd;
   int err = cj_parse_to_scan(&r, jpeg, size);
   if (err) return err;
